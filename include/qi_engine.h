@@ -315,7 +315,8 @@ typedef struct qi_exec_options {
 
 typedef struct qi_plan_stats {
     int64_t n_gates;          /* gates in the source list */
-    int64_t n_kernels;        /* kernel launches per execution */
+    int64_t n_kernels;        /* device operations (qi_plan_num_ops); an execution of a per-gate plan applies
+                                 several to a launch (qi_plan_run_info) */
     int64_t n_blocks_by_k[7]; /* fused blocks by width k (index 0 = per-gate ops) */
     double  predicted_us;     /* cost-model prediction of one execution (0 if none) */
 } qi_plan_stats;
@@ -463,6 +464,13 @@ qi_status qi_plan_op_phase_poly(const qi_plan *p, int64_t i, uint64_t *c0, uint6
  * xmask clear (one table of 2^rank[0] row-major 2x2 matrices acting on
  * (psi_i, psi_{i ^ xmask})).  rank: 4 entries, basis: 32.  Introspection aid. */
 qi_status qi_plan_op_pauli_group(const qi_plan *p, int64_t i, int32_t *n_tables, int32_t *rank, uint64_t *basis);
+/* How a per-gate plan (QI_FUSION_NONE, QI_FUSION_PAULI_GROUPS) is executed: n_passes launches that each
+ * apply a run of operations to tiles held in shared memory, in n_phases register phases altogether, and
+ * n_single operations with a launch of their own.  All 0 for fused plans.  Introspection aid. */
+qi_status qi_plan_run_info(const qi_plan *p, int64_t *n_passes, int64_t *n_phases, int64_t *n_single);
+/* The same passes executed on the host (FP64 plans without single operations) on 2^num_qubits
+ * interleaved amplitudes: a check of schedule and programs that needs no device. */
+qi_status qi_plan_run_replay(const qi_plan *p, double *amps);
 /* Execute the plan once with a CUDA event pair around every operation, on the
  * state's stream, and write each operation's device time in milliseconds to
  * ms_out (qi_plan_num_ops entries).  Measurement aid; no reference counterpart. */

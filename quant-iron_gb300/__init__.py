@@ -224,6 +224,20 @@ class Plan:
         return {"n_gates": s.n_gates, "n_kernels": s.n_kernels, "n_blocks_by_k": list(s.n_blocks_by_k),
                 "predicted_us": s.predicted_us}
 
+    def run_info(self):
+        """How a per-gate plan runs: (passes over the state, register phases, single operations)."""
+        v = [ctypes.c_int64() for _ in range(3)]
+        check(lib.qi_plan_run_info(self.h, *[ctypes.byref(x) for x in v]))
+        return tuple(x.value for x in v)
+
+    def run_replay(self, amps):
+        """The passes of an FP64 per-gate plan executed on the host (a check; no device work)."""
+        a = _as_c128(amps).copy()
+        if a.size != 1 << self.num_qubits:
+            raise ValueError("expected %d amplitudes, got %d" % (1 << self.num_qubits, a.size))
+        check(lib.qi_plan_run_replay(self.h, a.ctypes.data))
+        return a
+
     def ops(self):
         """The plan's device operations: list of dicts (kind, k, targets, control_mask,
         xmask, zmask, matrix as complex numpy array)."""

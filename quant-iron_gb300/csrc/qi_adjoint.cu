@@ -769,6 +769,7 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
         if (st.ok()) st = plan_execute(&plan, s);
         if (plan.d_mats) cudaFree(plan.d_mats);
         if (plan.d_tc) cudaFree(plan.d_tc);
+        release_runs(&plan);
         if (!st.ok()) return bail(st);
     }
     // lambda = H psi, and E = <psi|lambda> (one read pass of two states with FP64 sums, in place of
@@ -1070,6 +1071,7 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
     for (auto &sp : seg_plans) {
         if (sp->d_mats) cudaFree(sp->d_mats);
         if (sp->d_tc) cudaFree(sp->d_tc);
+        release_runs(sp.get());
     }
     if (d_gres) cudaFree(d_gres);
     qi_state_destroy(lam);

@@ -9,6 +9,7 @@
 #include "qi_internal.hpp"
 #include "qi_device.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 
@@ -444,6 +445,23 @@ Status state_scratch(qi_state *s, void **out) {
     return ok_status();
 }
 
+Status state_workspace(qi_state *s, size_t bytes, void **out) {
+    if (s->work_bytes < bytes) {
+        const size_t want = std::max<size_t>(bytes + bytes / 2, 64 * 1024);
+        void *p = nullptr;
+        cudaError_t e = cudaMalloc(&p, want);
+        if (e != cudaSuccess) {
+            (void)cudaGetLastError();
+            return cuda_status(e, "cudaMalloc(workspace)");
+        }
+        if (s->d_work) cudaFree(s->d_work);
+        s->d_work = p;
+        s->work_bytes = want;
+    }
+    *out = s->d_work;
+    return ok_status();
+}
+
 Status state_read_flag(qi_state *s, int *flag) {
     int h = 0;
     QI_CUDA(cudaMemcpyAsync(&h, s->d_flag, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
@@ -589,6 +607,7 @@ qi_status qi_state_destroy(qi_state *s) {
         if (s->d_flag) cudaFree(s->d_flag);
         if (s->d_staging) cudaFree(s->d_staging);
         if (s->d_scratch) cudaFree(s->d_scratch);
+        if (s->d_work) cudaFree(s->d_work);
         if (s->link_stream) {
             cudaStreamSynchronize(s->link_stream);
             cudaStreamDestroy(s->link_stream);

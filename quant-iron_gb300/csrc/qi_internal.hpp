@@ -65,6 +65,8 @@ struct qi_state {
     size_t staging_bytes = 0;
     int *d_flag = nullptr;            // device-side error flag (ZeroNorm inside async sequences)
     void *d_scratch = nullptr;        // second state buffer for out-of-place permutations (lazy)
+    void *d_work = nullptr;           // workspace of calls that finish before they return (lazy, grows)
+    size_t work_bytes = 0;
     cudaStream_t link_stream = nullptr;   // lowest-priority stream of uploads the GPU reads over the link (lazy)
     cudaEvent_t link_ev[2] = {nullptr, nullptr};   // orders it after, and before, this handle's stream
 
@@ -172,6 +174,10 @@ Status bitperm_async(qi_state *s, void *out, const void *in, const int8_t *perm,
 Status bitperm_in_place_async(qi_state *s, const int8_t *perm, uint64_t flip);
 // The state's second buffer (allocated on first use, freed with the state).
 Status state_scratch(qi_state *s, void **out);
+// The state's workspace, at least `bytes` long (16-byte aligned, freed with the state).  For calls that
+// wait for the state's stream before they return, so that nothing on the device still reads it
+// when the next call, on whichever stream, takes it.
+Status state_workspace(qi_state *s, size_t bytes, void **out);
 // Divide in by its FP64 norm into out (out != in; a norm of 0 or 1 copies unchanged, 0 flags ZeroNorm).
 Status state_normalise_device_to_async(qi_state *s, void *out, const void *in);
 // the same with the norm partials of `in` already in s->d_partials (nb rows)

@@ -5,7 +5,9 @@
 // A plan validates the whole gate list first (so an invalid gate leaves the
 // state untouched, as the reference's functional execute does), then lowers
 // it to device operations:
-//   QI_FUSION_NONE   one streaming kernel per gate (the plain per-gate method);
+//   QI_FUSION_NONE   per gate (the plain per-gate method): one op per gate; runs of
+//                    them execute several to a pass, each with its own arithmetic
+//                    (qi_gaterun.cu);
 //   QI_FUSION_GREEDY the greedy fuser below with block width k;
 //   QI_FUSION_LEARNED candidate partitions scored by the learned cost model
 //                    (qi_costmodel.cu), greedy as the fallback;
@@ -31,6 +33,7 @@
 // blocks and 8 diagonal runs instead of 142 and 9.
 #include "qi_internal.hpp"
 #include "qi_plan.hpp"
+#include "qi_gaterun.hpp"
 
 #include <algorithm>
 #include <cmath>
@@ -376,6 +379,35 @@ static void pad_block_to_5(int n, Op &op, std::vector<cd> &M) {
     for (int j = 0; j < 5; ++j) op.targets[j] = qs[j];
 }
 
+// The execution of a per-gate plan: every maximal run of two or more ops whose elements the passes
+// of qi_gaterun.cu can apply becomes one segment; any other op, and a run of one (the streaming
+// per-gate kernels touch the state as often as a pass would), its own.  first[i] is the first
+// element of op i (first[nops] = the element count).
+static void build_schedule(qi_plan *p, const std::vector<Elem> &elems, const std::vector<size_t> &first) {
+    const size_t nops = p->ops.size();
+    auto runnable = [&](size_t i) {
+        for (size_t e = first[i]; e < first[i + 1]; ++e)
+            if (!run_supported(p->n, p->prec, elems[e])) return false;
+        return true;
+    };
+    for (size_t i = 0; i < nops;) {
+        size_t j = i;
+        while (j < nops && runnable(j)) ++j;
+        if (j - i < 2) {
+            RunSegment seg;
+            seg.op = (int32_t)i++;
+            p->sched.push_back(std::move(seg));
+            continue;
+        }
+        std::vector<const Elem *> run;
+        for (size_t e = first[i]; e < first[j]; ++e) run.push_back(&elems[e]);
+        RunSegment seg;
+        schedule_run(p->n, p->prec, run, seg, p->run_prog);
+        p->sched.push_back(std::move(seg));
+        i = j;
+    }
+}
+
 Status build_plan(qi_plan *p, std::vector<Elem> &elems) {
     const int n = p->n;
     int fusion = p->opts.fusion;
@@ -387,6 +419,8 @@ Status build_plan(qi_plan *p, std::vector<Elem> &elems) {
     p->mats.clear();
     p->tc.clear();
     p->polys.clear();
+    p->sched.clear();
+    p->run_prog.clear();
     int tc_blocks_since = 0, tc_total = 0;
     std::fill(std::begin(p->stats.n_blocks_by_k), std::end(p->stats.n_blocks_by_k), 0);
     p->stats.n_gates = (int64_t)elems.size();
@@ -425,9 +459,14 @@ Status build_plan(qi_plan *p, std::vector<Elem> &elems) {
         auto groupable = [&](const Elem &e) {
             return fusion == QI_FUSION_PAULI_GROUPS && e.pauli && !e.gm.normalise_after;
         };
+        std::vector<size_t> first;   // element each op starts at
+        auto note = [&](size_t e) {
+            if (first.size() < p->ops.size()) first.push_back(e);
+        };
         for (size_t i = 0; i < elems.size();) {
             if (!groupable(elems[i])) {
-                lower_single(elems[i++]);
+                lower_single(elems[i]);
+                note(i++);
                 continue;
             }
             std::vector<const GateMatrix *> run;
@@ -442,10 +481,13 @@ Status build_plan(qi_plan *p, std::vector<Elem> &elems) {
                     p->ops.push_back(op);
                     p->stats.n_blocks_by_k[0]++;
                 }
+                note(i + used);
                 used += took;
             }
             i = j;
         }
+        first.push_back(elems.size());
+        build_schedule(p, elems, first);
     } else {
         std::vector<Block> blocks = p->partition_override.empty() ? partition_with_permutations(p, elems, kmax)
                                                                   : p->partition_override;
@@ -570,6 +612,10 @@ Status build_plan(qi_plan *p, std::vector<Elem> &elems) {
     return ok_status();
 }
 
+static bool not_uploaded(const qi_plan *p) {
+    return (!p->d_mats && !p->mats.empty()) || (!p->d_tc && !p->tc.empty());
+}
+
 Status upload_plan(qi_plan *p) {
     if (p->d_mats) { cudaFree(p->d_mats); p->d_mats = nullptr; }
     if (p->d_tc) { cudaFree(p->d_tc); p->d_tc = nullptr; }
@@ -615,6 +661,52 @@ Status plan_elems_from_gates(int n, const qi_gate *gates, int64_t ng, const doub
         elems.push_back(make_elem_from_gate(gm, (int)k));
     }
     return ok_status();
+}
+
+// Whether the plan's runs can execute on s: their program goes to s's device on first use.  Where that
+// is not possible (the stream is being captured, the program is on another device, no memory), the
+// plan's ops run one kernel each instead.
+static bool runs_ready(qi_plan *p, qi_state *s) {
+    if (p->run_prog.empty()) return false;
+    std::lock_guard<std::mutex> lk(p->run_mu);
+    if (p->d_run) return p->run_device == s->device;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    void *d = nullptr;
+    if (cudaMalloc(&d, p->run_prog.size()) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    if (cudaMemcpy(d, p->run_prog.data(), p->run_prog.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+        (void)cudaGetLastError();
+        cudaFree(d);
+        return false;
+    }
+    p->d_run = d;
+    p->run_device = s->device;
+    return true;
+}
+
+// The same for a plan that lives for one call on one state: its program is copied into the state's
+// workspace, in stream order (the caller waits for the stream before it lets go of the state).
+static void borrow_runs(qi_plan *p, qi_state *s) {
+    void *d = nullptr;
+    if (p->run_prog.empty() || !state_workspace(s, p->run_prog.size(), &d).ok()) return;
+    if (cudaMemcpyAsync(d, p->run_prog.data(), p->run_prog.size(), cudaMemcpyHostToDevice, s->stream) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return;
+    }
+    p->d_run = d;
+    p->run_device = s->device;
+    p->run_borrowed = true;
+}
+
+void release_runs(qi_plan *p) {
+    if (p->d_run && !p->run_borrowed) cudaFree(p->d_run);
+    p->d_run = nullptr;
 }
 
 // Launches a plan's ops on a state.  OP_BITPERM writes out of place: the amplitudes move to
@@ -670,13 +762,27 @@ struct PlanRunner {
 Status plan_execute(qi_plan *p, qi_state *s) {
     if (s->n != p->n) return err(QI_ERR_INVALID_NUMBER_OF_QUBITS, s->n);   // circuit.rs:161-163
     if (s->prec != p->prec) return err(QI_ERR_UNSUPPORTED, -1, -1, "plan precision differs from state");
-    if ((!p->d_mats && !p->mats.empty()) || (!p->d_tc && !p->tc.empty())) {   // matrices go to the device on first use
+    if (not_uploaded(p)) {   // matrices go to the device on first use
         Status up = upload_plan(p);
         if (!up.ok()) return up;
     }
     bool has_norm = false;
     PlanRunner run(p, s);
-    for (size_t i = 0; i < p->ops.size(); ++i) {
+    const bool runs = runs_ready(p, s);
+    for (size_t i = 0; runs && i < p->sched.size(); ++i) {
+        const RunSegment &seg = p->sched[i];
+        if (seg.op >= 0) {
+            const Op &op = p->ops[(size_t)seg.op];
+            Status st = run.op(op, -1);
+            if (!st.ok()) return run.finish(st);
+            has_norm = has_norm || op.kind == OP_PAULI_NORM;
+        }
+        for (const RunPass &pass : seg.passes) {
+            Status st = launch_run_pass(s, pass, p->d_run);
+            if (!st.ok()) return run.finish(st);
+        }
+    }
+    for (size_t i = 0; !runs && i < p->ops.size(); ++i) {
         const Op &op = p->ops[i];
         Status st = run.op(op, i + 1 < p->ops.size() ? p->ops[i + 1].kind : -1);
         if (!st.ok()) return run.finish(st);
@@ -752,7 +858,7 @@ qi_status qi_plan_profile(qi_plan *p, qi_state *s, float *ms_out) {
     cudaError_t e = cudaSetDevice(s->device);
     if (e != cudaSuccess) return publish(cuda_status(e, "cudaSetDevice"));
     if (s->n != p->n || s->prec != p->prec) return publish(err(QI_ERR_INVALID_NUMBER_OF_QUBITS, s->n));
-    if ((!p->d_mats && !p->mats.empty()) || (!p->d_tc && !p->tc.empty())) {
+    if (not_uploaded(p)) {
         Status up = upload_plan(p);
         if (!up.ok()) return publish(up);
     }
@@ -849,6 +955,30 @@ qi_status qi_plan_num_ops(const qi_plan *p, int64_t *out) {
     return publish(ok_status());
 }
 
+qi_status qi_plan_run_info(const qi_plan *p, int64_t *n_passes, int64_t *n_phases, int64_t *n_single) {
+    if (!p || !n_passes || !n_phases || !n_single) return publish(err(QI_ERR_NULL_ARGUMENT));
+    *n_passes = *n_phases = *n_single = 0;
+    for (const RunSegment &seg : p->sched) {
+        *n_single += seg.op >= 0;
+        for (const RunPass &pass : seg.passes) {
+            ++*n_passes;
+            *n_phases += pass.nphase;
+        }
+    }
+    return publish(ok_status());
+}
+
+qi_status qi_plan_run_replay(const qi_plan *p, double *amps) {
+    if (!p || !amps) return publish(err(QI_ERR_NULL_ARGUMENT));
+    if (p->prec != QI_F64) return publish(err(QI_ERR_UNSUPPORTED, p->prec, -1, "replay is of FP64 plans"));
+    for (const RunSegment &seg : p->sched)
+        if (seg.op >= 0) return publish(err(QI_ERR_UNSUPPORTED, seg.op, -1, "operation outside a run"));
+    for (const RunSegment &seg : p->sched)
+        for (const RunPass &pass : seg.passes)
+            replay_run_pass(p->n, pass, p->run_prog.data(), reinterpret_cast<cd *>(amps));
+    return publish(ok_status());
+}
+
 qi_status qi_plan_op_phase_poly(const qi_plan *p, int64_t i, uint64_t *c0, uint64_t *a, uint64_t *b) {
     if (!p || !c0 || !a || !b) return publish(err(QI_ERR_NULL_ARGUMENT));
     if (i < 0 || i >= (int64_t)p->ops.size()) return publish(err(QI_ERR_INVALID_INPUT_VALUE, i));
@@ -939,6 +1069,7 @@ qi_status qi_plan_destroy(qi_plan *p) {
     if (!p) return QI_OK;
     if (p->d_mats) cudaFree(p->d_mats);
     if (p->d_tc) cudaFree(p->d_tc);
+    release_runs(p);
     delete p;
     return QI_OK;
 }
@@ -949,9 +1080,10 @@ qi_status qi_circuit_execute(qi_state *s, const qi_gate *gates, int64_t n_gates,
     qi_plan *p = nullptr;
     qi_status st = qi_plan_create(s->n, s->prec, gates, n_gates, theta, n_theta, opts, &p);
     if (st != QI_OK) return st;
+    std::lock_guard<std::recursive_mutex> lk(s->mu);   // held until the plan's program is no longer in use
+    if (cudaSetDevice(s->device) == cudaSuccess) borrow_runs(p, s);
     st = qi_plan_execute(p, s);
     if (st == QI_OK) {
-        std::lock_guard<std::recursive_mutex> lk(s->mu);
         cudaError_t e = cudaStreamSynchronize(s->stream);
         if (e != cudaSuccess) {
             st = publish(cuda_status(e, "execute"));
@@ -980,14 +1112,17 @@ qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_t
         if (!st.ok()) return publish(st);
     }
     if (observable && observe_every > 0 && !energies_out) return publish(err(QI_ERR_NULL_ARGUMENT));
-    // One step as an ordered list of exponentials (time_evolution.rs:45-115).
-    std::vector<Elem> elems;
-    if (order == 1) {
-        for (int64_t k = 0; k < n_terms; ++k) elems.push_back(pauli_exp_elem(terms[k], 0.0, -dt, (int)k));
-    } else {
-        for (int64_t k = 0; k < n_terms; ++k) elems.push_back(pauli_exp_elem(terms[k], 0.0, -dt / 2.0, (int)k));
-        for (int64_t k = n_terms - 1; k >= 0; --k) elems.push_back(pauli_exp_elem(terms[k], 0.0, -dt / 2.0, (int)k));
-    }
+    // `steps` steps as an ordered list of exponentials (time_evolution.rs:45-115).
+    auto step_list = [&](int64_t steps) {
+        std::vector<Elem> elems;
+        for (int64_t r = 0; r < steps; ++r) {
+            const double f = order == 1 ? -dt : -dt / 2.0;
+            for (int64_t k = 0; k < n_terms; ++k) elems.push_back(pauli_exp_elem(terms[k], 0.0, f, (int)k));
+            for (int64_t k = n_terms - 1; order == 2 && k >= 0; --k)
+                elems.push_back(pauli_exp_elem(terms[k], 0.0, f, (int)k));
+        }
+        return elems;
+    };
     // FP32: the step is one fused plan: narrow exponentials compose into dense
     // blocks (FP64 composition) and runs of Z-type exponentials into phase
     // polynomials.  With real coefficients every exponential is unitary, so the
@@ -999,21 +1134,45 @@ qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_t
     // with a parity-indexed table; other terms are one pass each.
     bool unitary = true;
     for (int64_t k = 0; k < n_terms; ++k) unitary = unitary && terms[k].coeff_im == 0.0;
-    qi_plan plan;
-    plan.n = s->n;
-    plan.prec = s->prec;
-    plan.opts.fusion = s->prec == QI_F32 ? QI_FUSION_GREEDY : QI_FUSION_PAULI_GROUPS;
-    plan.opts.use_tensor_cores = unitary ? 1 : 2;
-    plan.opts.renorm_every = unitary ? 0 : -1;
-    plan.opts.max_block_qubits = 0;
-    Status st = build_plan(&plan, elems);
-    if (st.ok()) st = upload_plan(&plan);
-    if (!st.ok()) return publish(st);
+    const bool observing = observable && observe_every > 0;
+    // FP64 second-order steps: the terms that end one step begin the next, and equal exponentials with
+    // nothing between join (qi_gaterun.cu), so a plan covers several steps: the most up to 6 that divide
+    // the steps to take (one plan to build; the joined fraction grows as 1 - 1 / steps), else 4.
+    int64_t many = 1;
+    if (s->prec == QI_F64 && order == 2) {
+        const int64_t span = observing ? std::min(observe_every, num_steps) : num_steps;
+        const int64_t cap = std::min<int64_t>({span, 6, std::max<int64_t>(1, 1000 / n_terms)});
+        for (int64_t k = 2; k <= cap; ++k)
+            if (span % k == 0) many = k;
+        if (many == 1) many = std::min<int64_t>(cap, 4);
+    }
+    qi_plan single, several;
+    auto prepare = [&](qi_plan &plan, int64_t steps) {
+        plan.n = s->n;
+        plan.prec = s->prec;
+        plan.opts.fusion = s->prec == QI_F32 ? QI_FUSION_GREEDY : QI_FUSION_PAULI_GROUPS;
+        plan.opts.use_tensor_cores = unitary ? 1 : 2;
+        plan.opts.renorm_every = unitary ? 0 : -1;
+        plan.opts.max_block_qubits = 0;
+        std::vector<Elem> elems = step_list(steps);
+        Status st = build_plan(&plan, elems);
+        if (st.ok()) st = upload_plan(&plan);
+        return st;
+    };
+    Status st = ok_status();
+    bool have_single = false, have_several = false;
     int64_t obs_k = 0;
-    for (int64_t step = 0; step < num_steps; ++step) {
-        st = plan_execute(&plan, s);
+    for (int64_t step = 0; step < num_steps && st.ok();) {
+        const int64_t left = observing ? std::min(num_steps - step, observe_every - step % observe_every) : num_steps - step;
+        const bool more = many > 1 && left >= many;
+        qi_plan &plan = more ? several : single;
+        bool &have = more ? have_several : have_single;
+        if (!have) st = prepare(plan, more ? many : 1);
+        have = true;
+        if (st.ok()) st = plan_execute(&plan, s);
         if (!st.ok()) break;
-        if (observable && observe_every > 0 && ((step + 1) % observe_every) == 0) {
+        step += more ? many : 1;
+        if (observing && step % observe_every == 0) {
             double ev[2];
             st = sumop_expectation(s, observable, n_obs, ev);
             if (!st.ok()) break;
@@ -1022,10 +1181,13 @@ qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_t
             ++obs_k;
         }
     }
-    if (plan.d_mats) cudaFree(plan.d_mats);
-    if (plan.d_tc) cudaFree(plan.d_tc);
-    plan.d_tc = nullptr;
-    plan.d_mats = nullptr;
+    for (qi_plan *plan : {&single, &several}) {
+        if (plan->d_mats) cudaFree(plan->d_mats);
+        if (plan->d_tc) cudaFree(plan->d_tc);
+        release_runs(plan);
+        plan->d_tc = nullptr;
+        plan->d_mats = nullptr;
+    }
     if (!st.ok()) return publish(st);
     e = cudaStreamSynchronize(s->stream);
     if (e != cudaSuccess) return publish(cuda_status(e, "trotter"));

@@ -4,6 +4,8 @@
 #include "qi_internal.hpp"
 
 #include <complex>
+#include <cstdint>
+#include <mutex>
 #include <vector>
 
 namespace qi {
@@ -37,6 +39,22 @@ Block window_block(const std::vector<Elem> &elems, const std::vector<int> &remai
 void compose_block(const std::vector<Elem> &elems, const Block &b, std::vector<int> &qubits,
                    std::vector<std::complex<double>> &B);
 
+// One pass of a run of per-gate operations (qi_gaterun.cu): the local qubits (ascending) and the
+// byte range of its program.
+struct RunPass {
+    int32_t tbits = 0;          // local amplitude bits (tile of 2^tbits amplitudes)
+    int32_t low = 0;            // qubits 0 .. low-1 are local: contiguous runs of 2^low amplitudes
+    int8_t pos[16] = {0};
+    int32_t nphase = 0;
+    int32_t prog_off = 0, prog_bytes = 0;   // into the plan's run program (16-byte multiples)
+    std::vector<uint16_t> slot_at;          // 16-byte units (from prog_off) of the operations with a tile factor
+};
+// A step of a per-gate plan's execution: the passes of a run of operations, or one operation.
+struct RunSegment {
+    int32_t op = -1;            // index into the plan's ops; -1: passes
+    std::vector<RunPass> passes;
+};
+
 }  // namespace qi
 
 struct qi_plan {
@@ -50,6 +68,13 @@ struct qi_plan {
                                               // and phase-polynomial blocks, as raw 32-bit words
     void *d_tc = nullptr;
     std::vector<qi::PhasePoly> polys;         // host copy of each OP_PHASE_POLY op (op.mat_offset indexes it)
+    // Per-gate plans: how the ops are executed (several to a pass), and the passes' programs.
+    std::vector<qi::RunSegment> sched;
+    std::vector<uint8_t> run_prog;
+    void *d_run = nullptr;        // the programs on device run_device, once executed there
+    int32_t run_device = -1;
+    bool run_borrowed = false;    // d_run is a state's workspace
+    std::mutex run_mu;            // first use
     qi_plan_stats stats = {};
     std::vector<qi::Block> partition_override;   // set by callers that chose the partition
     bool learned_blocks = false;                 // QI_FUSION_LEARNED chose the model-scored partition
@@ -58,6 +83,7 @@ struct qi_plan {
 namespace qi {
 Status build_plan(qi_plan *p, std::vector<Elem> &elems);
 Status upload_plan(qi_plan *p);
+void release_runs(qi_plan *p);
 Status plan_execute(qi_plan *p, qi_state *s);
 Status plan_elems_from_gates(int n, const qi_gate *gates, int64_t ng, const double *theta, int64_t ntheta,
                              std::vector<Elem> &elems);
