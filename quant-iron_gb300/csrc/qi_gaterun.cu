@@ -23,7 +23,7 @@
 // Reference: Gate::apply / Circuit::execute (src/components/gate.rs:99-122, src/circuit.rs:160-172),
 // operator.rs:279-2285, PauliString::apply_exp_factor (src/components/pauli_string.rs:237-262).
 #include "qi_gaterun.hpp"
-#include "qi_device.cuh"
+#include "qi_runtile.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -52,12 +52,6 @@ enum RunCode : int {
     RC_SCALE = 14    // all amplitudes times a real or complex number
 };
 
-struct RunPhaseHdr {   // 32 bytes
-    uint8_t rb[4];     // unit bits held in registers
-    uint8_t tb[16];    // unit bit of thread-index bit j
-    uint16_t nops;
-    uint8_t pad[10];
-};
 struct RunOpHdr {      // 32 bytes
     uint8_t code, xi, nsub, units;   // xi: register partner mask / AND mask; units: 16-byte size, of the
                                      // header alone for RC_PHASE (its parts give their own)
@@ -80,20 +74,9 @@ enum RunPhaseFlags : uint32_t { kTileFactor = 1, kLaneTable = 2, kWarpTable = 4 
 constexpr size_t kRunMaxPhase = 48;   // elements of a phase: with headers, terms and (one per two terms) tables
                                       // 48 * 96 + 24 * 768 bytes, always less than a pass may hold
 constexpr int kRunMaxSlots = 64;   // tile factors a pass may hold
-static_assert(sizeof(RunPhaseHdr) == 32 && sizeof(RunOpHdr) == 32 && sizeof(RunSub) == 16, "program layout");
+static_assert(sizeof(RunOpHdr) == 32 && sizeof(RunSub) == 16, "program layout");
 
 // ------------------------------------------------------------- kernel ---
-__device__ __forceinline__ double flip_sign(double x, uint32_t s) {   // s = 0 or 1
-    return __hiloint2double(__double2hiint(x) ^ (int)(s << 31), __double2loint(x));
-}
-__device__ __forceinline__ float flip_sign(float x, uint32_t s) { return __int_as_float(__float_as_int(x) ^ (int)(s << 31)); }
-
-template <typename T> struct RunShape;
-template <> struct RunShape<double> { static constexpr int kRegBits = kRunSelBits, kUnitBits = 0; };
-template <> struct RunShape<float> { static constexpr int kRegBits = kRunSelBits + 1, kUnitBits = 1; };
-
-constexpr int top_bit(int x) { return x >= 8 ? 8 : x >= 4 ? 4 : x >= 2 ? 2 : 1; }
-
 // Pair updates on the register pairs (k, k ^ X).  SIGN: off-diagonal terms carry the sign of the
 // pair's Z parity.
 template <typename T, int CODE, int X, bool SIGN>
@@ -218,21 +201,11 @@ struct RunGeom {
     uint16_t slot_at[kRunMaxSlots];   // 16-byte unit of the RC_PHASE operation that owns the slot
 };
 
-// Unit address in shared memory: the low three bits are XORed with the higher groups of three, so
-// that eight lanes whose unit indices differ in three bits of distinct residues modulo 3 read
-// eight different 16-byte bank groups (the host orders the thread bits that way).
-__host__ __device__ __forceinline__ uint32_t run_swizzle(uint32_t u) { return u ^ (((u >> 3) ^ (u >> 6) ^ (u >> 9)) & 7u); }
-
-__device__ __forceinline__ void copy16(void *dst, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-                 : "memory");
-}
-
 // Shared memory: tile | offsets of the tile's rows | program.
 template <typename T>
 __global__ void __launch_bounds__(256) k_gate_run(typename Cx<T>::V2 *amps, const uint4 *prog, const __grid_constant__ RunGeom g) {
     using V2 = typename Cx<T>::V2;
-    constexpr int RS = kRunSelBits, RB = RunShape<T>::kRegBits, NV = 1 << RB, UB0 = RunShape<T>::kUnitBits;
+    constexpr int RB = RunShape<T>::kRegBits, NV = 1 << RB, UB0 = RunShape<T>::kUnitBits;
     extern __shared__ uint4 sm[];
     const int ubits = g.tbits - UB0, lowu = g.low - UB0;
     const uint32_t nunit = 1u << ubits, nrow = 1u << (ubits - lowu), nt = blockDim.x, tid = threadIdx.x;
@@ -241,17 +214,18 @@ __global__ void __launch_bounds__(256) k_gate_run(typename Cx<T>::V2 *amps, cons
     uint4 *code = sm + nunit + ((nrow + 1) >> 1);
     const uint64_t tbase = insert_zeros(blockIdx.x, g.pos, g.tbits);
     for (uint32_t r = tid; r < nrow; r += nt) {   // first unit of each row (2^low consecutive amplitudes)
-        uint64_t off = tbase;
+        uint64_t off = 0;
         for (int j = g.low; j < g.tbits; ++j) off |= (uint64_t)((r >> (j - g.low)) & 1u) << g.pos[j];
         rows[r] = off >> UB0;
     }
     for (uint32_t i = tid; i < (uint32_t)g.prog_units; i += nt) copy16(code + i, prog + i);
     __syncthreads();
-    uint4 *a4 = reinterpret_cast<uint4 *>(amps);
-    const uint32_t lmask = (1u << lowu) - 1u;
-    for (uint32_t u = tid; u < nunit; u += nt) copy16(tile + run_swizzle(u), a4 + (rows[u >> lowu] + (u & lmask)));
+    uint4 *a4 = reinterpret_cast<uint4 *>(amps) + (tbase >> UB0);
+    const RunCopy mine(rows, tid, lowu);
+    for (uint32_t u = 0; u < nunit; u += nt)
+        copy16((char *)tile + (mine.at ^ (run_swizzle(u) << 4)), a4 + (mine.first + RunCopy::step(rows, u, lowu)));
     __shared__ V2 slot[kRunMaxSlots];
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    copy_wait();
     __syncthreads();
     for (uint32_t i = tid; i < (uint32_t)g.nslot; i += nt) {   // read after the first phase's loads, below
         const RunOpHdr &h = *reinterpret_cast<const RunOpHdr *>(code + g.slot_at[i]);
@@ -268,22 +242,12 @@ __global__ void __launch_bounds__(256) k_gate_run(typename Cx<T>::V2 *amps, cons
     for (int ph = 0; ph < g.nphase; ++ph) {
         const RunPhaseHdr &hd = *reinterpret_cast<const RunPhaseHdr *>(code + pc);
         const int nops = hd.nops;
-        uint32_t ubase = 0;
-        for (int j = 0; j < ubits - RS; ++j) ubase |= ((tid >> j) & 1u) << hd.tb[j];
-        const uint32_t c0 = run_swizzle(1u << hd.rb[0]), c1 = run_swizzle(1u << hd.rb[1]), c2 = run_swizzle(1u << hd.rb[2]);
-        const uint32_t abase = run_swizzle(ubase), lbase = ubase << UB0;
+        const uint32_t place = run_place(hd, tid, ubits - kRunSelBits, UB0), lbase = place >> 16;
+        uint32_t at[1 << kRunSelBits];
+        run_units<kRunSelBits>(at, place, hd);
         pc += 2;
         V2 v[NV];
-#pragma unroll
-        for (int k = 0; k < (1 << RS); ++k) {
-            const uint4 q = tile[abase ^ ((k & 1) ? c0 : 0u) ^ ((k & 2) ? c1 : 0u) ^ ((k & 4) ? c2 : 0u)];
-            if constexpr (sizeof(T) == 8) {
-                v[k] = Cx<T>::make(__hiloint2double((int)q.y, (int)q.x), __hiloint2double((int)q.w, (int)q.z));
-            } else {
-                v[2 * k] = Cx<T>::make(__uint_as_float(q.x), __uint_as_float(q.y));
-                v[2 * k + 1] = Cx<T>::make(__uint_as_float(q.z), __uint_as_float(q.w));
-            }
-        }
+        run_load<T, kRunSelBits>(v, tile, at);
         for (int o = 0; o < nops; ++o) {
             const RunOpHdr &h = *reinterpret_cast<const RunOpHdr *>(code + pc);
             const int op = h.code, xi = h.xi;
@@ -379,21 +343,11 @@ __global__ void __launch_bounds__(256) k_gate_run(typename Cx<T>::V2 *amps, cons
             }
             }
         }
-#pragma unroll
-        for (int k = 0; k < (1 << RS); ++k) {
-            uint4 q;
-            if constexpr (sizeof(T) == 8) {
-                q = make_uint4((uint32_t)__double2loint(v[k].x), (uint32_t)__double2hiint(v[k].x),
-                               (uint32_t)__double2loint(v[k].y), (uint32_t)__double2hiint(v[k].y));
-            } else {
-                q = make_uint4(__float_as_uint(v[2 * k].x), __float_as_uint(v[2 * k].y), __float_as_uint(v[2 * k + 1].x),
-                               __float_as_uint(v[2 * k + 1].y));
-            }
-            tile[abase ^ ((k & 1) ? c0 : 0u) ^ ((k & 2) ? c1 : 0u) ^ ((k & 4) ? c2 : 0u)] = q;
-        }
+        run_store<T, kRunSelBits>(v, tile, at);
         __syncthreads();
     }
-    for (uint32_t u = tid; u < nunit; u += nt) a4[rows[u >> lowu] + (u & lmask)] = tile[run_swizzle(u)];
+    for (uint32_t u = 0; u < nunit; u += nt)
+        a4[mine.first + RunCopy::step(rows, u, lowu)] = *reinterpret_cast<uint4 *>((char *)tile + (mine.at ^ (run_swizzle(u) << 4)));
 }
 
 static size_t run_smem(const RunPass &p, int unit_bit) {
@@ -918,23 +872,10 @@ struct Encoder {
         int nr = 0;
         for (int u = 0; u < ubits; ++u)
             if ((R >> pass->pos[u + ub0]) & 1ull) {
-                hd.rb[nr] = (uint8_t)u;
-                rmap[u + ub0] = (int8_t)(nr + ub0);
+                rmap[u + ub0] = (int8_t)(nr++ + ub0);
                 regu |= 1u << u;
-                ++nr;
             }
-        // thread bits: three of distinct residues modulo 3 first (no bank conflicts), then ascending
-        int nb = 0;
-        uint32_t used = regu;
-        for (int r = 0; r < 3; ++r)
-            for (int u = r; u < ubits; u += 3)
-                if (!((used >> u) & 1u)) {
-                    hd.tb[nb++] = (uint8_t)u;
-                    used |= 1u << u;
-                    break;
-                }
-        for (int u = 0; u < ubits; ++u)
-            if (!((used >> u) & 1u)) hd.tb[nb++] = (uint8_t)u;
+        run_phase_bits(hd, regu, ubits);
 
         list.clear();
         terms.clear();

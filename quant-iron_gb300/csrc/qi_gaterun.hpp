@@ -7,10 +7,6 @@
 
 namespace qi {
 
-constexpr int kRunTileBits = 11;    // 16-byte units of a tile: at most 2^11 (32 KB of shared memory)
-constexpr int kRunSelBits = 3;      // selectable register bits of a phase (2^3 units per thread)
-constexpr int kRunMaxProg = 24576;  // bytes of program a pass may hold (copied to shared memory)
-
 // Whether the passes can apply this gate or Pauli exponential.
 bool run_supported(int n, int prec, const Elem &e);
 // Schedule elems (all run_supported) into passes appended to seg, their programs to prog.
