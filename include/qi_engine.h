@@ -343,7 +343,9 @@ qi_status qi_plan_destroy(qi_plan *p);
  * accumulates in FP64: runs of single-qubit gates share one pass, runs of fixed
  * X / CNOT / SWAP gates are one index permutation, other fixed runs one fused
  * plan of their inverses, the rest one pass per gate (qi_adjoint_sweep_plan
- * lists the passes).  Differentiable kinds: RX, RY, RZ, P, RYPHASE,
+ * lists the passes).  Where every gate is an uncontrolled RX / RY / RZ / P with
+ * a parameter or a fixed gate (FP64 states; FP32 up to 22 qubits), the sweep runs
+ * as passes over tiles of psi and lambda that hold many gates each.  Differentiable kinds: RX, RY, RZ, P, RYPHASE,
  * RYPHASE_DAG, MATCHGATE (any controls).
  * On entry `s` holds |psi0>; on return it holds |psi0> again (restored by the
  * reverse sweep up to rounding).  energy_out (may be NULL) receives E;

@@ -15,6 +15,7 @@
 #include "qi_internal.hpp"
 #include "qi_device.cuh"
 #include "qi_plan.hpp"
+#include "qi_gaterun.hpp"
 #include "qi_tile.cuh"
 
 #include <algorithm>
@@ -706,6 +707,8 @@ extern "C" qi_status qi_adjoint_sweep_plan(int32_t num_qubits, int32_t precision
     return publish(ok_status());
 }
 
+constexpr int kSweepMaxF32 = 22;   // FP32 sweeps in tile passes up to this many qubits (see below)
+
 extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int64_t n_gates, const double *theta,
                                          int64_t n_theta, const qi_pauli_term *terms, int64_t n_terms,
                                          const qi_exec_options *forward_opts, double *energy_out, double *grads_out) {
@@ -732,6 +735,7 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
     // alone took the gradient from 7e-7 to 1.3e-6 of the FP64 result.
     qi_exec_options plan_opts = {QI_FUSION_GREEDY, 0, 0, 0};
     if (forward_opts) plan_opts = *forward_opts;
+    const int chosen_block = plan_opts.max_block_qubits;
     if (s->prec == QI_F32 && plan_opts.max_block_qubits <= 0) plan_opts.max_block_qubits = 5;
     // psi_0 stays untouched in the caller's buffer: the sweep runs on a copy (un-applying psi in
     // FP32 would hand back psi_0 with the sweep's rounding in it); without room for the copy it
@@ -762,6 +766,11 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
         plan.n = n;
         plan.prec = s->prec;
         plan.opts = plan_opts;
+        // FP64 (dense FP64 blocks are bound by the FP64 pipe) and FP32 up to 22 qubits unless the caller
+        // chose a block size: the gate runs' own arithmetic, with no block matrices to compose (FP32
+        // gradients, fused / gate runs: 8 qubits 1.57 / 0.37 ms, 20 qubits 4.25 / 2.58, 22 qubits 7.8 /
+        // 6.2, 24 qubits 18.0 / 20.1; relative error at 20 qubits 6.1e-7 / 4.7e-7)
+        if (s->prec == QI_F64 || (chosen_block <= 0 && n <= kSweepMaxF32)) plan.opts.fusion = QI_FUSION_NONE;
         std::vector<Elem> elems;
         Status st = plan_elems_from_gates(n, gates, n_gates, theta, n_theta, elems);
         if (st.ok()) st = build_plan(&plan, elems);
@@ -814,11 +823,68 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
     // (the exact-scale matrices may carry a global phase into psi: only when psi_0 is not the
     // state the sweep hands back)
     const bool scale_fix = f32 && work != nullptr;
-    if (st.ok() && f32) st = state_reduce_norm_sqr(s, &npsi0);
-    if (st.ok() && f32 && n_terms > 0) st = state_reduce_norm_sqr(lam, &nlam0);
+    // Tile passes (qi_adjrun.cu) where every gate allows it: uncontrolled RX / RY / RZ / P with a
+    // parameter, any fixed gate of a gate run.  They need the copy of psi_0 (psi ends scaled); without
+    // fusion each gate keeps its own pass.  FP32 sweeps of more than 22 qubits stream faster through the
+    // grouped kernels, which keep one group's arithmetic in the instruction cache (12-layer ansatz, tiles
+    // against groups: 20 qubits 4.2 / 5.9 ms, 22 qubits 7.2 / 8.1, 23 qubits 11.4 / 11.3, 26 qubits 72 / 57).
+    bool tiles = st.ok() && work != nullptr && plan_opts.fusion != QI_FUSION_NONE && (!f32 || n <= kSweepMaxF32);
+    std::vector<SweepGate> sweep_gates;
+    std::vector<std::pair<int, int32_t>> term_param;   // term -> gate, parameter
+    for (int64_t j = n_gates - 1; j >= 0 && tiles; --j) {
+        int np = 0, id = -1;
+        for (int k = 0; k < 3; ++k)
+            if (resolved[(size_t)j].param_ids[k] >= 0) {
+                ++np;
+                id = resolved[(size_t)j].param_ids[k];
+            }
+        tiles = sweep_supported(n, s->prec, mats[(size_t)j], np);
+        sweep_gates.push_back({&mats[(size_t)j], np ? (int)term_param.size() : -1});
+        if (np) term_param.push_back({(int)j, id});
+    }
+    if (tiles && n_theta > 0) {
+        std::vector<SweepPass> passes;
+        std::vector<uint8_t> prog;
+        schedule_sweep(n, s->prec, sweep_gates, passes, prog);
+        // workspace: program, partials, terms
+        const size_t at_part = (prog.size() + 255) / 256 * 256;
+        const size_t at_term = at_part + (size_t)kSweepBlocks * kSweepTerms * sizeof(double);
+        void *ws = nullptr;
+        st = state_workspace(s, at_term + (term_param.size() + 1) * sizeof(double), &ws);
+        if (st.ok() && !prog.empty()) {
+            e = cudaMemcpyAsync(ws, prog.data(), prog.size(), cudaMemcpyHostToDevice, s->stream);
+            if (e != cudaSuccess) st = cuda_status(e, "sweep program");
+        }
+        double *terms_dev = reinterpret_cast<double *>((char *)ws + at_term);
+        size_t at = 0;
+        for (size_t i = 0; i < passes.size() && st.ok(); ++i) {
+            st = launch_sweep_pass(s, lam->amps, passes[i], ws, reinterpret_cast<double *>((char *)ws + at_part), terms_dev + at);
+            at += passes[i].slot.size();
+        }
+        std::vector<double> h(term_param.size() + 1, 0.0);
+        if (st.ok()) {
+            e = cudaMemcpyAsync(h.data(), terms_dev, term_param.size() * sizeof(double), cudaMemcpyDeviceToHost, s->stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+            if (e != cudaSuccess) st = cuda_status(e, "adjoint");
+        }
+        if (st.ok()) {
+            for (int64_t k = 0; k < n_theta; ++k) grads_out[k] = 0.0;
+            size_t i = 0;
+            for (const SweepPass &p : passes)
+                for (size_t k = 0; k < p.slot.size(); ++k, ++i) {
+                    const auto &tp = term_param[(size_t)p.slot[k]];
+                    const double f = mats[(size_t)tp.first].kind == QI_GATE_P ? -2.0 : 1.0;   // 2 Re <lambda| dU U^dagger |psi>
+                    grads_out[tp.second] += f * p.size2[k] * h[i];
+                }
+        }
+    }
+    const bool swept = tiles && n_theta > 0;
+    if (st.ok() && f32 && !swept) st = state_reduce_norm_sqr(s, &npsi0);
+    if (st.ok() && f32 && !swept && n_terms > 0) st = state_reduce_norm_sqr(lam, &nlam0);
     if (!(npsi0 > 0.0)) npsi0 = 1.0;
     if (!(nlam0 > 0.0)) nlam0 = 1.0;
-    const std::vector<SweepStep> steps = plan_reverse_sweep(mats, resolved, f32, plan_opts.fusion);
+    const std::vector<SweepStep> steps =
+        swept ? std::vector<SweepStep>() : plan_reverse_sweep(mats, resolved, f32, plan_opts.fusion);
     for (size_t si = 0; si < steps.size() && st.ok(); ++si) {
         const int64_t j = steps[si].hi, jj = steps[si].lo;
         const int32_t kind = steps[si].kind;
@@ -1046,7 +1112,7 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
         st = check_launch("k_adjoint");
         for (int q = 0; q < nd; ++q) slot_param.push_back({slot + q, g.param_ids[ids[q]], facg});
     }
-    if (st.ok()) {
+    if (st.ok() && !swept) {
         for (int64_t k = 0; k < n_theta; ++k) grads_out[k] = 0.0;
         std::vector<double> h((size_t)nslots, 0.0);
         if (nslots > 0) e = cudaMemcpyAsync(h.data(), d_gres, (size_t)nslots * sizeof(double), cudaMemcpyDeviceToHost,

@@ -23,7 +23,7 @@
 // Reference: Gate::apply / Circuit::execute (src/components/gate.rs:99-122, src/circuit.rs:160-172),
 // operator.rs:279-2285, PauliString::apply_exp_factor (src/components/pauli_string.rs:237-262).
 #include "qi_gaterun.hpp"
-#include "qi_runtile.cuh"
+#include "qi_runops.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -32,167 +32,6 @@
 #include <unordered_map>
 
 namespace qi {
-
-// ------------------------------------------------------------- program --
-// A pass's program: per phase one 32-byte header, then its operations.  An operation is a 32-byte
-// header and its coefficients; all sizes are multiples of 16 bytes.
-enum RunCode : int {
-    RC_REAL_A = 0,   // a' = a + s u b,      b' = b + s v a
-    RC_REAL_H = 1,   // a' = a + u b,        b' = v a - b
-    RC_REAL_X = 2,   // a' = s b + u a,      b' = v b - s a
-    RC_IMAG_A = 3,   // a' = a + i s u b,    b' = b + i s v a
-    RC_IMAG_X = 4,   // a' = s b + i u a,    b' = s a + i v b
-    RC_REAL_G = 5,   // real 2x2
-    RC_GEN = 6,      // complex 2x2, off-diagonal entries times s
-    RC_PERM = 7,     // exchange
-    RC_PHASE = 8,    // factor = product of what holds: tile factor, thread tables, sub-terms
-    RC_NEG = 9, RC_I = 10, RC_NI = 11,   // factor -1, i, -i
-    RC_PARITY = 12,  // factor c0 (even parity) or c1 (odd)
-    RC_LIFT = 13,    // factor exp(i phi) i^nsub by three shears (c0 = tan(phi/2), c1 = sin(phi))
-    RC_SCALE = 14    // all amplitudes times a real or complex number
-};
-
-struct RunOpHdr {      // 32 bytes
-    uint8_t code, xi, nsub, units;   // xi: register partner mask / AND mask; units: 16-byte size, of the
-                                     // header alone for RC_PHASE (its parts give their own)
-    uint32_t act;      // pairs (bit = index with xi's top bit clear) whose register controls hold
-    uint32_t sgn;      // pairs with a negative sign (before the thread's parity)
-    uint16_t cl, zl;   // local index bits outside the registers: controls, sign parity
-    uint64_t cg, zg;   // the same on the tile's fixed qubits
-};
-struct RunSub {        // 16 bytes, followed by a complex factor padded to 16
-    uint64_t cg;
-    uint32_t cl, pad;
-};
-// RC_PHASE (act, sgn, cl hold other things): act = flags, sgn = 16-byte units of the whole operation,
-// cl = tile slot, zl = number of its tile terms.  Its factor is the product of
-//   kTileFactor: the terms on the tile's fixed qubits, multiplied together once per tile into slot cl,
-//   kLaneTable / kWarpTable: 32 factors by lane / 16 by warp (terms on thread bits, tabulated on the host),
-//   nsub sub-terms with conditions on both (or too few to tabulate).
-// Layout: header, tile terms (RunSub + factor each), sub-terms, lane table, warp table.
-enum RunPhaseFlags : uint32_t { kTileFactor = 1, kLaneTable = 2, kWarpTable = 4 };
-constexpr size_t kRunMaxPhase = 48;   // elements of a phase: with headers, terms and (one per two terms) tables
-                                      // 48 * 96 + 24 * 768 bytes, always less than a pass may hold
-constexpr int kRunMaxSlots = 64;   // tile factors a pass may hold
-static_assert(sizeof(RunOpHdr) == 32 && sizeof(RunSub) == 16, "program layout");
-
-// ------------------------------------------------------------- kernel ---
-// Pair updates on the register pairs (k, k ^ X).  SIGN: off-diagonal terms carry the sign of the
-// pair's Z parity.
-template <typename T, int CODE, int X, bool SIGN>
-__device__ __forceinline__ void run_pair(typename Cx<T>::V2 (&v)[1 << RunShape<T>::kRegBits], uint32_t act, uint32_t sgn,
-                                         const T *c) {
-    using V2 = typename Cx<T>::V2;
-    constexpr int NV = 1 << RunShape<T>::kRegBits;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        if (k & top_bit(X)) continue;
-        if (!((act >> k) & 1u)) continue;
-        V2 &a = v[k], &b = v[k ^ X];
-        const uint32_t s = SIGN ? (sgn >> k) & 1u : 0u;
-        V2 na, nb;
-        if constexpr (CODE == RC_REAL_A) {
-            const T u = SIGN ? flip_sign(c[0], s) : c[0], w = SIGN ? flip_sign(c[1], s) : c[1];
-            na = Cx<T>::make(::fma(u, b.x, a.x), ::fma(u, b.y, a.y));
-            nb = Cx<T>::make(::fma(w, a.x, b.x), ::fma(w, a.y, b.y));
-        } else if constexpr (CODE == RC_REAL_H) {
-            na = Cx<T>::make(::fma(c[0], b.x, a.x), ::fma(c[0], b.y, a.y));
-            nb = Cx<T>::make(::fma(c[1], a.x, -b.x), ::fma(c[1], a.y, -b.y));
-        } else if constexpr (CODE == RC_REAL_X) {
-            const V2 sb = SIGN ? Cx<T>::make(flip_sign(b.x, s), flip_sign(b.y, s)) : b;
-            const V2 sa = SIGN ? Cx<T>::make(flip_sign(a.x, s), flip_sign(a.y, s)) : a;
-            na = Cx<T>::make(::fma(c[0], a.x, sb.x), ::fma(c[0], a.y, sb.y));
-            nb = Cx<T>::make(::fma(c[1], b.x, -sa.x), ::fma(c[1], b.y, -sa.y));
-        } else if constexpr (CODE == RC_IMAG_A) {
-            const T u = SIGN ? flip_sign(c[0], s) : c[0], w = SIGN ? flip_sign(c[1], s) : c[1];
-            na = Cx<T>::make(::fma(-u, b.y, a.x), ::fma(u, b.x, a.y));
-            nb = Cx<T>::make(::fma(-w, a.y, b.x), ::fma(w, a.x, b.y));
-        } else if constexpr (CODE == RC_IMAG_X) {
-            const V2 sb = SIGN ? Cx<T>::make(flip_sign(b.x, s), flip_sign(b.y, s)) : b;
-            const V2 sa = SIGN ? Cx<T>::make(flip_sign(a.x, s), flip_sign(a.y, s)) : a;
-            na = Cx<T>::make(::fma(-c[0], a.y, sb.x), ::fma(c[0], a.x, sb.y));
-            nb = Cx<T>::make(::fma(-c[1], b.y, sa.x), ::fma(c[1], b.x, sa.y));
-        } else if constexpr (CODE == RC_REAL_G) {
-            na = Cx<T>::make(::fma(c[1], b.x, c[0] * a.x), ::fma(c[1], b.y, c[0] * a.y));
-            nb = Cx<T>::make(::fma(c[3], b.x, c[2] * a.x), ::fma(c[3], b.y, c[2] * a.y));
-        } else if constexpr (CODE == RC_GEN) {
-            const V2 m01 = SIGN ? Cx<T>::make(flip_sign(c[2], s), flip_sign(c[3], s)) : Cx<T>::make(c[2], c[3]);
-            const V2 m10 = SIGN ? Cx<T>::make(flip_sign(c[4], s), flip_sign(c[5], s)) : Cx<T>::make(c[4], c[5]);
-            na = Cx<T>::fma(m01, b, Cx<T>::mul(Cx<T>::make(c[0], c[1]), a));
-            nb = Cx<T>::fma(Cx<T>::make(c[6], c[7]), b, Cx<T>::mul(m10, a));
-        } else {
-            na = b;
-            nb = a;
-        }
-        a = na;
-        b = nb;
-    }
-}
-
-// Dispatch on the partner mask: single bits, and with MULTI every mask of two bits (FP64: also
-// all three), the X masks of Pauli exponentials.
-template <typename T, int CODE, bool SIGN>
-__device__ __forceinline__ void run_pair_x(typename Cx<T>::V2 (&v)[1 << RunShape<T>::kRegBits], int xi, uint32_t act,
-                                           uint32_t sgn, const T *c) {
-#define QI_X(M) case M: run_pair<T, CODE, M, SIGN>(v, act, sgn, c); break;
-    constexpr bool f32 = sizeof(T) == 4;
-    switch (xi) {
-        QI_X(1) QI_X(2) QI_X(4)
-    default: break;
-    }
-    if constexpr (f32) {
-        if (xi == 8) run_pair<T, CODE, (f32 ? 8 : 1), SIGN>(v, act, sgn, c);
-    }
-    if constexpr (SIGN) {
-        switch (xi) {
-            QI_X(3) QI_X(5) QI_X(6)
-        default: break;
-        }
-        if constexpr (f32) {
-            if (xi == 9) run_pair<T, CODE, (f32 ? 9 : 1), SIGN>(v, act, sgn, c);
-            if (xi == 10) run_pair<T, CODE, (f32 ? 10 : 1), SIGN>(v, act, sgn, c);
-            if (xi == 12) run_pair<T, CODE, (f32 ? 12 : 1), SIGN>(v, act, sgn, c);
-        } else {
-            if (xi == 7) run_pair<T, CODE, 7, SIGN>(v, act, sgn, c);
-        }
-    }
-#undef QI_X
-}
-
-// Factor on the register amplitudes whose index contains all bits of M.  RC_LIFT: f = (tan(phi/2),
-// sin(phi)); the rotation is three shears, one operation less than a complex product.
-template <typename T, int CODE, int M>
-__device__ __forceinline__ void run_phase(typename Cx<T>::V2 (&v)[1 << RunShape<T>::kRegBits], typename Cx<T>::V2 f) {
-    constexpr int NV = 1 << RunShape<T>::kRegBits;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        if ((k & M) != M) continue;
-        if constexpr (CODE == RC_PHASE) v[k] = Cx<T>::mul(f, v[k]);
-        else if constexpr (CODE == RC_LIFT) {
-            const T x = ::fma(-f.x, v[k].y, v[k].x), y = ::fma(f.y, x, v[k].y);
-            v[k] = Cx<T>::make(::fma(-f.x, y, x), y);
-        }
-        else if constexpr (CODE == RC_NEG) v[k] = Cx<T>::make(-v[k].x, -v[k].y);
-        else if constexpr (CODE == RC_I) v[k] = Cx<T>::make(-v[k].y, v[k].x);
-        else v[k] = Cx<T>::make(v[k].y, -v[k].x);
-    }
-}
-template <typename T, int CODE>
-__device__ __forceinline__ void run_phase_m(typename Cx<T>::V2 (&v)[1 << RunShape<T>::kRegBits], int m,
-                                            typename Cx<T>::V2 f) {
-#define QI_M(M) case M: run_phase<T, CODE, M>(v, f); break;
-    switch (m) {
-        QI_M(0) QI_M(1) QI_M(2) QI_M(3) QI_M(4) QI_M(5) QI_M(6) QI_M(7)
-    default: break;
-    }
-    if constexpr (sizeof(T) == 4) {
-        switch (m) {
-            QI_M(8) QI_M(9) QI_M(10) QI_M(11) QI_M(12) QI_M(13) QI_M(14) QI_M(15)
-        default: break;
-        }
-    }
-#undef QI_M
-}
 
 struct RunGeom {
     int32_t tbits, low;
@@ -203,7 +42,7 @@ struct RunGeom {
 
 // Shared memory: tile | offsets of the tile's rows | program.
 template <typename T>
-__global__ void __launch_bounds__(256) k_gate_run(typename Cx<T>::V2 *amps, const uint4 *prog, const __grid_constant__ RunGeom g) {
+__global__ void __launch_bounds__(256, 3) k_gate_run(typename Cx<T>::V2 *amps, const uint4 *prog, const __grid_constant__ RunGeom g) {
     using V2 = typename Cx<T>::V2;
     constexpr int RB = RunShape<T>::kRegBits, NV = 1 << RB, UB0 = RunShape<T>::kUnitBits;
     extern __shared__ uint4 sm[];
@@ -314,7 +153,7 @@ __global__ void __launch_bounds__(256) k_gate_run(typename Cx<T>::V2 *amps, cons
                 break;
             case RC_REAL_G: run_pair_x<T, RC_REAL_G, false>(v, xi, act, sgn, c); break;
             case RC_GEN: run_pair_x<T, RC_GEN, true>(v, xi, act, sgn, c); break;
-            case RC_PERM: run_pair_x<T, RC_PERM, false>(v, xi, act, sgn, c); break;
+            case RC_PERM: run_perm_x<T>(v, xi, 255, act); break;   // one form: less code beats fewer selects
             case RC_LIFT:
                 run_phase_m<T, RC_LIFT>(v, xi, Cx<T>::make(c[0], c[1]));
                 if (nsub == 1) run_phase_m<T, RC_I>(v, xi, Cx<T>::make(T(0), T(0)));
@@ -435,6 +274,7 @@ struct RunElem {
     double c[8] = {0};
     CDD f;                           // RC_PHASE: the factor
     CDD scale;                       // left to the run's global factor
+    int der = 0, slot = -1;          // SweepDer of a parametric gate of a reverse sweep, and its slot
     bool rot = false;                // rc + rs P' with P' P' = -1: exp(i angle P), P = (xmask, zmask)
     DD rc, rs;
     bool diag() const { return xs == 0; }
@@ -553,17 +393,59 @@ struct Lowering {
             return rotation(x, 0, false, m[0], m[3]);
         pair(RC_GEN, x, 0, ctl, {m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7]});
     }
+    // The ratio t of a scaled rotation's entries and its scale (first: the entry that becomes 1).  FP32
+    // states: the scale of the rounded t, so that what is applied is a multiple of a unitary exactly.
+    double ratio(const DD &other, const DD &first, DD &scale) const {
+        const double t = dd_div(other, first).h;
+        scale = first;
+        if (prec != QI_F32) return t;
+        const double r = (double)(float)t;
+        scale = DD(std::copysign(1.0 / std::sqrt(1.0 + r * r), first.h));
+        return r;
+    }
     // odd = false: a' = c a + i s sigma b, b' = c b + i s sigma a; odd = true: a' = c a + s sigma b,
     // b' = c b - s sigma a.  The larger entry becomes the scale.
     void rotation(uint64_t x, uint64_t z, bool odd, const DD &c, const DD &s) {
+        DD f;
         if (std::fabs(c.h) >= std::fabs(s.h)) {
-            const double t = dd_div(s, c).h;
-            pair(odd ? RC_REAL_A : RC_IMAG_A, x, z, 0, {t, odd ? -t : t}, CDD(c, DD()));
+            const double t = ratio(s, c, f);
+            pair(odd ? RC_REAL_A : RC_IMAG_A, x, z, 0, {t, odd ? -t : t}, CDD(f, DD()));
         } else {
-            const double t = dd_div(c, s).h;
-            if (odd) pair(RC_REAL_X, x, z, 0, {t, t}, CDD(s, DD()));
-            else pair(RC_IMAG_X, x, z, 0, {-t, -t}, CDD(DD(), s));
+            const double t = ratio(c, s, f);
+            if (odd) pair(RC_REAL_X, x, z, 0, {t, t}, CDD(f, DD()));
+            else pair(RC_IMAG_X, x, z, 0, {-t, -t}, CDD(DD(), f));
         }
+    }
+    // diag(c + i s, c - i s) on qubit q
+    void rotation_z(int q, const DD &c, const DD &s) {
+        RunElem e;
+        DD f;
+        e.zs = e.zmask = 1ull << q;
+        if (std::fabs(c.h) >= std::fabs(s.h)) {
+            e.code = RC_ROTZ_A;
+            e.c[0] = ratio(s, c, f);
+            e.scale = CDD(f, DD());
+        } else {
+            e.code = RC_ROTZ_X;
+            e.c[0] = ratio(c, s, f);
+            e.scale = CDD(f, DD());
+        }
+        push(e);
+    }
+    // The inverse of an uncontrolled parametric gate; its derivative term goes to `slot`.
+    void unapply(const GateMatrix &g, int slot) {
+        const uint64_t x = 1ull << g.t[0];
+        switch (g.kind) {
+        case QI_GATE_RX: rotation(x, 0, false, g.m[0], -g.m[3]); break;
+        case QI_GATE_RY: rotation(x, 0, true, g.m[0], g.m[4]); break;
+        case QI_GATE_RZ: rotation_z(g.t[0], g.m[6], g.m[7]); break;
+        default: {   // P: half the angle each way, up to a phase psi and lambda share
+            const double h = 0.5 * std::atan2(g.m[7], g.m[6]);
+            rotation_z(g.t[0], std::cos(h), std::sin(h));
+        }
+        }
+        out.back().der = g.kind == QI_GATE_RX ? kDerX : g.kind == QI_GATE_RY ? kDerY : g.kind == QI_GATE_RZ ? kDerZ : kDerP;
+        out.back().slot = slot;
     }
     void pauli(const GateMatrix &g) {   // exp(alpha P)
         const double ar = g.alpha_re, ai = g.alpha_im;
@@ -713,6 +595,7 @@ uint64_t best_bits(const std::vector<Masks> &rem, uint64_t W0, const std::vector
 struct Encoder {
     int n, prec, ub0;
     RunPass *pass;
+    std::vector<int32_t> *der = nullptr;   // slots of the pass's derivative terms, in program order
     std::vector<uint8_t> &prog;
     uint64_t localmask = 0;
     int lbit[64];   // qubit -> local bit or -1
@@ -914,6 +797,7 @@ struct Encoder {
             o.h.cg = out;
             for (int k = 0; k < nv; ++k)
                 if (((uint32_t)k & reg) == reg) o.h.act |= 1u << k;
+            if (e.code == RC_PERM) o.h.nsub = (uint8_t)((reg & (reg - 1)) ? 255u : reg);
             split(e.xmask, rmap, reg, loc, out);
             o.h.xi = (uint8_t)reg;
             // sign parity is taken on the partner with the highest qubit of xmask clear: the register
@@ -923,11 +807,18 @@ struct Encoder {
             o.h.zg = out;
             for (int k = 0; k < nv; ++k)
                 if (__builtin_popcount((uint32_t)k & reg) & 1) o.h.sgn |= 1u << k;
+            if (e.code == RC_ROTZ_A || e.code == RC_ROTZ_X) o.h.xi = (uint8_t)reg;
             switch (e.code) {
             case RC_REAL_A: case RC_REAL_H: case RC_REAL_X: case RC_IMAG_A: case RC_IMAG_X: o.nc = 2; break;
             case RC_REAL_G: case RC_PARITY: o.nc = 4; break;
             case RC_GEN: o.nc = 8; break;
+            case RC_ROTZ_A: case RC_ROTZ_X: o.nc = 1; break;
             default: break;
+            }
+            if (e.der) {   // uncontrolled: cg holds the term's place
+                o.h.nsub = (uint8_t)e.der;
+                o.h.cg = der->size();
+                der->push_back(e.slot);
             }
             std::copy(e.c, e.c + 8, o.c);
         }
@@ -977,19 +868,17 @@ static int run_tile_units(int n, int ub0) {
     return std::min(u, ub0 && n >= 20 ? 11 : 10);
 }
 
-void schedule_run(int n, int prec, const std::vector<const Elem *> &elems, RunSegment &seg, std::vector<uint8_t> &prog) {
-    Lowering lw(prec);
+// The greedy schedule of E into passes.  sweep: reverse-sweep passes (each pass's derivative terms, with
+// the squared size of the scales left out when they are taken); no global factor at the end.
+static void schedule_elems(int n, int prec, const std::vector<RunElem> &E, CDD scalar, int tbits, std::vector<RunPass> *passes,
+                           std::vector<SweepPass> *sweep, std::vector<uint8_t> &prog) {
     const int ub0 = prec == QI_F32 ? 1 : 0;
-    for (const Elem *e : elems) lw.add(*e);
-    const std::vector<RunElem> &E = lw.out;
-    const int tbits = run_tile_units(n, ub0) + ub0;
     const int low = tbits >= n ? n : 3 + ub0;   // rows of 128 bytes (rows of 512: up to 10 % slower, more passes)
     const uint64_t lowmask = (1ull << low) - 1, always = ub0 ? 1ull : 0ull;
     // The product of the scales left out so far; it is applied at the end of the run, or earlier
     // when it has become small (the amplitudes grow as its reciprocal).
-    CDD scalar = lw.scalar;
     const double small = prec == QI_F32 ? 0x1p-30 : 0x1p-300;
-    if (E.empty() && scalar.one()) return;
+    if (E.empty() && (sweep || scalar.one())) return;
     std::vector<int> rem(E.size()), take, ptake, inner, group, rest, free_q, sel_q;
     std::vector<Masks> masks(E.size()), imasks;
     for (size_t i = 0; i < E.size(); ++i) {
@@ -1010,6 +899,8 @@ void schedule_run(int n, int prec, const std::vector<const Elem *> &elems, RunSe
             inner = rem;
         }
         RunPass pass;
+        SweepPass terms;
+        enc.der = &terms.slot;
         pass.tbits = tbits;
         int np = 0;
         sel_q.clear();
@@ -1031,16 +922,21 @@ void schedule_run(int n, int prec, const std::vector<const Elem *> &elems, RunSe
             if (ptake.size() > kRunMaxPhase) ptake.resize(kRunMaxPhase);
             for (int i : ptake) group.push_back(inner[(size_t)i]);
             CDD after = scalar;
-            for (int i : group)
+            for (int i : group) {
+                if (E[(size_t)i].der) terms.size2.push_back(std::norm(after.value()));
                 if (!E[(size_t)i].scale.one()) after = after * E[(size_t)i].scale;
-            const bool last = ndone + group.size() == rem.size();
+            }
+            const bool last = !sweep && ndone + group.size() == rem.size();
             const cd now = after.value();
             const bool apply = (last && !after.one()) || std::abs(now) < small;
-            const size_t used = prog.size(), slots = pass.slot_at.size();
+            const size_t used = prog.size(), slots = pass.slot_at.size(), nder = terms.slot.size();
             enc.phase(E, group, R, apply ? &now : nullptr);
-            if (prog.size() - (size_t)pass.prog_off > (size_t)kRunMaxProg) {   // left to the next pass
+            if (prog.size() - (size_t)pass.prog_off > (size_t)kRunMaxProg || (sweep && terms.slot.size() > (size_t)kSweepTerms) ||
+                (sweep && pass.nphase > kSweepPhases)) {   // left to the next pass
                 prog.resize(used);
                 pass.slot_at.resize(slots);
+                terms.slot.resize(nder);
+                terms.size2.resize(nder);
                 --pass.nphase;
                 break;
             }
@@ -1057,7 +953,12 @@ void schedule_run(int n, int prec, const std::vector<const Elem *> &elems, RunSe
             imasks.resize(k);
         } while (!inner.empty());
         pass.prog_bytes = (int32_t)(prog.size() - (size_t)pass.prog_off);
-        seg.passes.push_back(pass);
+        if (sweep) {
+            terms.run = std::move(pass);
+            sweep->push_back(std::move(terms));
+        } else {
+            passes->push_back(std::move(pass));
+        }
         size_t k = 0;
         for (size_t i = 0; i < rem.size(); ++i)
             if (!gone[(size_t)rem[i]]) {
@@ -1067,6 +968,62 @@ void schedule_run(int n, int prec, const std::vector<const Elem *> &elems, RunSe
         rem.resize(k);
         masks.resize(k);
     } while (!rem.empty());
+}
+
+void schedule_run(int n, int prec, const std::vector<const Elem *> &elems, RunSegment &seg, std::vector<uint8_t> &prog) {
+    Lowering lw(prec);
+    const int ub0 = prec == QI_F32 ? 1 : 0;
+    for (const Elem *e : elems) lw.add(*e);
+    schedule_elems(n, prec, lw.out, lw.scalar, run_tile_units(n, ub0) + ub0, &seg.passes, nullptr, prog);
+}
+
+bool sweep_supported(int n, int prec, const GateMatrix &g, int nparams) {
+    if (n < kRunSelBits + (prec == QI_F32 ? 1 : 0) || g.pauli || g.measure || g.normalise_after) return false;
+    if (nparams) {
+        const bool kind = g.kind == QI_GATE_RX || g.kind == QI_GATE_RY || g.kind == QI_GATE_RZ || g.kind == QI_GATE_P;
+        return nparams == 1 && kind && g.nt == 1 && g.controls.empty() && finite_all(g.m, 8);
+    }
+    if (g.nt == 0) return true;
+    if (g.nt == 2) return g.kind == QI_GATE_SWAP;
+    return finite_all(g.m, 8);
+}
+
+void schedule_sweep(int n, int prec, const std::vector<SweepGate> &gates, std::vector<SweepPass> &passes,
+                    std::vector<uint8_t> &prog) {
+    Lowering lw(prec);
+    const int ub0 = prec == QI_F32 ? 1 : 0;
+    for (const SweepGate &sg : gates) {
+        const GateMatrix &g = *sg.g;
+        if (sg.slot >= 0) {
+            lw.unapply(g, sg.slot);
+            continue;
+        }
+        if (g.nt == 0) continue;
+        if (prec == QI_F32 && g.nt == 1 && g.controls.empty() && g.diagonal) {
+            // a fixed phase as the same exact multiple of a unitary (up to a phase both states share);
+            // quarter turns stay exact factors
+            const cd r = std::conj(cdd_div(CDD(cd(g.m[6], g.m[7])), CDD(cd(g.m[0], g.m[1]))).value());
+            const bool quarter = r == cd(1, 0) || r == cd(-1, 0) || r == cd(0, 1) || r == cd(0, -1);
+            if (!quarter && std::fabs(std::norm(r) - 1.0) < 1e-12) {
+                const double h = -0.5 * std::arg(r);
+                lw.rotation_z(g.t[0], std::cos(h), std::sin(h));
+                continue;
+            }
+        }
+        Elem e;
+        e.gm = g;
+        if (g.nt == 1)
+            for (int i = 0; i < 2; ++i)
+                for (int j = 0; j < 2; ++j) {
+                    e.gm.m[2 * (2 * i + j)] = g.m[2 * (2 * j + i)];
+                    e.gm.m[2 * (2 * i + j) + 1] = -g.m[2 * (2 * j + i) + 1];
+                }
+        lw.add(e);
+    }
+    // 12-layer ansatz, ms with tiles of 2^9 / 2^10 / 2^11 units: FP32 20 qubits 5.1 / 4.3 / 4.2, 22 qubits
+    // 9.2 / 7.8 / 7.2 (larger blocks share the instruction stream); FP64 16 qubits, 8 layers 4.1 / 3.9 / 4.2
+    const int units = std::min(n - ub0, prec == QI_F32 && n >= 20 ? 11 : 10);
+    schedule_elems(n, prec, lw.out, CDD(), units + ub0, nullptr, &passes, prog);
 }
 
 // -------------------------------------------------------------- replay --
