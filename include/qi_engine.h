@@ -95,6 +95,10 @@ typedef struct qi_state qi_state;
  * Errors: InvalidNumberOfQubits(0) for num_qubits == 0 (state.rs:166-168). */
 qi_status qi_state_create(int32_t num_qubits, int32_t precision, qi_state **out);
 qi_status qi_state_destroy(qi_state *s);
+/* Destroyed handles of small states are kept for the next handle of the same size, precision and device
+ * (at most 64 of them, 64 MiB in all; none whose device pointer or stream was handed out).  Frees them;
+ * an allocation of the engine that fails does the same before it gives up. */
+qi_status qi_cache_trim(void);
 qi_status qi_state_info(const qi_state *s, int32_t *num_qubits, int32_t *precision);
 /* Run this handle's work on an external CUDA stream (a cudaStream_t passed as
  * void*); NULL restores the handle's own stream. */
@@ -232,6 +236,9 @@ qi_status qi_apply_gate(qi_state *s, const qi_gate *g);
  * unitarity check.  use_tensor_cores as in qi_exec_options. */
 qi_status qi_apply_matrix(qi_state *s, const int32_t *targets, int32_t k, const double *matrix,
                           int32_t use_tensor_cores);
+/* `Operator::apply` returning a new state (operator.rs:151-190): dst = gate applied to src (same number
+ * of qubits), in one pass for one-target gates.  Same checks and errors as qi_apply_gate. */
+qi_status qi_apply_gate_to(qi_state *dst, const qi_state *src, const qi_gate *gate);
 /* `Unitary2::new` unitarity check (operator.rs:2092-2125), tol 2*eps. */
 qi_status qi_unitary2_check(const double m[8]);
 

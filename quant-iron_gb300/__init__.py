@@ -33,6 +33,11 @@ def version():
     return lib.qi_version().decode()
 
 
+def trim_cache():
+    """Free the device memory of destroyed small states that is kept for new ones."""
+    check(lib.qi_cache_trim())
+
+
 def _as_c128(v):
     v = np.ascontiguousarray(v, dtype=np.complex128)
     return v
@@ -55,6 +60,11 @@ class DeviceState:
         if self.h:
             lib.qi_state_destroy(self.h)
             self.h = ctypes.c_void_p()
+
+    def apply_gate_from(self, other, gate_row):
+        """This state = the gate applied to `other`."""
+        g = np.ascontiguousarray(gate_row, dtype=GATE_DTYPE).reshape(())
+        check(lib.qi_apply_gate_to(self.h, other.h, g.ctypes.data))
 
     def release(self):
         """Hand the handle to a new owner: returns a DeviceState owning it and leaves this

@@ -96,6 +96,8 @@ SIGNATURES = {
     "qi_plan_stats_get": (_i32, [_vp, ctypes.POINTER(PlanStats)]),
     "qi_plan_destroy": (_i32, [_vp]),
     "qi_plan_num_ops": (_i32, [_vp, ctypes.POINTER(_i64)]),
+    "qi_apply_gate_to": (_i32, [_vp, _vp, _vp]),
+    "qi_cache_trim": (_i32, []),
     "qi_plan_run_info": (_i32, [_vp, ctypes.POINTER(_i64), ctypes.POINTER(_i64), ctypes.POINTER(_i64)]),
     "qi_plan_run_replay": (_i32, [_vp, _vp]),
     "qi_plan_op_get": (_i32, [_vp, _i64, ctypes.POINTER(PlanOpInfo), _pd, _i64]),

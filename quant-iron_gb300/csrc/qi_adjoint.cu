@@ -740,24 +740,37 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
     // psi_0 stays untouched in the caller's buffer: the sweep runs on a copy (un-applying psi in
     // FP32 would hand back psi_0 with the sweep's rounding in it); without room for the copy it
     // runs in place and psi_0 is restored by the sweep itself.
+    // A scratch handle's buffers are used on s's stream, behind what its own stream still holds.
+    auto join = [&](qi_state *q) {
+        cudaError_t je = cudaEventRecord(q->ev, q->own_stream);
+        if (je == cudaSuccess) je = cudaStreamWaitEvent(s->stream, q->ev, 0);
+        q->stream = s->stream;
+        return je;
+    };
+    auto give_back = [&](qi_state *q) {   // s's stream has been waited for
+        q->stream = q->own_stream;
+        qi_state_destroy(q);
+    };
     void *const psi_home = s->amps;
-    void *work = nullptr;
-    if (cudaMalloc(&work, s->bytes()) == cudaSuccess) {
-        e = cudaMemcpyAsync(work, psi_home, s->bytes(), cudaMemcpyDeviceToDevice, s->stream);
+    qi_state *work = nullptr;
+    if (qi_state_create(n, s->prec, &work) == QI_OK) {
+        e = join(work);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(work->amps, psi_home, s->bytes(), cudaMemcpyDeviceToDevice, s->stream);
         if (e != cudaSuccess) {
-            cudaFree(work);
+            cudaStreamSynchronize(s->stream);
+            give_back(work);
             return publish(cuda_status(e, "copy psi_0"));
         }
-        s->amps = work;
+        s->amps = work->amps;
     } else {
         work = nullptr;
         cudaGetLastError();
     }
     auto bail = [&](Status st) {   // before lambda exists: psi is in `work` (or in place)
+        cudaStreamSynchronize(s->stream);
         if (work) {
-            cudaStreamSynchronize(s->stream);
-            cudaFree(s->amps);
             s->amps = psi_home;
+            give_back(work);
         }
         return publish(st);
     };
@@ -786,11 +799,11 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
     qi_state *lam = nullptr;
     qi_status cs = qi_state_create(n, s->prec, &lam);
     if (cs != QI_OK) return bail(err(cs, -1, -1, "lambda state"));
-    qi_state_set_stream(lam, s->stream);
     Status st = ok_status();
+    if ((e = join(lam)) != cudaSuccess) st = cuda_status(e, "lambda state");
     double ev[2] = {0, 0};
     if (n_terms > 0) {
-        st = sumop_apply(lam, s, terms, n_terms);
+        if (st.ok()) st = sumop_apply(lam, s, terms, n_terms);
         if (st.ok()) st = state_inner(s, lam, ev);
         int flag = 0;
         if (st.ok()) st = state_read_flag(lam, &flag);
@@ -802,10 +815,6 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
     // derivative slots (one per parameter of a gate; a gate group uses one per member)
     const int64_t nslots = 3 * n_gates + kMultiComps;
     double *d_gres = nullptr;
-    if (st.ok() && nslots > 0) {
-        e = cudaMalloc(&d_gres, (size_t)nslots * sizeof(double));
-        if (e != cudaSuccess) st = cuda_status(e, "cudaMalloc(gradient slots)");
-    }
     struct SlotParam {
         int64_t slot;
         int32_t param;
@@ -879,6 +888,10 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
         }
     }
     const bool swept = tiles && n_theta > 0;
+    if (st.ok() && !swept && nslots > 0) {
+        e = cudaMalloc(&d_gres, (size_t)nslots * sizeof(double));
+        if (e != cudaSuccess) st = cuda_status(e, "cudaMalloc(gradient slots)");
+    }
     if (st.ok() && f32 && !swept) st = state_reduce_norm_sqr(s, &npsi0);
     if (st.ok() && f32 && !swept && n_terms > 0) st = state_reduce_norm_sqr(lam, &nlam0);
     if (!(npsi0 > 0.0)) npsi0 = 1.0;
@@ -990,7 +1003,7 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
         if (kind == kSweepAffine) {
             // X / CNOT / SWAP only: one index permutation per state, out[x] = in[f(x)] with f the
             // run's forward map (gathering through f un-applies the run)
-            if (!scratch && cudaMalloc(&scratch, s->bytes()) != cudaSuccess) {
+            if (!scratch && device_malloc(&scratch, s->bytes()) != cudaSuccess) {
                 scratch = nullptr;
                 cudaGetLastError();   // no room for a third state buffer: un-apply the run as a plan
                 as_plan = true;
@@ -1123,8 +1136,9 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
     }
     cudaStreamSynchronize(s->stream);
     if (work) {   // psi_0 never left the caller's buffer; psi ends in one of the sweep's buffers
-        cudaFree(s->amps);
+        work->amps = s->amps;
         s->amps = psi_home;
+        give_back(work);
     } else if (s->amps != psi_home) {   // psi_home is lambda's or the scratch buffer now
         e = cudaMemcpyAsync(psi_home, s->amps, s->bytes(), cudaMemcpyDeviceToDevice, s->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
@@ -1140,6 +1154,6 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
         release_runs(sp.get());
     }
     if (d_gres) cudaFree(d_gres);
-    qi_state_destroy(lam);
+    give_back(lam);
     return publish(st);
 }

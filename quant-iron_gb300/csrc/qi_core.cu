@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <vector>
 
 namespace qi {
 
@@ -434,7 +435,7 @@ Status state_normalise_to_from_partials_async(qi_state *s, void *out, const void
 
 Status state_scratch(qi_state *s, void **out) {
     if (!s->d_scratch) {
-        cudaError_t e = cudaMalloc(&s->d_scratch, s->bytes());
+        cudaError_t e = device_malloc(&s->d_scratch, s->bytes());
         if (e != cudaSuccess) {
             s->d_scratch = nullptr;
             cudaGetLastError();   // clear the allocation error: the caller falls back
@@ -445,20 +446,135 @@ Status state_scratch(qi_state *s, void **out) {
     return ok_status();
 }
 
-Status state_workspace(qi_state *s, size_t bytes, void **out) {
-    if (s->work_bytes < bytes) {
+Status read_begin(qi_state *dst, const qi_state *src) {
+    if (src->stream == dst->stream) return ok_status();
+    QI_CUDA(cudaEventRecord(src->ev, src->stream));
+    QI_CUDA(cudaStreamWaitEvent(dst->stream, src->ev, 0));
+    return ok_status();
+}
+
+Status read_end(qi_state *dst, const qi_state *src) {
+    if (src->stream == dst->stream) return ok_status();
+    QI_CUDA(cudaEventRecord(dst->ev, dst->stream));
+    QI_CUDA(cudaStreamWaitEvent(src->stream, dst->ev, 0));
+    return ok_status();
+}
+
+// ------------------------------------------------------------ handle cache --
+// A handle costs a stream, an event, three allocations and a page-locked one (about 60 us to make, and
+// frees wait for the device): programs that make a new small state per operation spend their time
+// there.  Destroyed handles of up to kCacheState bytes are kept, at most kCacheHandles of them and
+// kCacheBytes in all (the oldest goes first), and taken over by the next handle of the same size,
+// precision and device.  The new owner works on the same stream, so its work is ordered behind
+// whatever the old owner and the readers of its buffer (read_end) still have in flight.  Handles whose
+// buffer or stream was handed out are freed as ever; a handle that moved host data is waited for.
+// An allocation that fails empties the cache first; qi_cache_trim does so on request.
+constexpr size_t kCacheState = 8u << 20, kCacheBytes = 64u << 20;
+constexpr size_t kCacheHandles = 64;
+namespace {
+struct HandleCache {
+    std::mutex mu;
+    std::vector<qi_state *> kept;   // oldest first
+    size_t bytes = 0;
+};
+HandleCache &cache() {
+    static HandleCache *c = new HandleCache();   // never destroyed: the driver may be gone at exit
+    return *c;
+}
+size_t held_bytes(const qi_state *s) {
+    return s->bytes() + (s->d_scratch ? s->bytes() : 0) + s->staging_bytes + s->work_bytes + s->prog_bytes;
+}
+void free_handle(qi_state *s) {
+    cudaSetDevice(s->device);
+    cudaStreamSynchronize(s->stream);
+    if (s->own_stream && s->own_stream != s->stream) cudaStreamSynchronize(s->own_stream);
+    if (s->amps) cudaFree(s->amps);
+    if (s->d_partials) cudaFree(s->d_partials);   // d_result and d_flag lie behind it
+    if (s->h_result) cudaFreeHost(s->h_result);
+    if (s->d_staging) cudaFree(s->d_staging);
+    if (s->d_scratch) cudaFree(s->d_scratch);
+    if (s->d_work) cudaFree(s->d_work);
+    if (s->d_prog) cudaFree(s->d_prog);
+    if (s->link_stream) {
+        cudaStreamSynchronize(s->link_stream);
+        cudaStreamDestroy(s->link_stream);
+    }
+    for (cudaEvent_t e : s->link_ev)
+        if (e) cudaEventDestroy(e);
+    if (s->ev) cudaEventDestroy(s->ev);
+    if (s->own_stream) cudaStreamDestroy(s->own_stream);
+    delete s;
+}
+qi_state *cache_take(int n, int prec, int device) {
+    HandleCache &c = cache();
+    std::lock_guard<std::mutex> lk(c.mu);
+    for (size_t i = c.kept.size(); i-- > 0;) {
+        qi_state *s = c.kept[i];
+        if (s->n != n || s->prec != prec || s->device != device) continue;
+        c.kept.erase(c.kept.begin() + (long)i);
+        c.bytes -= held_bytes(s);
+        return s;
+    }
+    return nullptr;
+}
+bool cache_put(qi_state *s) {   // false: not cacheable
+    if (s->exposed || s->link_stream || s->stream != s->own_stream || s->bytes() > kCacheState) return false;
+    if (held_bytes(s) > 2 * kCacheState) return false;
+    if (s->host_io && cudaStreamSynchronize(s->stream) != cudaSuccess) return false;
+    std::vector<qi_state *> out;
+    {
+        HandleCache &c = cache();
+        std::lock_guard<std::mutex> lk(c.mu);
+        c.kept.push_back(s);
+        c.bytes += held_bytes(s);
+        while (c.kept.size() > kCacheHandles || c.bytes > kCacheBytes) {
+            out.push_back(c.kept.front());
+            c.bytes -= held_bytes(c.kept.front());
+            c.kept.erase(c.kept.begin());
+        }
+    }
+    for (qi_state *o : out) free_handle(o);
+    return true;
+}
+void cache_clear() {
+    std::vector<qi_state *> out;
+    {
+        HandleCache &c = cache();
+        std::lock_guard<std::mutex> lk(c.mu);
+        out.swap(c.kept);
+        c.bytes = 0;
+    }
+    int dev = 0;
+    const bool have = cudaGetDevice(&dev) == cudaSuccess;
+    for (qi_state *o : out) free_handle(o);
+    if (have) cudaSetDevice(dev);
+}
+}  // namespace
+
+cudaError_t device_malloc(void **p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    (void)cudaGetLastError();
+    cache_clear();
+    return cudaMalloc(p, bytes);
+}
+
+Status state_workspace(qi_state *s, size_t bytes, void **out, bool program) {
+    void *&have = program ? s->d_prog : s->d_work;
+    size_t &have_bytes = program ? s->prog_bytes : s->work_bytes;
+    if (have_bytes < bytes) {
         const size_t want = std::max<size_t>(bytes + bytes / 2, 64 * 1024);
         void *p = nullptr;
-        cudaError_t e = cudaMalloc(&p, want);
+        cudaError_t e = device_malloc(&p, want);
         if (e != cudaSuccess) {
             (void)cudaGetLastError();
             return cuda_status(e, "cudaMalloc(workspace)");
         }
-        if (s->d_work) cudaFree(s->d_work);
-        s->d_work = p;
-        s->work_bytes = want;
+        if (have) cudaFree(have);
+        have = p;
+        have_bytes = want;
     }
-    *out = s->d_work;
+    *out = have;
     return ok_status();
 }
 
@@ -473,10 +589,11 @@ Status state_read_flag(qi_state *s, int *flag) {
 
 Status state_copy_async(qi_state *dst, const qi_state *src) {
     if (dst->n != src->n) return err(QI_ERR_INVALID_NUMBER_OF_QUBITS, src->n, -1);
-    if (src->stream != dst->stream) QI_CUDA(cudaStreamSynchronize(src->stream));
+    Status st = read_begin(dst, src);
+    if (!st.ok()) return st;
     if (dst->prec == src->prec) {
         QI_CUDA(cudaMemcpyAsync(dst->amps, src->amps, src->bytes(), cudaMemcpyDeviceToDevice, dst->stream));
-        return ok_status();
+        return read_end(dst, src);
     }
     unsigned g = grid_for(src->dim());
     if (dst->prec == QI_F32)
@@ -484,13 +601,14 @@ Status state_copy_async(qi_state *dst, const qi_state *src) {
     else
         k_convert<double, float><<<g, 256, 0, dst->stream>>>((double2 *)dst->amps, (const float2 *)src->amps, src->dim());
     count_launch();
-    return check_launch("k_convert");
+    st = check_launch("k_convert");
+    return st.ok() ? read_end(dst, src) : st;
 }
 
 static Status ensure_staging(qi_state *s, size_t bytes) {
     if (s->staging_bytes >= bytes) return ok_status();
     if (s->d_staging) { cudaFree(s->d_staging); s->d_staging = nullptr; s->staging_bytes = 0; }
-    QI_CUDA(cudaMalloc(&s->d_staging, bytes));
+    QI_CUDA(device_malloc(&s->d_staging, bytes));
     s->staging_bytes = bytes;
     return ok_status();
 }
@@ -564,31 +682,39 @@ qi_status qi_state_create(int32_t num_qubits, int32_t precision, qi_state **out)
     if (num_qubits <= 0) return publish(err(QI_ERR_INVALID_NUMBER_OF_QUBITS, num_qubits < 0 ? 0 : num_qubits));
     if (num_qubits > 40) return publish(err(QI_ERR_INVALID_NUMBER_OF_QUBITS, num_qubits));
     if (precision != QI_F32 && precision != QI_F64) return publish(err(QI_ERR_INVALID_INPUT_VALUE, precision));
+    cudaError_t e = cudaSetDevice(g_device);
+    if (e != cudaSuccess) return publish(cuda_status(e, "cudaSetDevice"));
+    if (qi_state *s = cache_take(num_qubits, precision, g_device)) {
+        s->host_io = false;
+        if ((e = cudaMemsetAsync(s->d_flag, 0, sizeof(int), s->stream)) != cudaSuccess) {
+            free_handle(s);
+            return publish(cuda_status(e, "memset"));
+        }
+        *out = s;
+        return publish(ok_status());
+    }
     qi_state *s = new qi_state();
     s->n = num_qubits;
     s->prec = precision;
     s->device = g_device;
     auto fail = [&](Status st) {
-        if (s->amps) cudaFree(s->amps);
-        if (s->d_partials) cudaFree(s->d_partials);
-        if (s->d_result) cudaFree(s->d_result);
-        if (s->h_result) cudaFreeHost(s->h_result);
-        if (s->d_flag) cudaFree(s->d_flag);
-        if (s->own_stream) cudaStreamDestroy(s->own_stream);
-        delete s;
+        free_handle(s);
         return publish(st);
     };
-    cudaError_t e;
-    if ((e = cudaSetDevice(s->device)) != cudaSuccess) return fail(cuda_status(e, "cudaSetDevice"));
     if ((e = cudaStreamCreateWithFlags(&s->own_stream, cudaStreamNonBlocking)) != cudaSuccess)
         return fail(cuda_status(e, "cudaStreamCreate"));
     s->stream = s->own_stream;
-    if ((e = cudaMalloc(&s->amps, s->bytes())) != cudaSuccess) return fail(cuda_status(e, "cudaMalloc(state)"));
-    if ((e = cudaMalloc(&s->d_partials, kReduceBlocks * 4 * sizeof(double))) != cudaSuccess)
-        return fail(cuda_status(e, "cudaMalloc(partials)"));
-    if ((e = cudaMalloc(&s->d_result, 8 * sizeof(double))) != cudaSuccess) return fail(cuda_status(e, "cudaMalloc"));
+    if ((e = cudaEventCreateWithFlags(&s->ev, cudaEventDisableTiming)) != cudaSuccess)
+        return fail(cuda_status(e, "cudaEventCreate"));
+    if ((e = device_malloc(&s->amps, s->bytes())) != cudaSuccess) return fail(cuda_status(e, "cudaMalloc(state)"));
+    // one block: partials, results, error flag
+    constexpr size_t parts = kReduceBlocks * 4 * sizeof(double);
+    void *small = nullptr;
+    if ((e = device_malloc(&small, parts + 128)) != cudaSuccess) return fail(cuda_status(e, "cudaMalloc(partials)"));
+    s->d_partials = (double *)small;
+    s->d_result = (double *)((char *)small + parts);
+    s->d_flag = (int *)((char *)small + parts + 64);
     if ((e = cudaMallocHost(&s->h_result, 8 * sizeof(double))) != cudaSuccess) return fail(cuda_status(e, "cudaMallocHost"));
-    if ((e = cudaMalloc(&s->d_flag, sizeof(int))) != cudaSuccess) return fail(cuda_status(e, "cudaMalloc"));
     if ((e = cudaMemsetAsync(s->d_flag, 0, sizeof(int), s->stream)) != cudaSuccess) return fail(cuda_status(e, "memset"));
     *out = s;
     return publish(ok_status());
@@ -599,25 +725,14 @@ qi_status qi_state_destroy(qi_state *s) {
     {
         std::lock_guard<std::recursive_mutex> lk(s->mu);
         cudaSetDevice(s->device);
-        cudaStreamSynchronize(s->stream);
-        if (s->amps) cudaFree(s->amps);
-        if (s->d_partials) cudaFree(s->d_partials);
-        if (s->d_result) cudaFree(s->d_result);
-        if (s->h_result) cudaFreeHost(s->h_result);
-        if (s->d_flag) cudaFree(s->d_flag);
-        if (s->d_staging) cudaFree(s->d_staging);
-        if (s->d_scratch) cudaFree(s->d_scratch);
-        if (s->d_work) cudaFree(s->d_work);
-        if (s->link_stream) {
-            cudaStreamSynchronize(s->link_stream);
-            cudaStreamDestroy(s->link_stream);
-        }
-        for (cudaEvent_t ev : s->link_ev)
-            if (ev) cudaEventDestroy(ev);
-        if (s->own_stream) cudaStreamDestroy(s->own_stream);
     }
-    delete s;
+    if (!cache_put(s)) free_handle(s);
     return QI_OK;
+}
+
+qi_status qi_cache_trim(void) {
+    cache_clear();
+    return publish(ok_status());
 }
 
 qi_status qi_state_info(const qi_state *s, int32_t *num_qubits, int32_t *precision) {
@@ -629,18 +744,21 @@ qi_status qi_state_info(const qi_state *s, int32_t *num_qubits, int32_t *precisi
 
 qi_status qi_state_set_stream(qi_state *s, void *cuda_stream) {
     QI_GUARD(s);
+    s->exposed = true;
     s->stream = cuda_stream ? (cudaStream_t)cuda_stream : s->own_stream;
     return publish(ok_status());
 }
 
 qi_status qi_state_get_stream(qi_state *s, void **cuda_stream) {
     QI_GUARD(s);
+    s->exposed = true;
     if (cuda_stream) *cuda_stream = (void *)s->stream;
     return publish(ok_status());
 }
 
 qi_status qi_state_device_ptr(qi_state *s, void **dev_ptr) {
     QI_GUARD(s);
+    s->exposed = true;
     if (dev_ptr) *dev_ptr = s->amps;
     return publish(ok_status());
 }
@@ -690,6 +808,7 @@ qi_status qi_state_upload(qi_state *s, const double *amps, uint64_t num_amps) {
     QI_GUARD(s);
     if (!amps) return publish(err(QI_ERR_NULL_ARGUMENT));
     if (num_amps != s->dim()) return publish(err(QI_ERR_INVALID_NUMBER_OF_QUBITS, s->n));
+    s->host_io = true;
     if (s->prec == QI_F64) {
         cudaError_t e = cudaMemcpyAsync(s->amps, amps, s->bytes(), cudaMemcpyHostToDevice, s->stream);
         if (e != cudaSuccess) return publish(cuda_status(e, "upload"));
@@ -720,6 +839,7 @@ qi_status qi_state_upload_async(qi_state *s, const double *amps, uint64_t num_am
     QI_GUARD(s);
     if (!amps) return publish(err(QI_ERR_NULL_ARGUMENT));
     if (num_amps != s->dim()) return publish(err(QI_ERR_INVALID_NUMBER_OF_QUBITS, s->n));
+    s->host_io = true;
     if (!mapped_host_ptr(amps)) return publish(err(QI_ERR_INVALID_INPUT_VALUE, -1, -1, "host buffer not page-locked"));
     if (s->prec == QI_F64) {
         cudaError_t e = cudaMemcpyAsync(s->amps, amps, s->bytes(), cudaMemcpyHostToDevice, s->stream);
@@ -740,6 +860,7 @@ qi_status qi_state_download_async(qi_state *s, double *amps, uint64_t num_amps) 
     QI_GUARD(s);
     if (!amps) return publish(err(QI_ERR_NULL_ARGUMENT));
     if (num_amps != s->dim()) return publish(err(QI_ERR_INVALID_NUMBER_OF_QUBITS, s->n));
+    s->host_io = true;
     if (!mapped_host_ptr(amps)) return publish(err(QI_ERR_INVALID_INPUT_VALUE, -1, -1, "host buffer not page-locked"));
     if (s->prec == QI_F64) {
         cudaError_t e = cudaMemcpyAsync(amps, s->amps, s->bytes(), cudaMemcpyDeviceToHost, s->stream);
@@ -762,6 +883,7 @@ qi_status qi_state_download(qi_state *s, double *amps, uint64_t num_amps) {
     QI_GUARD(s);
     if (!amps) return publish(err(QI_ERR_NULL_ARGUMENT));
     if (num_amps != s->dim()) return publish(err(QI_ERR_INVALID_NUMBER_OF_QUBITS, s->n));
+    s->host_io = true;
     if (s->prec == QI_F64) {
         cudaError_t e = cudaMemcpyAsync(amps, s->amps, s->bytes(), cudaMemcpyDeviceToHost, s->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
@@ -886,17 +1008,16 @@ qi_status qi_state_axpy(qi_state *y, double re, double im, const qi_state *x) {
     if (!x) return publish(err(QI_ERR_NULL_ARGUMENT));
     if (x->n != y->n) return publish(err(QI_ERR_INVALID_NUMBER_OF_QUBITS, x->n));
     if (x->prec != y->prec) return publish(err(QI_ERR_UNSUPPORTED, -1, -1, "axpy needs equal precisions"));
-    if (x->stream != y->stream) {
-        cudaError_t e = cudaStreamSynchronize(x->stream);
-        if (e != cudaSuccess) return publish(cuda_status(e, "sync"));
-    }
+    Status st = read_begin(y, x);
+    if (!st.ok()) return publish(st);
     unsigned g = grid_for(y->dim());
     if (y->prec == QI_F32)
         k_axpy<float><<<g, 256, 0, y->stream>>>((float2 *)y->amps, (const float2 *)x->amps, y->dim(), (float)re, (float)im);
     else
         k_axpy<double><<<g, 256, 0, y->stream>>>((double2 *)y->amps, (const double2 *)x->amps, y->dim(), re, im);
     count_launch();
-    return publish(check_launch("k_axpy"));
+    st = check_launch("k_axpy");
+    return publish(st.ok() ? read_end(y, x) : st);
 }
 
 qi_status qi_state_inner_product(qi_state *a, qi_state *b, double out[2]) {
@@ -968,9 +1089,9 @@ qi_status qi_state_tensor_product(qi_state *out, qi_state *a, qi_state *b) {
     if (out->n != a->n + b->n) return publish(err(QI_ERR_INVALID_NUMBER_OF_QUBITS, out->n));
     if (a->prec != out->prec || b->prec != out->prec)
         return publish(err(QI_ERR_UNSUPPORTED, -1, -1, "tensor product needs equal precisions"));
-    cudaError_t e = cudaStreamSynchronize(a->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
-    if (e != cudaSuccess) return publish(cuda_status(e, "sync"));
+    Status st = read_begin(out, a);
+    if (st.ok()) st = read_begin(out, b);
+    if (!st.ok()) return publish(st);
     unsigned g = grid_for(out->dim());
     if (out->prec == QI_F32)
         k_tensor<float><<<g, 256, 0, out->stream>>>((float2 *)out->amps, (const float2 *)a->amps, (const float2 *)b->amps,
@@ -979,7 +1100,10 @@ qi_status qi_state_tensor_product(qi_state *out, qi_state *a, qi_state *b) {
         k_tensor<double><<<g, 256, 0, out->stream>>>((double2 *)out->amps, (const double2 *)a->amps,
                                                     (const double2 *)b->amps, out->dim(), b->n);
     count_launch();
-    return publish(check_launch("k_tensor"));
+    st = check_launch("k_tensor");
+    if (st.ok()) st = read_end(out, a);
+    if (st.ok()) st = read_end(out, b);
+    return publish(st);
 }
 
 qi_status qi_state_amplitude(qi_state *s, uint64_t n, double out[2]) {

@@ -397,6 +397,20 @@ __global__ void __launch_bounds__(256) k_mat1(typename Cx<T>::V2 *a, GateParams 
     }
 }
 
+// The same from one state into another (every amplitude is written): a gate on a copy in one launch.
+template <typename T, int MODE, int PH>
+__global__ void __launch_bounds__(256) k_mat1_to(typename Cx<T>::V2 *o, const typename Cx<T>::V2 *a, GateParams p) {
+    const Mat1Coef<T> c(p.m);
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, lo = p.b0 - 1;
+    for (uint64_t w = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; w < p.nwork; w += stride) {
+        const uint64_t i0 = ((w & ~lo) << 1) | (w & lo), i1 = i0 | p.b0;
+        typename Cx<T>::V2 x = a[i0], y = a[i1];
+        if ((i0 & p.cmask) == p.cmask) mat1_update<T, MODE, PH>(x, y, c);
+        o[i0] = x;
+        o[i1] = y;
+    }
+}
+
 // One target on qubit 0 (FP32): a pair (i0, i0 + 1) is one 16-byte load and store, so a
 // warp moves 512 contiguous bytes per instruction (the generic path's two 8-byte accesses
 // per pair sit 8 bytes apart).  Two pairs per thread are in flight.
@@ -564,6 +578,55 @@ static void launch_mat1_t(typename Cx<T>::V2 *a, const GateParams &p, int mode, 
 #undef QI_M1
 }
 
+template <typename T>
+static void launch_mat1_to(typename Cx<T>::V2 *o, const typename Cx<T>::V2 *a, const GateParams &p, int mode, int ph,
+                           unsigned g, cudaStream_t st) {
+#define QI_M1(MODE, PH) k_mat1_to<T, MODE, PH><<<g, 256, 0, st>>>(o, a, p)
+    switch (mode) {
+    case M1_GENERAL: QI_M1(M1_GENERAL, PH_GENERAL); break;
+    case M1_REAL: QI_M1(M1_REAL, PH_GENERAL); break;
+    case M1_DIAG: QI_M1(M1_DIAG, PH_GENERAL); break;
+    case M1_ANTIDIAG:
+        if (ph == PH_NEG) QI_M1(M1_ANTIDIAG, PH_NEG);
+        else if (ph == PH_I) QI_M1(M1_ANTIDIAG, PH_I);
+        else QI_M1(M1_ANTIDIAG, PH_GENERAL);
+        break;
+    default:
+        if (ph == PH_NEG) QI_M1(M1_PHASE1, PH_NEG);
+        else if (ph == PH_I) QI_M1(M1_PHASE1, PH_I);
+        else if (ph == PH_NEG_I) QI_M1(M1_PHASE1, PH_NEG_I);
+        else QI_M1(M1_PHASE1, PH_GENERAL);
+        break;
+    }
+#undef QI_M1
+}
+
+// dst = gate applied to src (same size and precision, dst != src).  One launch for a one-target gate; any
+// other gate works on a copy.
+static Status apply_gate_to(qi_state *dst, const qi_state *src, const Op &op) {
+    if (op.kind != OP_MAT1) {
+        Status st = state_copy_async(dst, src);
+        return st.ok() ? launch_op(dst, op, nullptr) : st;
+    }
+    GateParams p;
+    std::memset(&p, 0, sizeof(p));
+    p.cmask = op.cmask;
+    p.b0 = 1ull << op.targets[0];
+    std::copy(op.m, op.m + 8, p.m);
+    p.nwork = dst->dim() >> 1;
+    Status st = read_begin(dst, src);
+    if (!st.ok()) return st;
+    const unsigned g = gate_grid(p.nwork);
+    const int ph = phase_kind(op);
+    if (dst->prec == QI_F32)
+        launch_mat1_to<float>((float2 *)dst->amps, (const float2 *)src->amps, p, op.mode, ph, g, dst->stream);
+    else
+        launch_mat1_to<double>((double2 *)dst->amps, (const double2 *)src->amps, p, op.mode, ph, g, dst->stream);
+    count_launch();
+    st = check_launch("k_mat1_to");
+    return st.ok() ? read_end(dst, src) : st;
+}
+
 Status launch_op(qi_state *s, const Op &op, const void *d_mats, const void *d_tc) {
     const int n = s->n;
     const bool f32 = s->prec == QI_F32;
@@ -698,6 +761,23 @@ qi_status qi_apply_gate(qi_state *s, const qi_gate *g) {
     if (!st.ok()) return publish(st);
     Op op = lower_gate(s->n, gm);
     return publish(launch_op(s, op, nullptr));
+}
+
+qi_status qi_apply_gate_to(qi_state *dst, const qi_state *src, const qi_gate *g) {
+    if (!dst || !src || !g) return publish(err(QI_ERR_NULL_ARGUMENT));
+    std::lock_guard<std::recursive_mutex> lk(dst->mu);
+    cudaError_t e = cudaSetDevice(dst->device);
+    if (e != cudaSuccess) return publish(cuda_status(e, "cudaSetDevice"));
+    if (dst->n != src->n) return publish(err(QI_ERR_INVALID_NUMBER_OF_QUBITS, src->n));
+    if (dst == src) return qi_apply_gate(dst, g);
+    GateMatrix gm;
+    Status st = gate_to_matrix(dst->n, *g, &gm);
+    if (!st.ok()) return publish(st);
+    if (dst->prec != src->prec || gm.pauli || gm.measure) {
+        st = state_copy_async(dst, src);
+        return st.ok() ? qi_apply_gate(dst, g) : publish(st);
+    }
+    return publish(apply_gate_to(dst, src, lower_gate(dst->n, gm)));
 }
 
 qi_status qi_unitary2_check(const double m[8]) {   // operator.rs:2092-2125

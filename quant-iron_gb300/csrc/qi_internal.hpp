@@ -67,8 +67,13 @@ struct qi_state {
     void *d_scratch = nullptr;        // second state buffer for out-of-place permutations (lazy)
     void *d_work = nullptr;           // workspace of calls that finish before they return (lazy, grows)
     size_t work_bytes = 0;
+    void *d_prog = nullptr;
+    size_t prog_bytes = 0;
     cudaStream_t link_stream = nullptr;   // lowest-priority stream of uploads the GPU reads over the link (lazy)
     cudaEvent_t link_ev[2] = {nullptr, nullptr};   // orders it after, and before, this handle's stream
+    cudaEvent_t ev = nullptr;         // position of this handle's stream, for other handles' streams to wait on
+    bool exposed = false;             // its buffer or stream was handed out, or the caller's stream came in
+    bool host_io = false;             // a host buffer may still be in use by its stream
 
     uint64_t dim() const { return 1ull << n; }
     size_t amp_bytes() const { return prec == QI_F64 ? 16 : 8; }
@@ -84,6 +89,12 @@ Status state_scale_async(qi_state *s, double re, double im);
 Status state_normalise_device_async(qi_state *s);   // norm on device, divides if != 0 and != 1; flags ZeroNorm
 Status state_read_flag(qi_state *s, int *flag);      // sync; resets the flag
 Status state_copy_async(qi_state *dst, const qi_state *src);
+// Around work on dst's stream that reads src's buffer: dst's stream waits for the work issued on src, and
+// src's later work (and the next owner of its buffer) waits for the read.
+Status read_begin(qi_state *dst, const qi_state *src);
+Status read_end(qi_state *dst, const qi_state *src);
+// cudaMalloc; on failure the cached handles are freed and it is tried once more.
+cudaError_t device_malloc(void **p, size_t bytes);
 
 // ----------------------------------------------------------------- gates --
 // A gate lowered to one primitive device operation.
@@ -177,7 +188,8 @@ Status state_scratch(qi_state *s, void **out);
 // The state's workspace, at least `bytes` long (16-byte aligned, freed with the state).  For calls that
 // wait for the state's stream before they return, so that nothing on the device still reads it
 // when the next call, on whichever stream, takes it.
-Status state_workspace(qi_state *s, size_t bytes, void **out);
+// program: the space of the call's plan programs, apart from that of the operations between them.
+Status state_workspace(qi_state *s, size_t bytes, void **out, bool program = false);
 // Divide in by its FP64 norm into out (out != in; a norm of 0 or 1 copies unchanged, 0 flags ZeroNorm).
 Status state_normalise_device_to_async(qi_state *s, void *out, const void *in);
 // the same with the norm partials of `in` already in s->d_partials (nb rows)

@@ -1532,11 +1532,10 @@ qi_status qi_pauli_apply(qi_state *out, qi_state *in, const qi_pauli_term *t) {
         // in place: pair update with cosh = 0, sinh = coefficient
         return publish(launch_pauli_exp(out, t->xmask, t->zmask, 0.0, 0.0, t->coeff_re, t->coeff_im));
     }
-    if (in->stream != out->stream) {
-        cudaError_t e = cudaStreamSynchronize(in->stream);
-        if (e != cudaSuccess) return publish(cuda_status(e, "sync"));
-    }
-    return publish(launch_pauli_apply(out, in, t->xmask, t->zmask, t->coeff_re, t->coeff_im));
+    st = read_begin(out, in);
+    if (st.ok()) st = launch_pauli_apply(out, in, t->xmask, t->zmask, t->coeff_re, t->coeff_im);
+    if (st.ok()) st = read_end(out, in);
+    return publish(st);
 }
 
 qi_status qi_pauli_apply_normalised(qi_state *s, const qi_pauli_term *t) {

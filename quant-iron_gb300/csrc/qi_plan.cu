@@ -690,18 +690,25 @@ static bool runs_ready(qi_plan *p, qi_state *s) {
     return true;
 }
 
-// The same for a plan that lives for one call on one state: its program is copied into the state's
-// workspace, in stream order (the caller waits for the stream before it lets go of the state).
-static void borrow_runs(qi_plan *p, qi_state *s) {
+// The same for plans that live for one call on one state: their programs are copied into the state's
+// program space, in stream order (the caller waits for the stream before it lets go of the state).
+static void borrow_runs(std::initializer_list<qi_plan *> plans, qi_state *s) {
+    size_t total = 0;
+    for (qi_plan *p : plans) total += (p->run_prog.size() + 15) / 16 * 16;
     void *d = nullptr;
-    if (p->run_prog.empty() || !state_workspace(s, p->run_prog.size(), &d).ok()) return;
-    if (cudaMemcpyAsync(d, p->run_prog.data(), p->run_prog.size(), cudaMemcpyHostToDevice, s->stream) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return;
+    if (total == 0 || !state_workspace(s, total, &d, true).ok()) return;
+    char *at = static_cast<char *>(d);
+    for (qi_plan *p : plans) {
+        if (p->run_prog.empty()) continue;
+        if (cudaMemcpyAsync(at, p->run_prog.data(), p->run_prog.size(), cudaMemcpyHostToDevice, s->stream) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return;
+        }
+        p->d_run = at;
+        p->run_device = s->device;
+        p->run_borrowed = true;
+        at += (p->run_prog.size() + 15) / 16 * 16;
     }
-    p->d_run = d;
-    p->run_device = s->device;
-    p->run_borrowed = true;
 }
 
 void release_runs(qi_plan *p) {
@@ -762,13 +769,16 @@ struct PlanRunner {
 Status plan_execute(qi_plan *p, qi_state *s) {
     if (s->n != p->n) return err(QI_ERR_INVALID_NUMBER_OF_QUBITS, s->n);   // circuit.rs:161-163
     if (s->prec != p->prec) return err(QI_ERR_UNSUPPORTED, -1, -1, "plan precision differs from state");
-    if (not_uploaded(p)) {   // matrices go to the device on first use
+    const bool runs = runs_ready(p, s);
+    bool matrices = !runs;   // only operations outside the runs need them
+    for (size_t i = 0; !matrices && i < p->sched.size(); ++i)
+        matrices = p->sched[i].op >= 0 && p->ops[(size_t)p->sched[i].op].mat_offset >= 0;
+    if (matrices && not_uploaded(p)) {   // they go to the device on first use
         Status up = upload_plan(p);
         if (!up.ok()) return up;
     }
     bool has_norm = false;
     PlanRunner run(p, s);
-    const bool runs = runs_ready(p, s);
     for (size_t i = 0; runs && i < p->sched.size(); ++i) {
         const RunSegment &seg = p->sched[i];
         if (seg.op >= 0) {
@@ -1081,7 +1091,7 @@ qi_status qi_circuit_execute(qi_state *s, const qi_gate *gates, int64_t n_gates,
     qi_status st = qi_plan_create(s->n, s->prec, gates, n_gates, theta, n_theta, opts, &p);
     if (st != QI_OK) return st;
     std::lock_guard<std::recursive_mutex> lk(s->mu);   // held until the plan's program is no longer in use
-    if (cudaSetDevice(s->device) == cudaSuccess) borrow_runs(p, s);
+    if (cudaSetDevice(s->device) == cudaSuccess) borrow_runs({p}, s);
     st = qi_plan_execute(p, s);
     if (st == QI_OK) {
         cudaError_t e = cudaStreamSynchronize(s->stream);
@@ -1129,17 +1139,18 @@ qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_t
     // plan may use the tensor-core blocks and renormalise once per step; complex
     // coefficients (a non-unitary step) keep the CUDA-core blocks and the norm.
     // FP64: FP64 arithmetic is scarce on this part (dense FP64 blocks would be
-    // compute-bound), so each run of exponentials whose X-masks lie in {0, X}
-    // (e.g. the XX, YY, ZZ terms of one bond, or a run of Z fields) is one pass
-    // with a parity-indexed table; other terms are one pass each.
+    // compute-bound), so the exponentials run as gate runs, two operations per
+    // amplitude each; where some cannot (wide X strings), each run of exponentials whose
+    // X-masks lie in {0, X} is one pass with a parity-indexed table.
     bool unitary = true;
     for (int64_t k = 0; k < n_terms; ++k) unitary = unitary && terms[k].coeff_im == 0.0;
     const bool observing = observable && observe_every > 0;
     // FP64 second-order steps: the terms that end one step begin the next, and equal exponentials with
     // nothing between join (qi_gaterun.cu), so a plan covers several steps: the most up to 6 that divide
     // the steps to take (one plan to build; the joined fraction grows as 1 - 1 / steps), else 4.
+    // Below 17 qubits a step takes the device less time than the host needs to schedule it.
     int64_t many = 1;
-    if (s->prec == QI_F64 && order == 2) {
+    if (s->prec == QI_F64 && order == 2 && s->n >= 17) {
         const int64_t span = observing ? std::min(observe_every, num_steps) : num_steps;
         const int64_t cap = std::min<int64_t>({span, 6, std::max<int64_t>(1, 1000 / n_terms)});
         for (int64_t k = 2; k <= cap; ++k)
@@ -1147,29 +1158,41 @@ qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_t
         if (many == 1) many = std::min<int64_t>(cap, 4);
     }
     qi_plan single, several;
+    bool have_single = false, have_several = false;
     auto prepare = [&](qi_plan &plan, int64_t steps) {
         plan.n = s->n;
         plan.prec = s->prec;
-        plan.opts.fusion = s->prec == QI_F32 ? QI_FUSION_GREEDY : QI_FUSION_PAULI_GROUPS;
         plan.opts.use_tensor_cores = unitary ? 1 : 2;
         plan.opts.renorm_every = unitary ? 0 : -1;
         plan.opts.max_block_qubits = 0;
         std::vector<Elem> elems = step_list(steps);
-        Status st = build_plan(&plan, elems);
-        if (st.ok()) st = upload_plan(&plan);
-        return st;
+        // FP64: grouped exponentials only where some element cannot join a gate run
+        plan.opts.fusion = QI_FUSION_GREEDY;
+        if (s->prec == QI_F64) {
+            plan.opts.fusion = QI_FUSION_NONE;
+            for (const Elem &el : elems)
+                if (!run_supported(s->n, s->prec, el)) plan.opts.fusion = QI_FUSION_PAULI_GROUPS;
+        }
+        return build_plan(&plan, elems);
     };
+    // which of the two plans the steps will take
+    auto chunk = [&](int64_t step) {
+        const int64_t left = observing ? std::min(num_steps - step, observe_every - step % observe_every) : num_steps - step;
+        return many > 1 && left >= many ? many : 1;
+    };
+    for (int64_t step = 0; step < num_steps; step += chunk(step)) {
+        have_single = have_single || chunk(step) == 1;
+        have_several = have_several || chunk(step) > 1;
+        if (have_single && (have_several || many == 1)) break;
+    }
     Status st = ok_status();
-    bool have_single = false, have_several = false;
+    if (have_single) st = prepare(single, 1);
+    if (st.ok() && have_several) st = prepare(several, many);
+    if (st.ok()) borrow_runs({&single, &several}, s);
     int64_t obs_k = 0;
     for (int64_t step = 0; step < num_steps && st.ok();) {
-        const int64_t left = observing ? std::min(num_steps - step, observe_every - step % observe_every) : num_steps - step;
-        const bool more = many > 1 && left >= many;
-        qi_plan &plan = more ? several : single;
-        bool &have = more ? have_several : have_single;
-        if (!have) st = prepare(plan, more ? many : 1);
-        have = true;
-        if (st.ok()) st = plan_execute(&plan, s);
+        const bool more = chunk(step) > 1;
+        st = plan_execute(more ? &several : &single, s);
         if (!st.ok()) break;
         step += more ? many : 1;
         if (observing && step % observe_every == 0) {
@@ -1188,8 +1211,8 @@ qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_t
         plan->d_tc = nullptr;
         plan->d_mats = nullptr;
     }
+    e = cudaStreamSynchronize(s->stream);   // the programs are in use until then
     if (!st.ok()) return publish(st);
-    e = cudaStreamSynchronize(s->stream);
     if (e != cudaSuccess) return publish(cuda_status(e, "trotter"));
     return publish(ok_status());
 }

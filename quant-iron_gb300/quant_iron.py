@@ -20,6 +20,7 @@ the device copy.  Errors raise QuantIronError whose `.variant` is the name of
 the Rust Error variant.
 """
 import math
+import struct
 
 import numpy as np
 
@@ -29,6 +30,7 @@ from . import pauli_apply as _pauli_apply, pauli_apply_normalised as _pauli_norm
 from . import pauli_apply_exp_factor as _pauli_exp_factor, trotter_evolve as _trotter
 from . import measure as _measure, measure_n as _measure_n
 from ._abi import F32, F64, FUSION_GREEDY, FUSION_NONE, GATE_DTYPE, TERM_DTYPE, QuantIronError, check, lib
+from ._types import GATE_KINDS, MAX_CONTROLS
 from .workloads import GateList, qft as _qft
 
 PRECISION = F64          # precision of device states created by this module
@@ -353,6 +355,26 @@ class MeasurementResult:
 
 
 # ----------------------------------------------------------------- operators
+_ROW = struct.Struct("<3i3i2i%di8d2Q" % MAX_CONTROLS)
+assert _ROW.size == GATE_DTYPE.itemsize
+
+
+def _packed_row(kind, targets, controls, params):
+    """The bytes of a gate row (the C struct), or None where GateList has to build (or refuse) it."""
+    nt, nc, npar = len(targets), len(controls), len(params)
+    if nt > 2 or nc > MAX_CONTROLS or npar > 8:
+        return None
+    try:
+        return _ROW.pack(GATE_KINDS[kind], nt, nc, -1, -1, -1, *targets, *_NO_INTS[:2 - nt], *controls,
+                         *_NO_INTS[:MAX_CONTROLS - nc], *params, *_NO_FLOATS[:8 - npar], 0, 0)
+    except (struct.error, TypeError, KeyError):
+        return None
+
+
+_NO_INTS = (0,) * MAX_CONTROLS
+_NO_FLOATS = (0.0,) * 8
+
+
 class Operator:
     """`trait Operator` (operator.rs:151-190): apply(state, targets, controls) -> State."""
     KIND = None
@@ -370,10 +392,13 @@ class Operator:
         return gl.array()[0]
 
     def apply(self, state, target_qubits, control_qubits=()):
-        row = self.gate_row(target_qubits, control_qubits)
-        with state._device() as d:
-            d.apply_gate(row)
-            return State._take(d, state.num_qubits)
+        row = _packed_row(self.KIND, target_qubits, control_qubits, self.params())
+        if row is None:
+            row = self.gate_row(target_qubits, control_qubits).tobytes()
+        src = state._resident()
+        d = DeviceState(state.num_qubits, PRECISION)
+        check(lib.qi_apply_gate_to(d.h, src.h, row))   # row: the C struct's bytes
+        return State(None, state.num_qubits, _dev=d)
 
 
 def _op(name, kind, base=1):
@@ -613,7 +638,10 @@ class Circuit:
     def gate_array(self):
         if not self.gates:
             return np.zeros(0, dtype=GATE_DTYPE)
-        return np.stack([g.row if isinstance(g, Gate) else g for g in self.gates]).astype(GATE_DTYPE)
+        rows = [g.row if isinstance(g, Gate) else g for g in self.gates]
+        if all(isinstance(r, (np.void, np.ndarray)) and r.dtype == GATE_DTYPE and r.ndim == 0 for r in rows):
+            return np.frombuffer(b"".join([r.tobytes() for r in rows]), dtype=GATE_DTYPE)
+        return np.stack(rows).astype(GATE_DTYPE)
 
     def execute(self, initial_state):   # circuit.rs:160-172
         if initial_state.num_qubits != self.num_qubits:
