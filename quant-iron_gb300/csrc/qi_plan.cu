@@ -408,7 +408,76 @@ static void build_schedule(qi_plan *p, const std::vector<Elem> &elems, const std
     }
 }
 
-Status build_plan(qi_plan *p, std::vector<Elem> &elems) {
+// Plans that execute as gate runs from end to end, without looking at their ops: per-gate plans whose
+// every element a pass can apply, and FP32 fused plans of run_min to run_max qubits for which the
+// caller chose neither block size nor tensor cores.  A tensor-core block of a small state fills a few of
+// the SMs (17 qubits: 16 tiles) for 8 to 16 us; 40 layers + QFT, fused blocks / gate runs, among others and
+// alone (us): 10 qubits 103 / 70, 265 / 217; 12 qubits 194 / 98, 569 / 296; 17 qubits 226 / 174, 621 / 460;
+// 18 qubits 240 / 224, 657 / 500; 19 qubits 277 / 330, 722 / 594; 20 qubits 429 / 585, 769 / 900.  The
+// ops (with the fused blocks' matrices, most of a plan's build time) are made when something asks for them.
+
+static bool build_runs(qi_plan *p, const std::vector<Elem> &elems, int fusion, int kmax) {
+    p->lazy = false;
+    p->run_normalise = false;
+    const bool per_gate = fusion == QI_FUSION_NONE || fusion == QI_FUSION_PAULI_GROUPS;
+    const bool small_fused = fusion == QI_FUSION_GREEDY && p->opts.fusion == QI_FUSION_GREEDY && p->prec == QI_F32 &&
+                             p->opts.use_tensor_cores == 0 && p->opts.max_block_qubits == 0 &&
+                             p->partition_override.empty() && p->n >= p->run_min && p->n <= p->run_max;
+    if (!per_gate && !small_fused) return false;
+    int64_t count = 0;
+    for (const Elem &e : elems) {
+        if (!run_supported(p->n, p->prec, e)) return false;
+        count += e.gm.pauli || e.gm.nt > 0;
+    }
+    if (count < 2) return false;
+    if (small_fused) {
+        // the state is renormalised at the end when tensor-core blocks would have run (build_plan)
+        p->lazy_blocks = partition_with_permutations(p, elems, kmax);
+        for (const Block &b : p->lazy_blocks) {
+            const int k = __builtin_popcountll(b.mask);
+            bool diag = true;
+            for (int i : b.members) diag = diag && elems[(size_t)i].diagonal;
+            if (!b.single && !b.perm && !diag && ((k >= 3 && k <= 5 && p->n >= 12) || (k == 6 && p->n >= 13)))
+                p->run_normalise = p->opts.renorm_every >= 0;
+        }
+    }
+    std::vector<const Elem *> run;
+    for (const Elem &e : elems) run.push_back(&e);
+    RunSegment seg;
+    schedule_run(p->n, p->prec, run, seg, p->run_prog);
+    p->sched.push_back(std::move(seg));
+    p->lazy_elems = elems;
+    p->lazy = true;
+    return true;
+}
+
+static Status build_plan_ops(qi_plan *p, std::vector<Elem> &elems, bool ops);
+Status build_plan(qi_plan *p, std::vector<Elem> &elems) { return build_plan_ops(p, elems, false); }
+
+// The ops of a plan that executes as gate runs, made on first request.
+static Status ensure_ops(const qi_plan *cp) {
+    qi_plan *p = const_cast<qi_plan *>(cp);
+    std::lock_guard<std::mutex> lk(p->run_mu);
+    if (!p->lazy) return ok_status();
+    qi_plan q;   // built apart: the runs may be executing
+    q.n = p->n;
+    q.prec = p->prec;
+    q.opts = p->opts;
+    q.partition_override = p->lazy_blocks;
+    Status st = build_plan_ops(&q, p->lazy_elems, true);
+    if (!st.ok()) return st;
+    p->ops.swap(q.ops);
+    p->mats.swap(q.mats);
+    p->tc.swap(q.tc);
+    p->polys.swap(q.polys);
+    p->stats = q.stats;
+    p->lazy = false;
+    p->lazy_elems.clear();
+    return ok_status();
+}
+
+// ops: make the ops and nothing else.
+static Status build_plan_ops(qi_plan *p, std::vector<Elem> &elems, bool ops) {
     const int n = p->n;
     int fusion = p->opts.fusion;
     int kmax = p->opts.max_block_qubits > 0 ? p->opts.max_block_qubits : 6;
@@ -441,6 +510,7 @@ Status build_plan(qi_plan *p, std::vector<Elem> &elems) {
         if (e.pauli && !e.gm.normalise_after && fusion != QI_FUSION_NONE && __builtin_popcountll(e.mask) <= kmax)
             e.fusable = true;
     }
+    if (!ops && build_runs(p, elems, fusion, kmax)) return ok_status();
     auto lower_single = [&](const Elem &e) {
         Op op = lower_gate(n, e.gm);
         if (op.kind == OP_PAULI_EXP) {
@@ -487,7 +557,7 @@ Status build_plan(qi_plan *p, std::vector<Elem> &elems) {
             i = j;
         }
         first.push_back(elems.size());
-        build_schedule(p, elems, first);
+        if (!ops) build_schedule(p, elems, first);
     } else {
         std::vector<Block> blocks = p->partition_override.empty() ? partition_with_permutations(p, elems, kmax)
                                                                   : p->partition_override;
@@ -773,6 +843,10 @@ Status plan_execute(qi_plan *p, qi_state *s) {
     bool matrices = !runs;   // only operations outside the runs need them
     for (size_t i = 0; !matrices && i < p->sched.size(); ++i)
         matrices = p->sched[i].op >= 0 && p->ops[(size_t)p->sched[i].op].mat_offset >= 0;
+    if (!runs) {
+        Status have = ensure_ops(p);
+        if (!have.ok()) return have;
+    }
     if (matrices && not_uploaded(p)) {   // they go to the device on first use
         Status up = upload_plan(p);
         if (!up.ok()) return up;
@@ -791,6 +865,10 @@ Status plan_execute(qi_plan *p, qi_state *s) {
             Status st = launch_run_pass(s, pass, p->d_run);
             if (!st.ok()) return run.finish(st);
         }
+    }
+    if (runs && p->run_normalise) {
+        Status st = state_normalise_device_async(s);
+        if (!st.ok()) return run.finish(st);
     }
     for (size_t i = 0; !runs && i < p->ops.size(); ++i) {
         const Op &op = p->ops[i];
@@ -830,8 +908,9 @@ using namespace qi;
 
 extern "C" {
 
-qi_status qi_plan_create(int32_t num_qubits, int32_t precision, const qi_gate *gates, int64_t n_gates,
-                         const double *theta, int64_t n_theta, const qi_exec_options *opts, qi_plan **out) {
+static qi_status plan_create(int32_t num_qubits, int32_t precision, const qi_gate *gates, int64_t n_gates,
+                             const double *theta, int64_t n_theta, const qi_exec_options *opts, bool one_call,
+                             qi_plan **out) {
     if (!out || (!gates && n_gates > 0)) return publish(err(QI_ERR_NULL_ARGUMENT));
     *out = nullptr;
     if (num_qubits <= 0 || num_qubits > 40) return publish(err(QI_ERR_INVALID_NUMBER_OF_QUBITS, num_qubits));
@@ -840,12 +919,21 @@ qi_status qi_plan_create(int32_t num_qubits, int32_t precision, const qi_gate *g
     p->n = num_qubits;
     p->prec = precision;
     if (opts) p->opts = *opts;
+    if (one_call) {   // the plan's build counts too: 40 layers, 22 qubits 0.7 + 2.9 ms as runs, 6 + 1.4 ms as blocks
+        p->run_min = 4;
+        p->run_max = 23;
+    }
     std::vector<Elem> elems;
     Status st = plan_elems_from_gates(num_qubits, gates, n_gates, theta, n_theta, elems);
     if (st.ok()) st = build_plan(p, elems);
     if (!st.ok()) { delete p; return publish(st); }
     *out = p;
     return publish(ok_status());
+}
+
+qi_status qi_plan_create(int32_t num_qubits, int32_t precision, const qi_gate *gates, int64_t n_gates,
+                         const double *theta, int64_t n_theta, const qi_exec_options *opts, qi_plan **out) {
+    return plan_create(num_qubits, precision, gates, n_gates, theta, n_theta, opts, false, out);
 }
 
 qi_status qi_plan_execute(qi_plan *p, qi_state *s) {
@@ -858,6 +946,8 @@ qi_status qi_plan_execute(qi_plan *p, qi_state *s) {
 
 qi_status qi_plan_stats_get(const qi_plan *p, qi_plan_stats *out) {
     if (!p || !out) return publish(err(QI_ERR_NULL_ARGUMENT));
+    Status st = ensure_ops(p);
+    if (!st.ok()) return publish(st);
     *out = p->stats;
     return publish(ok_status());
 }
@@ -868,6 +958,10 @@ qi_status qi_plan_profile(qi_plan *p, qi_state *s, float *ms_out) {
     cudaError_t e = cudaSetDevice(s->device);
     if (e != cudaSuccess) return publish(cuda_status(e, "cudaSetDevice"));
     if (s->n != p->n || s->prec != p->prec) return publish(err(QI_ERR_INVALID_NUMBER_OF_QUBITS, s->n));
+    {
+        Status have = ensure_ops(p);
+        if (!have.ok()) return publish(have);
+    }
     if (not_uploaded(p)) {
         Status up = upload_plan(p);
         if (!up.ok()) return publish(up);
@@ -961,6 +1055,8 @@ qi_status qi_apply_matrix(qi_state *s, const int32_t *targets, int32_t k, const 
 
 qi_status qi_plan_num_ops(const qi_plan *p, int64_t *out) {
     if (!p || !out) return publish(err(QI_ERR_NULL_ARGUMENT));
+    Status st = ensure_ops(p);
+    if (!st.ok()) return publish(st);
     *out = (int64_t)p->ops.size();
     return publish(ok_status());
 }
@@ -991,6 +1087,10 @@ qi_status qi_plan_run_replay(const qi_plan *p, double *amps) {
 
 qi_status qi_plan_op_phase_poly(const qi_plan *p, int64_t i, uint64_t *c0, uint64_t *a, uint64_t *b) {
     if (!p || !c0 || !a || !b) return publish(err(QI_ERR_NULL_ARGUMENT));
+    {
+        Status have = ensure_ops(p);
+        if (!have.ok()) return publish(have);
+    }
     if (i < 0 || i >= (int64_t)p->ops.size()) return publish(err(QI_ERR_INVALID_INPUT_VALUE, i));
     const Op &op = p->ops[(size_t)i];
     const int64_t idx = op.kind == OP_PHASE_POLY ? op.mat_offset : op.kind == OP_FUSED ? op.poly_idx : -1;
@@ -1005,6 +1105,10 @@ qi_status qi_plan_op_phase_poly(const qi_plan *p, int64_t i, uint64_t *c0, uint6
 
 qi_status qi_plan_op_pauli_group(const qi_plan *p, int64_t i, int32_t *n_tables, int32_t *rank, uint64_t *basis) {
     if (!p || !n_tables || !rank || !basis) return publish(err(QI_ERR_NULL_ARGUMENT));
+    {
+        Status have = ensure_ops(p);
+        if (!have.ok()) return publish(have);
+    }
     if (i < 0 || i >= (int64_t)p->ops.size()) return publish(err(QI_ERR_INVALID_INPUT_VALUE, i));
     const Op &op = p->ops[(size_t)i];
     if (op.kind != OP_PAULI_GROUP) return publish(err(QI_ERR_INVALID_INPUT_VALUE, i, op.kind, "not a Pauli-group op"));
@@ -1016,6 +1120,10 @@ qi_status qi_plan_op_pauli_group(const qi_plan *p, int64_t i, int32_t *n_tables,
 
 qi_status qi_plan_op_bitperm(const qi_plan *p, int64_t i, int32_t *source_bit, uint64_t *flip) {
     if (!p || !source_bit || !flip) return publish(err(QI_ERR_NULL_ARGUMENT));
+    {
+        Status have = ensure_ops(p);
+        if (!have.ok()) return publish(have);
+    }
     if (i < 0 || i >= (int64_t)p->ops.size()) return publish(err(QI_ERR_INVALID_INPUT_VALUE, i));
     const Op &op = p->ops[(size_t)i];
     if (op.kind != OP_BITPERM) return publish(err(QI_ERR_INVALID_INPUT_VALUE, op.kind, OP_BITPERM));
@@ -1026,6 +1134,10 @@ qi_status qi_plan_op_bitperm(const qi_plan *p, int64_t i, int32_t *source_bit, u
 
 qi_status qi_plan_op_get(const qi_plan *p, int64_t i, qi_plan_op_info *info, double *matrix_out, int64_t capacity) {
     if (!p || !info) return publish(err(QI_ERR_NULL_ARGUMENT));
+    {
+        Status have = ensure_ops(p);
+        if (!have.ok()) return publish(have);
+    }
     if (i < 0 || i >= (int64_t)p->ops.size()) return publish(err(QI_ERR_INVALID_INPUT_VALUE, i));
     const Op &op = p->ops[(size_t)i];
     std::memset(info, 0, sizeof(*info));
@@ -1088,7 +1200,7 @@ qi_status qi_circuit_execute(qi_state *s, const qi_gate *gates, int64_t n_gates,
                              const qi_exec_options *opts) {
     if (!s) return publish(err(QI_ERR_NULL_ARGUMENT));
     qi_plan *p = nullptr;
-    qi_status st = qi_plan_create(s->n, s->prec, gates, n_gates, theta, n_theta, opts, &p);
+    qi_status st = plan_create(s->n, s->prec, gates, n_gates, theta, n_theta, opts, true, &p);
     if (st != QI_OK) return st;
     std::lock_guard<std::recursive_mutex> lk(s->mu);   // held until the plan's program is no longer in use
     if (cudaSetDevice(s->device) == cudaSuccess) borrow_runs({p}, s);
@@ -1162,7 +1274,14 @@ qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_t
     auto prepare = [&](qi_plan &plan, int64_t steps) {
         plan.n = s->n;
         plan.prec = s->prec;
-        plan.opts.use_tensor_cores = unitary ? 1 : 2;
+        plan.opts.use_tensor_cores = unitary ? 0 : 2;
+        // A plan for one call: composing its blocks takes 1.2 ms and more (177-term lattice), so gate runs win
+        // up to 20 qubits, and above that for as many steps as cost less than that in slower passes (XYZ
+        // lattice, ms, runs / blocks: 20 qubits 20 steps 3.3 / 4.2; 22 qubits 5 steps 2.1 / 2.2, 20 steps
+        // 8.2 / 5.3; 24 qubits 1 step 1.8 / 2.1, 5 steps 8.6 / 4.8)
+        plan.run_min = 4;
+        plan.run_max = 20;
+        while (plan.run_max < 24 && num_steps <= (int64_t)20 >> (plan.run_max + 1 - 20)) ++plan.run_max;
         plan.opts.renorm_every = unitary ? 0 : -1;
         plan.opts.max_block_qubits = 0;
         std::vector<Elem> elems = step_list(steps);

@@ -72,6 +72,12 @@ struct qi_plan {
     std::vector<qi::RunSegment> sched;
     std::vector<uint8_t> run_prog;
     void *d_run = nullptr;        // the programs on device run_device, once executed there
+    bool run_normalise = false;   // a renormalisation follows the runs
+    // ops not made yet (every op is in a run): what they are made from
+    bool lazy = false;
+    int32_t run_min = 10, run_max = 18;   // qubits of an FP32 fused plan that executes as gate runs
+    std::vector<qi::Elem> lazy_elems;
+    std::vector<qi::Block> lazy_blocks;
     int32_t run_device = -1;
     bool run_borrowed = false;    // d_run is a state's workspace
     std::mutex run_mu;            // first use
