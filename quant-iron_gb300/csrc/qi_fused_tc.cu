@@ -10,35 +10,32 @@
 //   [D_re | D_im][m] += Im X[.][m] . [-Im U ; Re U ]^T     (imaginary half)
 // The B operands are the R x R blocks -Im U, Re U, Im U stored one after the
 // other along N (K-major, shared memory), so [Re U ; Im U] starts at block 1
-// and [-Im U ; Re U] at block 0.  Pair mode with k = 6 (below), short of shared memory,
-// keeps only Re U, Im U and splits the imaginary half into two N = R products,
-//   D_re -= Im X . Im U^T (negate-B)   and   D_im += Im X . Re U^T.
+// and [-Im U ; Re U] at block 0.
 // Every operand is split as x = hi + lo with
 // hi = tf32(x) (round to nearest) and lo = tf32(x - hi); the products
 // A_hi B_hi + A_hi B_lo + A_lo B_hi are accumulated in FP32, which keeps
 // about 22 significant bits (the dropped A_lo B_lo term is ~2^-22 relative).
 //
 // One persistent CTA per SM, warp-specialised, synchronised by mbarriers:
-//   producer (1 thread): cp.async.bulk copies of each tile (2^nhigh runs of
-//     2^L contiguous amplitudes) into one of NBUF shared buffers, in address
-//     order; completion by transaction count on raw_full[b]
+//   producer (1 warp): cp.async.bulk copies of each tile (2^nhigh runs of
+//     2^L contiguous amplitudes, a run per lane) into one of NBUF shared
+//     buffers; completion by transaction count on raw_full[b]
 //   converters (8 warps; warp w owns TMEM lanes 32*(w%4).. = tile columns and
 //     rows slice w/4): once A stage 0 is free, read the tile in 16-row chunks,
 //     splitting the real parts into A_hi/A_lo of stage 0 (tcgen05.st) and
 //     keeping the imaginary parts in registers; release the buffer
 //     (raw_empty[b]); split the imaginary parts into stage 1 once it is free;
 //     each stage is signalled on a_full[h]
-//   MMA issuer (1 thread): per half 3 products x R/8 MMAs (M128 x N2R x K8;
-//     pair mode's imaginary half: two M128 x NR x K8 per step) into
-//     accumulator buffer it%2; tcgen05.commit frees the A stage
-//     (a_empty[h]) and publishes the accumulator (d_full[d])
+//   MMA issuer (1 warp, one elected lane): per half 3 products x R/8 MMAs
+//     (M128 x N2R x K8) into accumulator buffer it%2; tcgen05.commit frees
+//     the A stage (a_empty[h]) and publishes the accumulator (d_full[d])
 //   epilogue (4 warps): tcgen05.ld the accumulator, release it (d_empty[d]),
 //     store the amplitudes straight to global memory (rows r, r+1 as one
 //     16-byte store when qubit 0 is a target; adjacent lanes are adjacent
 //     amplitudes when it is a column)
 // Every wait is bounded; a timeout sets the state's error flag (2) and a
 // shared abort flag that every other wait polls, so all roles leave their
-// loops; the MMA thread then waits for its own products and the producer for
+// loops; the MMA warp then waits for its own products and the producer for
 // its copies before the tensor memory is freed.
 // Tensor-memory columns: A stage h at h*2R (A_hi [0,R), A_lo [R,2R)),
 // accumulator d at 4R + d*2R (D_re [0,R), D_im [R,2R)): 8R columns in all.
@@ -84,9 +81,9 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
 }
 
 // Instruction descriptor, kind::tf32: D = F32, A = B = TF32, both K-major,
-// negate B at bit 14, N >> 3 at bit 17, M >> 4 at bit 24.
-__host__ __device__ constexpr uint32_t tf32_idesc(uint32_t M, uint32_t N, bool negate_b = false) {
-    return (1u << 4) | (2u << 7) | (2u << 10) | ((negate_b ? 1u : 0u) << 14) | ((N >> 3) << 17) | ((M >> 4) << 24);
+// N >> 3 at bit 17, M >> 4 at bit 24.
+__host__ __device__ constexpr uint32_t tf32_idesc(uint32_t M, uint32_t N) {
+    return (1u << 4) | (2u << 7) | (2u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
 __device__ __forceinline__ void mma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
@@ -97,6 +94,16 @@ __device__ __forceinline__ void mma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, ui
         "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d_tmem),
         "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
+}
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t on;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(on));
+    return on != 0;
 }
 
 __device__ __forceinline__ void mma_commit(uint64_t *bar) {
@@ -188,29 +195,24 @@ __device__ __forceinline__ bool warp_wait_or_abort(uint64_t *bar, uint32_t parit
 constexpr int kPhaseLane = 64, kPhaseTile = 64 + 128 * 8;
 
 // ------------------------------------------------------------------ kernel
-template <int K, bool PAIR = false>
+template <int K>
 struct TcCfg {
     static constexpr int R = 1 << K;                   // rows (target patterns)
     static constexpr int BLK = R * R;                  // floats per operand block
     static constexpr uint32_t LBO = 128;               // next core matrix along K
     static constexpr uint32_t SBO = (R / 4) * 128;     // next 8-row group along N
-    // shared buffers: whole tiles, or (pair mode) a ring of units of 16 rows x 2 KB runs
-    static constexpr int NBUF = PAIR ? (K == 6 ? 10 : 12) : (K == 6 ? 2 : 6);
+    // Shared buffers of one tile: what fits at k = 6; at k = 5 loads that run further ahead of the stores
+    // only cost memory rate (26 qubits, 2 / 3 / 4 / 6 buffers: 185 / 179 / 181 / 181 us a launch).
+    static constexpr int NBUF = K == 6 ? 2 : 3;
     static constexpr uint32_t STAGE = 2 * R;           // TMEM columns of one A stage or one accumulator
     static constexpr uint32_t COL_A = 0, COL_D = 2 * STAGE;
     static constexpr uint32_t TMEM_COLS = 4 * STAGE;   // 512 for k = 6, 256 for k = 5
     static constexpr int CONV_ROWS = R / 2;            // rows per converter thread (2 row slices)
-    static constexpr int CHUNK = PAIR ? 8 : 16;        // rows converted per step (register footprint)
+    static constexpr int CHUNK = 16;                   // rows converted per step (register footprint)
     static constexpr uint32_t TILE_BYTES = (uint32_t)R * 128 * sizeof(float2);
-    static constexpr int UNIT_ROWS = 8;                // pair mode: rows per ring unit (one chunk)
-    static constexpr int UNITS_PER_PAIR = 2 * CONV_ROWS / UNIT_ROWS;   // pair mode: 8
-    static constexpr uint32_t BUF_BYTES = PAIR ? (uint32_t)UNIT_ROWS * 2 * 128 * sizeof(float2) : TILE_BYTES;
-    // operand blocks in shared memory: -Im U, Re U, Im U (hi, then lo); pair mode with k = 6,
-    // short of shared memory, Re U, Im U (the imaginary half as two N = R products)
-    static constexpr bool SPLIT_IM = PAIR && K == 6;
-    static constexpr int NBLK = SPLIT_IM ? 4 : 6;
+    static constexpr int NBLK = 6;                     // operand blocks -Im U, Re U, Im U (hi, then lo)
     static constexpr size_t OFF_TILES = (size_t)NBLK * BLK * sizeof(float);
-    static constexpr size_t OFF_ROWX = OFF_TILES + (size_t)NBUF * BUF_BYTES;
+    static constexpr size_t OFF_ROWX = OFF_TILES + (size_t)NBUF * TILE_BYTES;
     static constexpr size_t OFF_GROW = OFF_ROWX + 64 * sizeof(uint32_t);
     static constexpr size_t OFF_BAR = OFF_GROW + 64 * sizeof(uint64_t);
     static constexpr int NBARS = 2 * NBUF + 9;
@@ -274,25 +276,16 @@ __device__ __forceinline__ void st_cs_v8(float2 *p, float a0, float a1, float a2
                  : "memory");
 }
 
-// PAIR: a CTA takes tiles in pairs (2p, 2p+1), which differ in qubit L = 7, so the row
-// runs of the two tiles are adjacent in memory; one bulk copy of 2 x 2^L amplitudes per
-// row run loads both.  The pair's rows go through a ring of NBUF units of 8 rows
-// (unit u = 2c + s: chunk c of converter slice s); a unit is released after the pair's
-// second tile has read it, so the next pair's first units load while the second tile
-// is converted.  Used when the runs are 1 KB (all targets above qubit 7), where the
-// copy granularity bounds the load rate.
 // ROT: qubits 0-3 are all targets, so the tile's columns are 128 bytes or more apart and the
 // 8 lanes of a quarter warp would read the same banks for one row pair; each lane then reads the
 // chunk's row pairs starting at its own (lane mod 8), undone in registers.
 // PHASE: a diagonal phase polynomial exp(2 pi i f(x)) that follows the block in the plan is
 // applied by the epilogue before the store (its phase table at `poly`, tc_phase_table).
-template <int K, bool PAIR, bool ROT, bool PHASE>
+template <int K, bool ROT, bool PHASE>
 __global__ void __launch_bounds__(kTcThreads, 1) k_fused_tc(float2 *a, const float *blocks, TileGeom g, int *err_flag,
                                                             const uint32_t *__restrict__ poly) {
-    using C = TcCfg<K, PAIR>;
+    using C = TcCfg<K>;
     constexpr int R = C::R, NB = C::NBUF;
-    static_assert(!PAIR || ((K == 5 || K == 6) && C::UNIT_ROWS == C::CHUNK), "pair mode: K = 5 or 6, one ring unit per chunk");
-    static_assert(!(PAIR && ROT), "pair-mode tiles have qubit 0 as a column");
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     float *sB = reinterpret_cast<float *>(smem_raw);   // operand blocks (C::NBLK)
     unsigned char *tiles = smem_raw + C::OFF_TILES;
@@ -306,17 +299,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_fused_tc(float2 *a, const flo
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-    // operand blocks -> shared memory (16-byte vectors), visible to the async proxy;
-    // pair mode with k = 6 takes blocks 1, 2, 4, 5 (Re U, Im U; hi then lo) of the six
+    // operand blocks -> shared memory (16-byte vectors), visible to the async proxy
     {
         const uint4 *src = reinterpret_cast<const uint4 *>(blocks);
         uint4 *dst = reinterpret_cast<uint4 *>(sB);
-        constexpr int per_blk = C::BLK * (int)sizeof(float) / 16;
-        for (int i = tid; i < C::NBLK * per_blk; i += kTcThreads) {
-            const int blk = i / per_blk;
-            const int from = C::NBLK == 4 ? (blk < 2 ? blk + 1 : blk + 2) : blk;
-            dst[i] = src[from * per_blk + i % per_blk];
-        }
+        for (int i = tid; i < C::NBLK * C::BLK * (int)sizeof(float) / 16; i += kTcThreads) dst[i] = src[i];
     }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     // row r (bit j <-> target j) -> tile-local position and global offset
@@ -330,10 +317,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_fused_tc(float2 *a, const flo
         }
         for (int j = 0; j < g.nhigh; ++j) {
             const uint32_t bit = ((uint32_t)tid >> (g.nlow_t + j)) & 1u;
-            // pair mode: the top row bits select the ring unit (slice, chunk); the others index
-            // its runs of 2 x 2^L
-            if (!PAIR) x |= bit << (g.L + j);
-            else if ((1 << j) < C::UNIT_ROWS) x |= bit << (g.L + 1 + j);
+            x |= bit << (g.L + j);
             go |= (uint64_t)bit << g.high_t[j];
         }
         rowx[tid] = x;
@@ -342,7 +326,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_fused_tc(float2 *a, const flo
     if (tid == 0) {
         for (int i = 0; i < NB; ++i) {
             mbar_init(raw_full + i, 1);
-            mbar_init(raw_empty + i, PAIR ? kConvWarps / 2 : kConvWarps);   // pair mode: one slice per unit
+            mbar_init(raw_empty + i, kConvWarps);
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(a_full + i, kConvWarps);
@@ -361,11 +345,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_fused_tc(float2 *a, const flo
     const uint32_t tmem = *tmem_slot;
     // tile counts stay below 2^32 (2^(n-13) tiles for n <= 44)
     const uint32_t ntiles = (uint32_t)g.ntiles;
-    // iteration -> tile; pair mode takes 2p and 2p + 1 in consecutive iterations
-    auto tile_of = [&](int it) -> uint32_t {
-        return PAIR ? 2u * (blockIdx.x + (uint32_t)(it >> 1) * gridDim.x) + (uint32_t)(it & 1)
-                    : blockIdx.x + (uint32_t)it * gridDim.x;
-    };
+    auto tile_of = [&](int it) -> uint32_t { return blockIdx.x + (uint32_t)it * gridDim.x; };
     const bool pair_rows = !g.q0_is_col;   // qubit 0 is target 0: rows r, r+1 are adjacent amplitudes
     // qubits 0 and 1 both targets: rows r..r+3 are four adjacent amplitudes (one 32-byte store)
     const bool quad_rows = pair_rows && g.nlow_t >= 2 && g.low_t[1] == 1;
@@ -377,30 +357,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_fused_tc(float2 *a, const flo
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
         const int r0 = slice * C::CONV_ROWS;
         for (int it = 0; tile_of(it) < ntiles; ++it) {
-            const int b = it % NB;   // whole-tile buffer (pair mode: units, below)
-            if (!PAIR && !warp_wait_or_abort(raw_full + b, (uint32_t)(it / NB) & 1u, abort_flag, err_flag)) break;
+            const int b = it % NB;
+            if (!warp_wait_or_abort(raw_full + b, (uint32_t)(it / NB) & 1u, abort_flag, err_flag)) break;
             // real half -> A stage 0, once the products of the previous tile have read it;
             // the imaginary parts stay in registers for stage 1
             if (it > 0 && !warp_wait_or_abort(a_empty + 0, (uint32_t)(it - 1) & 1u, abort_flag, err_flag)) break;
             tc_fence_after();
-            bool ok = true;
+            const float2 *S = reinterpret_cast<const float2 *>(tiles + (size_t)b * C::TILE_BYTES);
             float im[C::CONV_ROWS];
 #pragma unroll
             for (int c0 = 0; c0 < C::CONV_ROWS; c0 += C::CHUNK) {
-                const float2 *S;
-                uint32_t unit = 0;
-                if constexpr (PAIR) {
-                    const uint32_t k = (uint32_t)C::UNITS_PER_PAIR * (uint32_t)(it >> 1) +
-                                       2u * (uint32_t)(c0 / C::CHUNK) + (uint32_t)slice;
-                    unit = k % NB;
-                    if (!(it & 1) && !warp_wait_or_abort(raw_full + unit, (k / NB) & 1u, abort_flag, err_flag)) {
-                        ok = false;
-                        break;
-                    }
-                    S = reinterpret_cast<const float2 *>(tiles + (size_t)unit * C::BUF_BYTES) + ((uint32_t)(it & 1) << g.L);
-                } else {
-                    S = reinterpret_cast<const float2 *>(tiles + (size_t)b * C::BUF_BYTES);
-                }
                 float re[C::CHUNK];
                 if constexpr (ROT) {
                     static_assert(C::CHUNK == 16, "8 row pairs per chunk");
@@ -446,16 +412,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_fused_tc(float2 *a, const flo
                 }
                 split_store<C::CHUNK>(tmem + lane_base + C::COL_A + r0 + c0, tmem + lane_base + C::COL_A + R + r0 + c0,
                                       re);
-                if constexpr (PAIR) {   // the pair's second tile was the unit's last reader
-                    __syncwarp();
-                    if (lane == 0 && (it & 1)) mbar_arrive(raw_empty + unit);
-                }
             }
-            if (!ok) break;
-            if (!PAIR) {
-                __syncwarp();
-                if (lane == 0) mbar_arrive(raw_empty + b);   // the buffer may take the next tile
-            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(raw_empty + b);   // the buffer may take the next tile
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
@@ -560,114 +519,85 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_fused_tc(float2 *a, const flo
             };
             // Not unrolled: the kernel's four roles run different code, and with the epilogue unrolled
             // over its chunks the warps waited on instruction fetch ("no instruction" stalls 3.2-4.7
-            // per issue). Rolled, 30-qubit launches took 3.09 against 3.44 ms (pairs), 2.67 against
-            // 2.80 ms (single tiles) and, carrying a phase polynomial, 2.83 against 3.81 ms.
+            // per issue). Rolled, 30-qubit launches took 2.67 against 2.80 ms and, carrying a phase
+            // polynomial, 2.83 against 3.81 ms.
 #pragma unroll 1
             for (int c = 0; c < R / 16; ++c) chunk(c);
         }
     } else if (warp == kProducerWarp) {
-        // ------------------------------------------------ producer (one thread)
-        if (lane == 0) {
-            const uint32_t run_bytes = (uint32_t)sizeof(float2) << g.L;
-            if (!PAIR) {
-                const int nruns = 1 << g.nhigh;
-                int issued = 0;
-                for (int it = 0; tile_of(it) < ntiles; ++it) {
-                    const int b = it % NB;
-                    if (it >= NB && !wait_or_abort(raw_empty + b, (uint32_t)(it / NB - 1) & 1u, abort_flag, err_flag))
-                        break;
-                    mbar_arrive_expect_tx(raw_full + b, C::TILE_BYTES);
-                    const uint64_t base = tile_base(g, tile_of(it));
-                    unsigned char *dst = tiles + (size_t)b * C::TILE_BYTES;
-                    for (int h = 0; h < nruns; ++h)
-                        bulk_load(dst + (size_t)h * run_bytes, a + (base | grow[h << g.nlow_t]), run_bytes, raw_full + b);
-                    issued = it + 1;
-                }
-                // copies still in flight (only after an abort) land before the CTA exits
-                for (int j = issued > NB ? issued - NB : 0; j < issued; ++j)
-                    if (!mbar_wait_bounded(raw_full + (j % NB), (uint32_t)(j / NB) & 1u)) atomicExch(err_flag, 2);
-            } else {
-                // ring unit k (pair k / 4, u = k % 4 = 2c + s) <- rows 32 s + 16 c .. + 15 of the
-                // pair: runs of 2 x 2^L amplitudes (both tiles), in the order the converters use them
-                int issued = 0;
-                bool ok = true;
-                for (uint32_t lp = 0; ok && tile_of(2 * (int)lp) < ntiles; ++lp) {
-                    const uint64_t base = tile_base(g, tile_of(2 * (int)lp));
-                    for (uint32_t u = 0; u < (uint32_t)C::UNITS_PER_PAIR; ++u) {
-                        const uint32_t k = (uint32_t)C::UNITS_PER_PAIR * lp + u, unit = k % NB;
-                        if (k >= (uint32_t)NB &&
-                            !wait_or_abort(raw_empty + unit, (k / NB - 1) & 1u, abort_flag, err_flag)) {
-                            ok = false;
-                            break;
-                        }
-                        mbar_arrive_expect_tx(raw_full + unit, C::BUF_BYTES);
-                        unsigned char *dst = tiles + (size_t)unit * C::BUF_BYTES;
-                        const int row0 = C::CONV_ROWS * (int)(u & 1u) + C::UNIT_ROWS * (int)(u >> 1);
-                        for (int i = 0; i < C::UNIT_ROWS; ++i)
-                            bulk_load(dst + (size_t)i * 2 * run_bytes, a + (base | grow[row0 + i]), 2 * run_bytes,
-                                      raw_full + unit);
-                        issued = (int)k + 1;
-                    }
-                }
-                // copies still in flight (only after an abort) land before the CTA exits
-                for (int j = issued > NB ? issued - NB : 0; j < issued; ++j)
-                    if (!mbar_wait_bounded(raw_full + (j % NB), (uint32_t)(j / NB) & 1u)) atomicExch(err_flag, 2);
-            }
+        // ------------------------------------------------ producer (one warp, a run per lane)
+        // A run per lane: issued by one thread, a copy took about 170 cycles (its address comes from
+        // shared memory and goes to uniform registers), so tiles of 64 runs of 1 KB loaded at less than
+        // half the memory's rate.  30-qubit launches of such tiles took 4.4 ms, and 2.61 a run per lane;
+        // pairs of adjacent tiles in runs of 2 KB, which halve the copies, 3.02 and 2.77 (they hold
+        // their buffers for two tiles, so the loads come in bursts).
+        const uint32_t run_bytes = (uint32_t)sizeof(float2) << g.L;
+        const int nruns = 1 << g.nhigh;
+        int issued = 0;
+        for (int it = 0; tile_of(it) < ntiles; ++it) {
+            const int b = it % NB;
+            const float2 *src = a + tile_base(g, tile_of(it));
+            unsigned char *dst = tiles + (size_t)b * C::TILE_BYTES;
+            if (it >= NB && !warp_wait_or_abort(raw_empty + b, (uint32_t)(it / NB - 1) & 1u, abort_flag, err_flag)) break;
+            if (lane == 0) mbar_arrive_expect_tx(raw_full + b, C::TILE_BYTES);
+            __syncwarp();
+            for (int h = lane; h < nruns; h += 32)
+                bulk_load(dst + (size_t)h * run_bytes, src + grow[h << g.nlow_t], run_bytes, raw_full + b);
+            __syncwarp();
+            issued = it + 1;
         }
+        // copies still in flight (only after an abort) land before the CTA exits
+        for (int j = issued > NB ? issued - NB : 0; j < issued; ++j)
+            if (!mbar_wait_bounded(raw_full + (j % NB), (uint32_t)(j / NB) & 1u)) atomicExch(err_flag, 2);
         __syncwarp();
     } else {
-        // ------------------------------------------------ MMA issuer (one thread)
-        if (lane == 0) {
-            // Descriptor of block 0 at K offset 0; every MMA adds a constant byte offset
-            // (>> 4 into the start-address field, which cannot carry: blocks stay below 256 KB).
-            const uint64_t desc0 = smem_desc(smem_u32(sB), C::LBO, C::SBO);
-            constexpr uint32_t idesc = tf32_idesc(128, 2 * R), idesc_r = tf32_idesc(128, R),
-                               idesc_rneg = tf32_idesc(128, R, true);
-            bool ok = true;
-            for (int it = 0; ok && tile_of(it) < ntiles; ++it) {
-                const int d = it & 1;
-                if (it >= 2 && !wait_or_abort(d_empty + d, (uint32_t)((it >> 1) - 1) & 1u, abort_flag, err_flag))
-                    break;
-                tc_fence_after();
-                const uint32_t dcol = tmem + C::COL_D + d * C::STAGE;
+        // ------------------------------------------------ MMA issuer (one elected thread)
+        // The warp stays converged through the waits and one elected lane issues, so descriptors and
+        // tensor-memory addresses are warp-uniform: an MMA then issues in about the 64 cycles that it
+        // runs (M128 N128 K8), against 80-98 from a lane that had left its warp (blocks of 22 qubits:
+        // 0.81 -> 0.76 ms per 20 layers).
+        const bool leader = elect_one();
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+        // Descriptor of block 0 at K offset 0; every MMA adds a constant byte offset
+        // (>> 4 into the start-address field, which cannot carry: blocks stay below 256 KB).
+        const uint64_t desc0 = smem_desc(smem_u32(sB), C::LBO, C::SBO);
+        constexpr uint32_t idesc = tf32_idesc(128, 2 * R);
+        bool ok = true;
+        for (int it = 0; ok && tile_of(it) < ntiles; ++it) {
+            const int d = it & 1;
+            if (it >= 2 && !warp_wait_or_abort(d_empty + d, (uint32_t)((it >> 1) - 1) & 1u, abort_flag, err_flag)) break;
+            const uint32_t dcol = tm + C::COL_D + d * C::STAGE;
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    if (!wait_or_abort(a_full + h, (uint32_t)it & 1u, abort_flag, err_flag)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t acol = tmem + C::COL_A + h * C::STAGE;
+            for (int h = 0; h < 2; ++h) {
+                if (!warp_wait_or_abort(a_full + h, (uint32_t)it & 1u, abort_flag, err_flag)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t acol = tm + C::COL_A + h * C::STAGE;
+                if (leader) {
 #pragma unroll
                     for (int p = 0; p < 3; ++p) {   // (A_hi, B_hi), (A_hi, B_lo), (A_lo, B_hi)
 #pragma unroll
                         for (int j = 0; j < R / 8; ++j) {
                             const uint32_t kstep = (uint32_t)(2 * j) * C::LBO;
                             const uint32_t a_col = acol + (p == 2 ? R : 0) + 8 * j;
-                            if constexpr (!C::SPLIT_IM) {   // window [Re U ; Im U] (block 1) or [-Im U ; Re U] (block 0)
-                                const int blk = (p == 1 ? 3 : 0) + (h == 0 ? 1 : 0);
-                                const uint32_t boff = (uint32_t)(blk * C::BLK * 4) + kstep;
-                                mma_tf32_ts(dcol, a_col, desc0 + (uint64_t)(boff >> 4), idesc, (h | p | j) ? 1u : 0u);
-                            } else {
-                                const int blk = p == 1 ? 2 : 0;   // Re U of the hi or lo pair, Im U next to it
-                                const uint32_t b_re = (uint32_t)(blk * C::BLK * 4) + kstep, b_im = b_re + C::BLK * 4;
-                                if (h == 0) {   // [D_re | D_im] += Re X . [Re U ; Im U]^T
-                                    mma_tf32_ts(dcol, a_col, desc0 + (uint64_t)(b_re >> 4), idesc, (p | j) ? 1u : 0u);
-                                } else {        // D_re -= Im X . Im U^T;  D_im += Im X . Re U^T
-                                    mma_tf32_ts(dcol, a_col, desc0 + (uint64_t)(b_im >> 4), idesc_rneg, 1u);
-                                    mma_tf32_ts(dcol + R, a_col, desc0 + (uint64_t)(b_re >> 4), idesc_r, 1u);
-                                }
-                            }
+                            // window [Re U ; Im U] (block 1) or [-Im U ; Re U] (block 0)
+                            const int blk = (p == 1 ? 3 : 0) + (h == 0 ? 1 : 0);
+                            const uint32_t boff = (uint32_t)(blk * C::BLK * 4) + kstep;
+                            mma_tf32_ts(dcol, a_col, desc0 + (uint64_t)(boff >> 4), idesc, (h | p | j) ? 1u : 0u);
                         }
                     }
                     mma_commit(a_empty + h);
+                    if (h == 1) mma_commit(d_full + d);
                 }
-                if (ok) mma_commit(d_full + d);
+                __syncwarp();
             }
-            // every product issued here has completed before the tensor memory is freed
-            mma_commit(mma_done);
-            if (!mbar_wait_bounded(mma_done, 0)) atomicExch(err_flag, 2);
         }
+        // every product issued here has completed before the tensor memory is freed
+        if (leader) mma_commit(mma_done);
+        __syncwarp();
+        if (!mbar_wait_bounded(mma_done, 0)) atomicExch(err_flag, 2);
         __syncwarp();
     }
     tc_fence_before();
@@ -795,9 +725,9 @@ bool tc_phase_table(const PhasePoly &pp, int k, const int32_t *targets, std::vec
     return true;
 }
 
-template <int K, bool PAIR, bool ROT, bool PHASE>
+template <int K, bool ROT, bool PHASE>
 static Status launch_tc_t(qi_state *s, const TileGeom &g, const void *d_tc, const void *poly) {
-    using C = TcCfg<K, PAIR>;
+    using C = TcCfg<K>;
     static_assert(C::SMEM <= 232448, "shared memory per CTA");
     // the shared-memory opt-in and the SM count are per device (state handles may live on several)
     static std::atomic<int> num_sms_of[64];
@@ -806,14 +736,14 @@ static Status launch_tc_t(qi_state *s, const TileGeom &g, const void *d_tc, cons
     if (dev < 0 || dev >= 64) return err(QI_ERR_UNSUPPORTED, dev, 64, "device ordinal");
     int num_sms = num_sms_of[dev].load();
     if (num_sms == 0) {
-        QI_CUDA(cudaFuncSetAttribute(k_fused_tc<K, PAIR, ROT, PHASE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        QI_CUDA(cudaFuncSetAttribute(k_fused_tc<K, ROT, PHASE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)C::SMEM));
         QI_CUDA(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
         num_sms_of[dev].store(num_sms);
     }
-    uint64_t grid = PAIR ? g.ntiles / 2 : g.ntiles;   // one persistent CTA per SM
+    uint64_t grid = g.ntiles;   // one persistent CTA per SM
     if (grid > (uint64_t)num_sms) grid = (uint64_t)num_sms;
-    k_fused_tc<K, PAIR, ROT, PHASE><<<(unsigned)grid, kTcThreads, C::SMEM, s->stream>>>(
+    k_fused_tc<K, ROT, PHASE><<<(unsigned)grid, kTcThreads, C::SMEM, s->stream>>>(
         (float2 *)s->amps, (const float *)d_tc, g, s->d_flag, (const uint32_t *)poly);
     count_launch();
     return check_launch("k_fused_tc");
@@ -826,20 +756,13 @@ Status launch_fused_tc(qi_state *s, int k, const int32_t *targets, const void *d
     const TileGeom g = make_tile_geom(n, k, targets, 7);
     if (g.nfree != n - k - 7) return err(QI_ERR_UNKNOWN, g.nfree, n - k - 7, "tile decomposition");
     if (((uintptr_t)d_tc & 15) != 0) return err(QI_ERR_UNKNOWN, -1, -1, "operand blocks must be 16-byte aligned");
-    // Tile pairs when a tile's rows are 1 KB runs (all targets above qubit 7): tiles 2p, 2p + 1
-    // differ in qubit L = 7, so each pair of runs is one 2 KB copy.  (Measured at 30 qubits: 3.28 ms
-    // per launch against 4.4 ms for single tiles of 1 KB runs; a 4-unit ring with the N = 2R
-    // imaginary half took 3.83 ms, so the ring depth matters more than the extra MMAs.)
-    const bool pair = g.nlow_t == 0 && g.nhigh == k && g.nfree >= 1 && g.L == 7 && g.L < n;
     // qubits 0-3 all targets: lane-rotated row reads (k_fused_tc's ROT)
     bool rot = true;
     for (int q = 0; q < 4; ++q) rot = rot && std::find(targets, targets + k, q) != targets + k;
     if (poly && ((uintptr_t)poly & 15) != 0) return err(QI_ERR_UNKNOWN, -1, -1, "phase block must be 16-byte aligned");
-#define QI_TC(KK, PA, RO)                                                                    \
-    (poly ? launch_tc_t<KK, PA, RO, true>(s, g, d_tc, poly) : launch_tc_t<KK, PA, RO, false>(s, g, d_tc, nullptr))
-    if (k == 5) return pair ? QI_TC(5, true, false) : rot ? QI_TC(5, false, true) : QI_TC(5, false, false);
-    if (pair) return QI_TC(6, true, false);
-    return rot ? QI_TC(6, false, true) : QI_TC(6, false, false);
+#define QI_TC(KK, RO) (poly ? launch_tc_t<KK, RO, true>(s, g, d_tc, poly) : launch_tc_t<KK, RO, false>(s, g, d_tc, nullptr))
+    if (k == 5) return rot ? QI_TC(5, true) : QI_TC(5, false);
+    return rot ? QI_TC(6, true) : QI_TC(6, false);
 #undef QI_TC
 }
 
