@@ -17,7 +17,9 @@
 // about 22 significant bits (the dropped A_lo B_lo term is ~2^-22 relative).
 //
 // One persistent CTA per SM, warp-specialised, synchronised by mbarriers:
-//   producer (1 warp): cp.async.bulk copies of each tile (2^nhigh runs of
+//   producer (1 warp): one copy of the operand blocks (b_full); waits for the
+//     stream's earlier work (the kernel starts before that has ended, see the
+//     launch); then cp.async.bulk copies of each tile (2^nhigh runs of
 //     2^L contiguous amplitudes, a run per lane) into one of NBUF shared
 //     buffers; completion by transaction count on raw_full[b]
 //   converters (8 warps; warp w owns TMEM lanes 32*(w%4).. = tile columns and
@@ -215,7 +217,7 @@ struct TcCfg {
     static constexpr size_t OFF_ROWX = OFF_TILES + (size_t)NBUF * TILE_BYTES;
     static constexpr size_t OFF_GROW = OFF_ROWX + 64 * sizeof(uint32_t);
     static constexpr size_t OFF_BAR = OFF_GROW + 64 * sizeof(uint64_t);
-    static constexpr int NBARS = 2 * NBUF + 9;
+    static constexpr int NBARS = 2 * NBUF + 10;
     static constexpr size_t OFF_MISC = OFF_BAR + NBARS * sizeof(uint64_t);
     static constexpr size_t OFF_FR = OFF_MISC + 16;    // phase polynomial: terms among each row's bits
     static constexpr size_t SMEM = OFF_FR + 64 * sizeof(uint32_t);
@@ -293,19 +295,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_fused_tc(float2 *a, const flo
     uint64_t *grow = reinterpret_cast<uint64_t *>(smem_raw + C::OFF_GROW);
     uint64_t *raw_full = reinterpret_cast<uint64_t *>(smem_raw + C::OFF_BAR);
     uint64_t *raw_empty = raw_full + NB, *a_full = raw_empty + NB, *a_empty = a_full + 2;
-    uint64_t *d_full = a_empty + 2, *d_empty = d_full + 2, *mma_done = d_empty + 2;
+    uint64_t *d_full = a_empty + 2, *d_empty = d_full + 2, *mma_done = d_empty + 2, *b_full = mma_done + 1;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_raw + C::OFF_MISC);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-    // operand blocks -> shared memory (16-byte vectors), visible to the async proxy
-    {
-        const uint4 *src = reinterpret_cast<const uint4 *>(blocks);
-        uint4 *dst = reinterpret_cast<uint4 *>(sB);
-        for (int i = tid; i < C::NBLK * C::BLK * (int)sizeof(float) / 16; i += kTcThreads) dst[i] = src[i];
-    }
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     // row r (bit j <-> target j) -> tile-local position and global offset
     if (tid < R) {
         uint32_t x = 0;
@@ -335,6 +330,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_fused_tc(float2 *a, const flo
             mbar_init(d_empty + i, kEpiWarps);
         }
         mbar_init(mma_done, 1);
+        mbar_init(b_full, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -531,6 +527,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_fused_tc(float2 *a, const flo
         // half the memory's rate.  30-qubit launches of such tiles took 4.4 ms, and 2.61 a run per lane;
         // pairs of adjacent tiles in runs of 2 KB, which halve the copies, 3.02 and 2.77 (they hold
         // their buffers for two tiles, so the loads come in bursts).
+        if (lane == 0) {
+            mbar_arrive_expect_tx(b_full, (uint32_t)C::OFF_TILES);
+            bulk_load(sB, blocks, (uint32_t)C::OFF_TILES, b_full);
+        }
+        // The amplitudes are the earlier kernels'; the operand blocks and phase tables are not.  The next
+        // kernel of the stream may start its own prologue from here on (it waits likewise).
+        asm volatile("griddepcontrol.wait;\n" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
         const uint32_t run_bytes = (uint32_t)sizeof(float2) << g.L;
         const int nruns = 1 << g.nhigh;
         int issued = 0;
@@ -549,6 +553,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_fused_tc(float2 *a, const flo
         // copies still in flight (only after an abort) land before the CTA exits
         for (int j = issued > NB ? issued - NB : 0; j < issued; ++j)
             if (!mbar_wait_bounded(raw_full + (j % NB), (uint32_t)(j / NB) & 1u)) atomicExch(err_flag, 2);
+        // (the operand blocks always, even when no product waited for them)
+        if (!mbar_wait_bounded(b_full, 0)) atomicExch(err_flag, 2);
         __syncwarp();
     } else {
         // ------------------------------------------------ MMA issuer (one elected thread)
@@ -562,7 +568,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_fused_tc(float2 *a, const flo
         // (>> 4 into the start-address field, which cannot carry: blocks stay below 256 KB).
         const uint64_t desc0 = smem_desc(smem_u32(sB), C::LBO, C::SBO);
         constexpr uint32_t idesc = tf32_idesc(128, 2 * R);
-        bool ok = true;
+        bool ok = warp_wait_or_abort(b_full, 0, abort_flag, err_flag);
         for (int it = 0; ok && tile_of(it) < ntiles; ++it) {
             const int d = it & 1;
             if (it >= 2 && !warp_wait_or_abort(d_empty + d, (uint32_t)((it >> 1) - 1) & 1u, abort_flag, err_flag)) break;
@@ -743,8 +749,22 @@ static Status launch_tc_t(qi_state *s, const TileGeom &g, const void *d_tc, cons
     }
     uint64_t grid = g.ntiles;   // one persistent CTA per SM
     if (grid > (uint64_t)num_sms) grid = (uint64_t)num_sms;
-    k_fused_tc<K, ROT, PHASE><<<(unsigned)grid, kTcThreads, C::SMEM, s->stream>>>(
-        (float2 *)s->amps, (const float *)d_tc, g, s->d_flag, (const uint32_t *)poly);
+    // Over all SMs, a block's setup (operand blocks, barriers, tensor memory) overlaps the end of the kernel
+    // before it (programmatic launch); a smaller grid would hold SMs that other streams can use.  With the
+    // operand blocks as one copy beside the first tile's: 20 layers of 20 / 22 / 24 / 27 qubits 0.46 / 0.75 /
+    // 2.06 / 8.27 -> 0.36 / 0.53 / 1.73 / 8.03 ms.
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = (unsigned)grid;
+    cfg.blockDim = kTcThreads;
+    cfg.dynamicSmemBytes = C::SMEM;
+    cfg.stream = s->stream;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = grid == (uint64_t)num_sms ? 1 : 0;
+    QI_CUDA(cudaLaunchKernelEx(&cfg, k_fused_tc<K, ROT, PHASE>, (float2 *)s->amps, (const float *)d_tc, g, s->d_flag,
+                               (const uint32_t *)poly));
     count_launch();
     return check_launch("k_fused_tc");
 }

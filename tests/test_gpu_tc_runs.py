@@ -22,3 +22,29 @@ def test_tensor_core_blocks_by_run_count(qi, k, n):
             qi.apply_matrix(st, targets, U, use_tensor_cores=1)
             got = st.download()
         assert np.max(np.abs(got - apply_np(init, n, targets, U))) < 1e-6, targets
+
+
+@pytest.mark.parametrize("n", [19, 21, 23])
+def test_back_to_back_blocks(qi, n):
+    """Each launch sets up while the one before ends: a plan's blocks back to back, on two states in turn
+    without a wait between, against the same plan with a wait after every execution (bit for bit) and
+    against FP64 gates.  Tolerance: 50 blocks of 2^-21 relative error on amplitudes of at most 2^-6."""
+    from quant_iron_gb300 import workloads
+    gates = workloads.random_circuit(n, layers=6, seed=n)
+    plan = qi.Plan(n, qi.F32, gates, fusion=qi.FUSION_GREEDY, use_tensor_cores=1)
+    exact = qi.Plan(n, qi.F64, gates, fusion=qi.FUSION_NONE)
+    with qi.DeviceState(n, qi.F32) as a, qi.DeviceState(n, qi.F32) as b, qi.DeviceState(n, qi.F32) as c, \
+            qi.DeviceState(n, qi.F64) as d:
+        for s in (a, b, c, d):
+            s.set_plus()
+        for _ in range(3):
+            plan.execute(a)
+            plan.execute(b)
+        for _ in range(3):
+            plan.execute(c)
+            c.synchronize()
+            exact.execute(d)
+        got, want = a.download(), d.download()
+        assert np.array_equal(got, b.download()) and np.array_equal(got, c.download())
+    assert np.max(np.abs(want)) < 2.0 ** -6
+    assert np.max(np.abs(got - want)) < 50 * 2.0 ** -21 * 2.0 ** -6
