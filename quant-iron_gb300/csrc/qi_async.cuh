@@ -80,4 +80,26 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t b
                  : "memory");
 }
 
+// Programmatic launches: the kernel may start while the one before it in the stream ends.  launch_wait()
+// returns when all earlier work of the stream has completed and its writes are visible; nothing that earlier
+// kernels write is touched before it, nor written.  After launch_next() in every block the next such kernel
+// may start.
+__device__ __forceinline__ void launch_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+struct ChainedLaunch {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr = {};
+    ChainedLaunch(unsigned blocks, unsigned threads, size_t smem, cudaStream_t stream, bool early = true) {
+        cfg.gridDim = blocks;
+        cfg.blockDim = threads;
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr.val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = early ? 1 : 0;
+    }
+    ChainedLaunch(const ChainedLaunch &) = delete;
+};
+
 }  // namespace qi

@@ -533,8 +533,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_fused_tc(float2 *a, const flo
         }
         // The amplitudes are the earlier kernels'; the operand blocks and phase tables are not.  The next
         // kernel of the stream may start its own prologue from here on (it waits likewise).
-        asm volatile("griddepcontrol.wait;\n" ::: "memory");
-        asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+        launch_wait();
+        launch_next();
         const uint32_t run_bytes = (uint32_t)sizeof(float2) << g.L;
         const int nruns = 1 << g.nhigh;
         int issued = 0;
@@ -753,17 +753,8 @@ static Status launch_tc_t(qi_state *s, const TileGeom &g, const void *d_tc, cons
     // before it (programmatic launch); a smaller grid would hold SMs that other streams can use.  With the
     // operand blocks as one copy beside the first tile's: 20 layers of 20 / 22 / 24 / 27 qubits 0.46 / 0.75 /
     // 2.06 / 8.27 -> 0.36 / 0.53 / 1.73 / 8.03 ms.
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = (unsigned)grid;
-    cfg.blockDim = kTcThreads;
-    cfg.dynamicSmemBytes = C::SMEM;
-    cfg.stream = s->stream;
-    cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = grid == (uint64_t)num_sms ? 1 : 0;
-    QI_CUDA(cudaLaunchKernelEx(&cfg, k_fused_tc<K, ROT, PHASE>, (float2 *)s->amps, (const float *)d_tc, g, s->d_flag,
+    ChainedLaunch at((unsigned)grid, kTcThreads, C::SMEM, s->stream, grid == (uint64_t)num_sms);
+    QI_CUDA(cudaLaunchKernelEx(&at.cfg, k_fused_tc<K, ROT, PHASE>, (float2 *)s->amps, (const float *)d_tc, g, s->d_flag,
                                (const uint32_t *)poly));
     count_launch();
     return check_launch("k_fused_tc");

@@ -24,6 +24,7 @@
 // operator.rs:279-2285, PauliString::apply_exp_factor (src/components/pauli_string.rs:237-262).
 #include "qi_gaterun.hpp"
 #include "qi_runops.cuh"
+#include "qi_async.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -59,6 +60,7 @@ __global__ void __launch_bounds__(256, 3) k_gate_run(typename Cx<T>::V2 *amps, c
     }
     for (uint32_t i = tid; i < (uint32_t)g.prog_units; i += nt) copy16(code + i, prog + i);
     __syncthreads();
+    launch_wait();       // the program was there before the pass before this one began; the amplitudes are its result
     uint4 *a4 = reinterpret_cast<uint4 *>(amps) + (tbase >> UB0);
     const RunCopy mine(rows, tid, lowu);
     for (uint32_t u = 0; u < nunit; u += nt)
@@ -185,6 +187,9 @@ __global__ void __launch_bounds__(256, 3) k_gate_run(typename Cx<T>::V2 *amps, c
         run_store<T, kRunSelBits>(v, tile, at);
         __syncthreads();
     }
+    // Not earlier: while this pass still computes, the next one's blocks would crowd the SMs that are free
+    // (256 tiles, FP32, 20 qubits: 0.50 -> 0.63 ms per 20 layers).
+    launch_next();
     for (uint32_t u = 0; u < nunit; u += nt)
         a4[mine.first + RunCopy::step(rows, u, lowu)] = *reinterpret_cast<uint4 *>((char *)tile + (mine.at ^ (run_swizzle(u) << 4)));
 }
@@ -213,8 +218,11 @@ Status launch_run_pass(qi_state *s, const RunPass &p, const void *d_prog) {
         if (f32) QI_CUDA(cudaFuncSetAttribute(k_gate_run<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));
         else QI_CUDA(cudaFuncSetAttribute(k_gate_run<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));
     }
-    if (f32) k_gate_run<float><<<blocks, threads, sm, s->stream>>>((float2 *)s->amps, prog, g);
-    else k_gate_run<double><<<blocks, threads, sm, s->stream>>>((double2 *)s->amps, prog, g);
+    // A pass's setup (row table, program) overlaps the end of the pass before it: 20 layers of FP64, 12 / 16 /
+    // 20 qubits 0.255 / 0.351 / 1.503 -> 0.239 / 0.328 / 1.458 ms; FP32 plan of 17 qubits 178 -> 162 us.
+    ChainedLaunch at(blocks, threads, sm, s->stream);
+    if (f32) QI_CUDA(cudaLaunchKernelEx(&at.cfg, k_gate_run<float>, (float2 *)s->amps, prog, g));
+    else QI_CUDA(cudaLaunchKernelEx(&at.cfg, k_gate_run<double>, (double2 *)s->amps, prog, g));
     count_launch();
     return check_launch("k_gate_run");
 }
