@@ -48,3 +48,37 @@ def test_back_to_back_blocks(qi, n):
         assert np.array_equal(got, b.download()) and np.array_equal(got, c.download())
     assert np.max(np.abs(want)) < 2.0 ** -6
     assert np.max(np.abs(got - want)) < 50 * 2.0 ** -21 * 2.0 ** -6
+
+
+@pytest.mark.parametrize("n, prec", [(12, "F64"), (16, "F32"), (21, "F32")])
+def test_chained_launches_on_other_streams_and_in_graphs(qi, n, prec):
+    """The default stream, a caller's stream and a replayed graph of a plan's execution (gate runs at 12 and
+    16 qubits, tensor-core blocks at 21) give what the state's own stream gives, bit for bit."""
+    torch = pytest.importorskip("torch")
+    from quant_iron_gb300 import workloads
+    gates = workloads.random_circuit(n, layers=5, seed=n)
+    plan = qi.Plan(n, getattr(qi, prec), gates, fusion=qi.FUSION_GREEDY if prec == "F32" else qi.FUSION_NONE)
+    with qi.DeviceState(n, getattr(qi, prec)) as own, qi.DeviceState(n, getattr(qi, prec)) as s:
+        own.set_plus()
+        for _ in range(4):
+            plan.execute(own)
+        want = own.download()
+        st = torch.cuda.Stream()
+        for stream in (0, st.cuda_stream):
+            s.set_stream(stream)
+            s.set_plus()
+            for _ in range(4):
+                plan.execute(s)
+            assert np.array_equal(s.download(), want), stream
+        s.set_plus()
+        s.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=st):
+            plan.execute(s)
+            plan.execute(s)
+        with torch.cuda.stream(st):
+            graph.replay()
+            graph.replay()
+        st.synchronize()
+        assert np.array_equal(s.download(), want)
+        del graph
