@@ -778,6 +778,7 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
         qi_plan plan;
         plan.n = n;
         plan.prec = s->prec;
+        plan.device_blocks = true;
         plan.opts = plan_opts;
         // FP64 (dense FP64 blocks are bound by the FP64 pipe) and FP32 up to 22 qubits unless the caller
         // chose a block size: the gate runs' own arithmetic, with no block matrices to compose (FP32

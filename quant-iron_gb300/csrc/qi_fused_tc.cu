@@ -732,7 +732,7 @@ bool tc_phase_table(const PhasePoly &pp, int k, const int32_t *targets, std::vec
 }
 
 template <int K, bool ROT, bool PHASE>
-static Status launch_tc_t(qi_state *s, const TileGeom &g, const void *d_tc, const void *poly) {
+static Status launch_tc_t(qi_state *s, const TileGeom &g, const void *d_tc, const void *poly, bool fresh) {
     using C = TcCfg<K>;
     static_assert(C::SMEM <= 232448, "shared memory per CTA");
     // the shared-memory opt-in and the SM count are per device (state handles may live on several)
@@ -750,17 +750,17 @@ static Status launch_tc_t(qi_state *s, const TileGeom &g, const void *d_tc, cons
     uint64_t grid = g.ntiles;   // one persistent CTA per SM
     if (grid > (uint64_t)num_sms) grid = (uint64_t)num_sms;
     // Over all SMs, a block's setup (operand blocks, barriers, tensor memory) overlaps the end of the kernel
-    // before it (programmatic launch); a smaller grid would hold SMs that other streams can use.  With the
+    // before it (programmatic launch; not behind the kernel that writes the operand blocks); a smaller grid would hold SMs that other streams can use.  With the
     // operand blocks as one copy beside the first tile's: 20 layers of 20 / 22 / 24 / 27 qubits 0.46 / 0.75 /
     // 2.06 / 8.27 -> 0.36 / 0.53 / 1.73 / 8.03 ms.
-    ChainedLaunch at((unsigned)grid, kTcThreads, C::SMEM, s->stream, grid == (uint64_t)num_sms);
+    ChainedLaunch at((unsigned)grid, kTcThreads, C::SMEM, s->stream, grid == (uint64_t)num_sms && !fresh);
     QI_CUDA(cudaLaunchKernelEx(&at.cfg, k_fused_tc<K, ROT, PHASE>, (float2 *)s->amps, (const float *)d_tc, g, s->d_flag,
                                (const uint32_t *)poly));
     count_launch();
     return check_launch("k_fused_tc");
 }
 
-Status launch_fused_tc(qi_state *s, int k, const int32_t *targets, const void *d_tc, const void *poly) {
+Status launch_fused_tc(qi_state *s, int k, const int32_t *targets, const void *d_tc, const void *poly, bool fresh) {
     const int n = s->n;
     if (s->prec != QI_F32 || (k != 5 && k != 6) || n < k + 7)
         return err(QI_ERR_UNSUPPORTED, k, n, "tensor-core blocks need FP32, k in {5, 6}, n >= k + 7");
@@ -771,7 +771,8 @@ Status launch_fused_tc(qi_state *s, int k, const int32_t *targets, const void *d
     bool rot = true;
     for (int q = 0; q < 4; ++q) rot = rot && std::find(targets, targets + k, q) != targets + k;
     if (poly && ((uintptr_t)poly & 15) != 0) return err(QI_ERR_UNKNOWN, -1, -1, "phase block must be 16-byte aligned");
-#define QI_TC(KK, RO) (poly ? launch_tc_t<KK, RO, true>(s, g, d_tc, poly) : launch_tc_t<KK, RO, false>(s, g, d_tc, nullptr))
+#define QI_TC(KK, RO) \
+    (poly ? launch_tc_t<KK, RO, true>(s, g, d_tc, poly, fresh) : launch_tc_t<KK, RO, false>(s, g, d_tc, nullptr, fresh))
     if (k == 5) return rot ? QI_TC(5, true) : QI_TC(5, false);
     return rot ? QI_TC(6, true) : QI_TC(6, false);
 #undef QI_TC

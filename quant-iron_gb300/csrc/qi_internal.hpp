@@ -126,6 +126,7 @@ struct Op {
     uint64_t cmask = 0;            // control mask (controls must be 1)
     double m[32] = {0};            // MAT1: 4 complex; MAT2: 16 complex (row-major re, im)
     int64_t mat_offset = -1;       // OP_FUSED / OP_DIAGK: offset (complex entries) into the plan's matrix buffer
+    bool fresh_tc = false;         // OP_FUSED: the operand blocks are the work of a kernel just before
     int64_t tc_offset = -1;        // OP_FUSED: offset (floats) of the tensor-core operand blocks, -1 if none
     uint64_t xmask = 0, zmask = 0; // Pauli ops
     double alpha_re = 0, alpha_im = 0;   // Pauli exp: cosh/sinh coefficients are derived from this
@@ -222,11 +223,12 @@ Status launch_pauli_group(qi_state *s, const Op &op, const void *d_mats);
 // Apply a dense 2^k x 2^k complex matrix (device pointer, row-major, element
 // type matches the state's precision) on sorted targets.
 Status launch_fused(qi_state *s, int k, const int32_t *targets, const void *d_mat, const void *d_tc, int use_tc,
-                    const void *poly = nullptr);
+                    const void *poly = nullptr, bool fresh_tc = false);
 // 3xTF32 tcgen05 kernel (FP32 states, k = 5 or 6, n >= k + 7); d_tc holds the
 // six operand blocks prepared by tc_blocks().
 // poly: device block of a phase polynomial applied after the block in the same pass (or null)
-Status launch_fused_tc(qi_state *s, int k, const int32_t *targets, const void *d_tc, const void *poly = nullptr);
+Status launch_fused_tc(qi_state *s, int k, const int32_t *targets, const void *d_tc, const void *poly = nullptr,
+                       bool fresh = false);
 // Host: the six K-major operand blocks {-Im U, Re U, Im U} x {tf32 hi, lo}
 // (each 2^k x 2^k floats in the no-swizzle core-matrix layout) of a fused
 // matrix U (row-major complex, FP64).  Appends 6 * 4^k floats to `out`.

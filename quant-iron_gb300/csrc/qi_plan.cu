@@ -250,6 +250,28 @@ std::vector<Block> window_partition(const std::vector<Elem> &elems, int n, int k
     });
 }
 
+// A block's members for the device's composition, on its qubits and those of `padded`.
+static void compose_job(const std::vector<Elem> &elems, const Block &b, uint64_t padded, ComposeJobs &jobs) {
+    ComposeBlock job = {};
+    job.first = (uint32_t)jobs.members.size();
+    job.count = (uint32_t)b.members.size();
+    job.k = (uint32_t)__builtin_popcountll(padded);
+    job.tc = jobs.words;
+    std::vector<int> sup;
+    std::vector<cd> D;
+    for (int idx : b.members) {
+        dense_of(elems[idx], sup, D);
+        ComposeMember m = {};
+        m.off = (uint32_t)jobs.data.size();
+        m.m = (uint8_t)sup.size();
+        for (size_t j = 0; j < sup.size(); ++j) m.pos[j] = (uint8_t)__builtin_popcountll(padded & ((1ull << sup[j]) - 1));
+        jobs.members.push_back(m);
+        jobs.data.insert(jobs.data.end(), D.begin(), D.end());
+    }
+    jobs.blocks.push_back(job);
+    jobs.words += (size_t)6 << (2 * job.k);
+}
+
 // Dense (or diagonal) matrix of a block on its sorted qubits.
 void compose_block(const std::vector<Elem> &elems, const Block &b, std::vector<int> &qubits, std::vector<cd> &B) {
     qubits.clear();
@@ -339,16 +361,20 @@ static Op bitperm_op(const std::vector<Elem> &elems, const Block &b) {
 // Widen a dense k-qubit block (k < 5; local bit j <-> op.targets[j], ascending) to 5 qubits: the
 // lowest qubits outside it join as identity factors.  op.targets / op.k and the matrix M are
 // rewritten in place (local bits again ascending by qubit).
-static void pad_block_to_5(int n, Op &op, std::vector<cd> &M) {
-    const int k = op.k;
-    uint64_t mask = 0;
-    for (int j = 0; j < k; ++j) mask |= 1ull << op.targets[j];
+static uint64_t padded_to_5(int n, uint64_t mask) {
     uint64_t sel = mask;
-    for (int q = 0, need = 5 - k; q < n && need > 0; ++q)
+    for (int q = 0, need = 5 - __builtin_popcountll(mask); q < n && need > 0; ++q)
         if (!((mask >> q) & 1ull)) {
             sel |= 1ull << q;
             --need;
         }
+    return sel;
+}
+static void pad_block_to_5(int n, Op &op, std::vector<cd> &M) {
+    const int k = op.k;
+    uint64_t mask = 0;
+    for (int j = 0; j < k; ++j) mask |= 1ull << op.targets[j];
+    const uint64_t sel = padded_to_5(n, mask);
     int qs[5], nq = 0;
     for (int q = 0; q < 64 && nq < 5; ++q)
         if ((sel >> q) & 1ull) qs[nq++] = q;
@@ -487,6 +513,7 @@ static Status build_plan_ops(qi_plan *p, std::vector<Elem> &elems, bool ops) {
     p->ops.clear();
     p->mats.clear();
     p->tc.clear();
+    p->compose = ComposeJobs();
     p->polys.clear();
     p->sched.clear();
     p->run_prog.clear();
@@ -564,12 +591,28 @@ static Status build_plan_ops(qi_plan *p, std::vector<Elem> &elems, bool ops) {
         // compose block matrices in parallel (independent)
         std::vector<std::vector<int>> qb(blocks.size());
         std::vector<std::vector<cd>> mb(blocks.size());
-        const unsigned nth = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+        // ... those the device does not compose: tensor-core blocks of a plan for one call
+        std::vector<uint64_t> on_device(blocks.size(), 0);   // the block's qubits, padded
+        size_t on_host = 0;
+        for (size_t bi = 0; bi < blocks.size(); ++bi) {
+            const Block &b = blocks[bi];
+            if (b.single || b.perm) continue;
+            bool diag = true;
+            for (int idx : b.members) diag = diag && elems[idx].diagonal;
+            const int k = __builtin_popcountll(b.mask);
+            const uint64_t padded = k == 3 || k == 4 ? (n >= 12 ? padded_to_5(n, b.mask) : 0) : k >= 5 ? b.mask : 0;
+            if (p->device_blocks && !ops && use_tc && p->prec == QI_F32 && !diag && padded &&
+                n >= __builtin_popcountll(padded) + 7)
+                on_device[bi] = padded;
+            else
+                ++on_host;
+        }
+        const unsigned nth = (unsigned)std::min<size_t>({on_host, 16, std::max(1u, std::thread::hardware_concurrency())});
         std::vector<std::thread> th;
         for (unsigned w = 0; w < nth; ++w) {
             th.emplace_back([&, w] {
                 for (size_t bi = w; bi < blocks.size(); bi += nth)
-                    if (!blocks[bi].single && !blocks[bi].perm) compose_block(elems, blocks[bi], qb[bi], mb[bi]);
+                    if (!blocks[bi].single && !blocks[bi].perm && !on_device[bi]) compose_block(elems, blocks[bi], qb[bi], mb[bi]);
             });
         }
         for (auto &t : th) t.join();
@@ -607,6 +650,20 @@ static Status build_plan_ops(qi_plan *p, std::vector<Elem> &elems, bool ops) {
             pending_ops.clear();
             if (poly_ok) pending.init(n);
         };
+        auto emit = [&](const Op &op) {
+            p->ops.push_back(op);
+            p->stats.n_blocks_by_k[op.k]++;
+            if (op.tc_offset >= 0) {
+                ++tc_blocks_since;
+                ++tc_total;
+                if (p->opts.renorm_every > 0 && tc_blocks_since >= p->opts.renorm_every) {
+                    Op nrm;
+                    nrm.kind = OP_NORMALISE;
+                    p->ops.push_back(nrm);
+                    tc_blocks_since = 0;
+                }
+            }
+        };
         for (size_t bi = 0; bi < blocks.size(); ++bi) {
             const Block &b = blocks[bi];
             if (b.single) {
@@ -618,6 +675,19 @@ static Status build_plan_ops(qi_plan *p, std::vector<Elem> &elems, bool ops) {
                 flush();
                 p->ops.push_back(bitperm_op(elems, b));
                 p->stats.n_blocks_by_k[0]++;
+                continue;
+            }
+            if (on_device[bi]) {
+                flush();
+                Op op;
+                op.kind = OP_FUSED;
+                op.mode = use_tc;
+                op.mat_offset = 0;
+                for (uint64_t m = on_device[bi]; m; m &= m - 1) op.targets[op.k++] = __builtin_ctzll(m);
+                op.tc_offset = (int64_t)p->compose.words;
+                p->compose.ops.push_back(p->ops.size());
+                compose_job(elems, b, on_device[bi], p->compose);
+                emit(op);
                 continue;
             }
             bool diag = true;
@@ -656,18 +726,7 @@ static Status build_plan_ops(qi_plan *p, std::vector<Elem> &elems, bool ops) {
                     tc_blocks(kk, reinterpret_cast<const double *>(mb[bi].data()), p->tc);
                 }
             }
-            p->ops.push_back(op);
-            p->stats.n_blocks_by_k[op.k]++;
-            if (op.tc_offset >= 0) {
-                ++tc_blocks_since;
-                ++tc_total;
-                if (p->opts.renorm_every > 0 && tc_blocks_since >= p->opts.renorm_every) {
-                    Op nrm;
-                    nrm.kind = OP_NORMALISE;
-                    p->ops.push_back(nrm);
-                    tc_blocks_since = 0;
-                }
-            }
+            emit(op);
         }
         flush();
     }
@@ -678,6 +737,7 @@ static Status build_plan_ops(qi_plan *p, std::vector<Elem> &elems, bool ops) {
         nrm.kind = OP_NORMALISE;
         p->ops.push_back(nrm);
     }
+    finish_compose(p);
     p->stats.n_kernels = (int64_t)p->ops.size();
     return ok_status();
 }
@@ -690,7 +750,8 @@ Status upload_plan(qi_plan *p) {
     if (p->d_mats) { cudaFree(p->d_mats); p->d_mats = nullptr; }
     if (p->d_tc) { cudaFree(p->d_tc); p->d_tc = nullptr; }
     if (!p->tc.empty()) {
-        QI_CUDA(cudaMalloc(&p->d_tc, p->tc.size() * sizeof(float)));
+        QI_CUDA(cudaMalloc(&p->d_tc, (p->tc.size() + p->compose.words) * sizeof(float)));
+        p->composed = false;
         QI_CUDA(cudaMemcpy(p->d_tc, p->tc.data(), p->tc.size() * sizeof(float), cudaMemcpyHostToDevice));
     }
     if (p->mats.empty()) return ok_status();
@@ -852,6 +913,12 @@ Status plan_execute(qi_plan *p, qi_state *s) {
         if (!up.ok()) return up;
     }
     bool has_norm = false;
+    const bool compose = !runs && !p->compose.blocks.empty() && !p->composed;
+    if (compose) {
+        Status st = launch_compose(p, s);
+        if (!st.ok()) return st;
+        p->ops[p->compose.ops[0]].fresh_tc = p->composed = true;
+    }
     PlanRunner run(p, s);
     for (size_t i = 0; runs && i < p->sched.size(); ++i) {
         const RunSegment &seg = p->sched[i];
@@ -876,6 +943,7 @@ Status plan_execute(qi_plan *p, qi_state *s) {
         if (!st.ok()) return run.finish(st);
         has_norm = has_norm || op.kind == OP_PAULI_NORM;
     }
+    if (compose) p->ops[p->compose.ops[0]].fresh_tc = false;
     {
         Status st = run.finish(ok_status());
         if (!st.ok()) return st;
@@ -919,6 +987,7 @@ static qi_status plan_create(int32_t num_qubits, int32_t precision, const qi_gat
     p->n = num_qubits;
     p->prec = precision;
     if (opts) p->opts = *opts;
+    p->device_blocks = one_call;
     if (one_call) {   // the plan's build counts too: 40 layers, 22 qubits 0.7 + 2.9 ms as runs, 6 + 1.4 ms as blocks
         p->run_min = 4;
         p->run_max = 23;
@@ -1275,6 +1344,7 @@ qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_t
         plan.n = s->n;
         plan.prec = s->prec;
         plan.opts.use_tensor_cores = unitary ? 0 : 2;
+        plan.device_blocks = true;
         // A plan for one call: composing its blocks takes 1.2 ms and more (177-term lattice), so gate runs win
         // up to 20 qubits, and above that for as many steps as cost less than that in slower passes (XYZ
         // lattice, ms, runs / blocks: 20 qubits 20 steps 3.3 / 4.2; 22 qubits 5 steps 2.1 / 2.2, 20 steps

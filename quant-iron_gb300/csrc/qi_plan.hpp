@@ -55,6 +55,27 @@ struct RunSegment {
     std::vector<RunPass> passes;
 };
 
+// Blocks composed on the device (qi_compose.cu): a matrix per block, members multiplied on from the left.
+struct ComposeMember {
+    uint32_t off;               // its matrix: 2^m x 2^m complex numbers from this one of the data
+    uint8_t m, pos[6];          // local bits of the block it acts on
+    uint8_t pad[5];
+};
+struct ComposeBlock {
+    uint64_t tc;                // operand blocks: word of the plan's device words
+    uint32_t first, count;      // members
+    uint32_t k, pad;
+};
+static_assert(sizeof(ComposeMember) == 16 && sizeof(ComposeBlock) == 24, "read as such by the device");
+struct ComposeJobs {
+    std::vector<ComposeBlock> blocks;
+    std::vector<ComposeMember> members;
+    std::vector<std::complex<double>> data;
+    std::vector<size_t> ops;    // the blocks' ops
+    size_t at_blocks = 0, at_members = 0, at_data = 0;   // words
+    size_t words = 0;           // of the operand blocks
+};
+
 }  // namespace qi
 
 struct qi_plan {
@@ -67,6 +88,10 @@ struct qi_plan {
     std::vector<float> tc;                    // FP32 device blocks: tensor-core operands (fused ops, k >= 5)
                                               // and phase-polynomial blocks, as raw 32-bit words
     void *d_tc = nullptr;
+    // A plan for one state's use in one call: operand blocks are composed on the device, before the first
+    // execution; its ops have no host matrices.
+    bool device_blocks = false, composed = false;
+    qi::ComposeJobs compose;
     std::vector<qi::PhasePoly> polys;         // host copy of each OP_PHASE_POLY op (op.mat_offset indexes it)
     // Per-gate plans: how the ops are executed (several to a pass), and the passes' programs.
     std::vector<qi::RunSegment> sched;
@@ -89,6 +114,8 @@ struct qi_plan {
 namespace qi {
 Status build_plan(qi_plan *p, std::vector<Elem> &elems);
 Status upload_plan(qi_plan *p);
+void finish_compose(qi_plan *p);
+Status launch_compose(qi_plan *p, qi_state *s);
 void release_runs(qi_plan *p);
 Status plan_execute(qi_plan *p, qi_state *s);
 Status plan_elems_from_gates(int n, const qi_gate *gates, int64_t ng, const double *theta, int64_t ntheta,
