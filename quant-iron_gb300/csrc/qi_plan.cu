@@ -437,9 +437,9 @@ static void build_schedule(qi_plan *p, const std::vector<Elem> &elems, const std
 // Plans that execute as gate runs from end to end, without looking at their ops: per-gate plans whose
 // every element a pass can apply, and FP32 fused plans of run_min to run_max qubits for which the
 // caller chose neither block size nor tensor cores.  A tensor-core block of a small state fills a few of
-// the SMs (17 qubits: 16 tiles) for 8 to 16 us; 40 layers + QFT, fused blocks / gate runs, among others and
-// alone (us): 10 qubits 103 / 70, 265 / 217; 12 qubits 194 / 98, 569 / 296; 17 qubits 226 / 174, 621 / 460;
-// 18 qubits 240 / 224, 657 / 500; 19 qubits 277 / 330, 722 / 594; 20 qubits 429 / 585, 769 / 900.  The
+// the SMs (17 qubits: 16 tiles) for 4 to 8 us; 40 layers + QFT, fused blocks / gate runs, among others and
+// alone (us): 13 qubits 125 / 107, 323 / 323; 15 qubits 152 / 127, 395 / 374; 16 qubits 160 / 140, 420 / 420;
+// 17 qubits 174 / 165, 445 / 438; 18 qubits 180 / 216, 462 / 471.  The
 // ops (with the fused blocks' matrices, most of a plan's build time) are made when something asks for them.
 
 static bool build_runs(qi_plan *p, const std::vector<Elem> &elems, int fusion, int kmax) {
@@ -988,12 +988,17 @@ static qi_status plan_create(int32_t num_qubits, int32_t precision, const qi_gat
     p->prec = precision;
     if (opts) p->opts = *opts;
     p->device_blocks = one_call;
-    if (one_call) {   // the plan's build counts too: 40 layers, 22 qubits 0.7 + 2.9 ms as runs, 6 + 1.4 ms as blocks
-        p->run_min = 4;
-        p->run_max = 23;
-    }
     std::vector<Elem> elems;
     Status st = plan_elems_from_gates(num_qubits, gates, n_gates, theta, n_theta, elems);
+    // The plan's build counts too, 1.3-1.7 ms for blocks, so gate runs win until their slower passes have cost
+    // as much: 4 / 10 / 20 / 40 layers, runs and (blocks), us: 20 qubits 486 / 720 / 1159 / 1981 (1661 / 1868 /
+    // 2183 / 2726); 21 qubits 640 / 1018 / 1628 / 2829 (1764 / 1848 / 2195 / 2781); 22 qubits 927 / 1463 / 2371 /
+    // 4156 (1860 / 2055 / 2486 / 3226); 23 qubits 1559 / 2458 / 4054 / 7189 (2172 / 2386 / 3129 / 3976): even at
+    // about 1700 gates of 21 qubits (40 layers), half as many a qubit more.
+    if (one_call) {
+        p->run_min = 4;
+        if (num_qubits <= 23 && std::ldexp((double)elems.size(), num_qubits - 21) <= 1700.0) p->run_max = 23;
+    }
     if (st.ok()) st = build_plan(p, elems);
     if (!st.ok()) { delete p; return publish(st); }
     *out = p;
@@ -1345,13 +1350,17 @@ qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_t
         plan.prec = s->prec;
         plan.opts.use_tensor_cores = unitary ? 0 : 2;
         plan.device_blocks = true;
-        // A plan for one call: composing its blocks takes 1.2 ms and more (177-term lattice), so gate runs win
-        // up to 20 qubits, and above that for as many steps as cost less than that in slower passes (XYZ
-        // lattice, ms, runs / blocks: 20 qubits 20 steps 3.3 / 4.2; 22 qubits 5 steps 2.1 / 2.2, 20 steps
-        // 8.2 / 5.3; 24 qubits 1 step 1.8 / 2.1, 5 steps 8.6 / 4.8)
+        // FP32: gate runs cost by the exponential, blocks by the step (about 10 blocks of a lattice, whether it
+        // has 50 terms or 140) and by the plan (composing).  Per call, us, runs / blocks: 20 qubits, 113-term
+        // XYZ, 1 step 228 / 239, 5 steps 823 / 680, 51-term TFIM, 20 steps 1423 / 2292; 21 qubits, XYZ 332 / 378
+        // and 1336 / 816, TFIM 2231 / 2655; 22 qubits XYZ, 1 step 474 / 406, TFIM, 2 and 10 steps 403 / 554,
+        // 1819 / 1580; 24 qubits, XYZ and TFIM, 1 step 1786 / 823, 667 / 712; second order, 20 qubits XYZ, 1 and 5
+        // steps 370 / 554, 1286 / 1256.  The constants below are fitted to these.
+        const double size = std::ldexp(1.0, s->n - 20), halves = (double)(order * num_steps), nt = (double)n_terms;
+        const double runs = halves * nt * (0.65 + 0.68 * size);
+        const double blocks = 150.0 * order + halves * std::max(1.0, nt / 140.0) * std::max(110.0, 33.0 * size);
         plan.run_min = 4;
-        plan.run_max = 20;
-        while (plan.run_max < 24 && num_steps <= (int64_t)20 >> (plan.run_max + 1 - 20)) ++plan.run_max;
+        plan.run_max = runs <= blocks ? s->n : 0;
         plan.opts.renorm_every = unitary ? 0 : -1;
         plan.opts.max_block_qubits = 0;
         std::vector<Elem> elems = step_list(steps);
