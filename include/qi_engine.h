@@ -314,7 +314,7 @@ typedef struct qi_exec_options {
     int32_t fusion;            /* QI_FUSION_* */
     int32_t max_block_qubits;  /* k <= 6; 0 = default (6) */
     int32_t use_tensor_cores;  /* 0 (default) or 1: 3xTF32 tcgen05 kernel for FP32 blocks of k >= 5; 2: CUDA cores only.
-                                  0 with max_block_qubits 0: greedy FP32 plans of 10 to 17 qubits execute as passes
+                                  0 with max_block_qubits 0: greedy FP32 plans of 10 to 12 qubits execute as passes
                                   over their gates instead of blocks (qi_plan_run_info), which is faster there */
     int32_t renorm_every;      /* FP64 renormalisation on the device: 0 = once at the end when tensor-core
                                   blocks ran (their FP32 accumulation rounds toward zero, so the norm drifts

@@ -749,11 +749,12 @@ static Status launch_tc_t(qi_state *s, const TileGeom &g, const void *d_tc, cons
     }
     uint64_t grid = g.ntiles;   // one persistent CTA per SM
     if (grid > (uint64_t)num_sms) grid = (uint64_t)num_sms;
-    // Over all SMs, a block's setup (operand blocks, barriers, tensor memory) overlaps the end of the kernel
-    // before it (programmatic launch; not behind the kernel that writes the operand blocks); a smaller grid would hold SMs that other streams can use.  With the
-    // operand blocks as one copy beside the first tile's: 20 layers of 20 / 22 / 24 / 27 qubits 0.46 / 0.75 /
-    // 2.06 / 8.27 -> 0.36 / 0.53 / 1.73 / 8.03 ms.
-    ChainedLaunch at((unsigned)grid, kTcThreads, C::SMEM, s->stream, grid == (uint64_t)num_sms && !fresh);
+    // A block's setup (operand blocks, barriers, tensor memory) overlaps the end of the kernel before it, but
+    // for the kernel that writes the operand blocks.  With the operand blocks as one copy beside the first
+    // tile's: 20 layers of 20 / 22 / 24 / 27 qubits 0.46 / 0.75 / 2.06 / 8.27 -> 0.36 / 0.53 / 1.73 / 8.03 ms.
+    // Also where the grid leaves SMs free, although its successor then waits on them: 40 layers of 18 qubits,
+    // alone 462 -> 320 us, among three streams 178 -> 125; 20 qubits 531 -> 420 and 355 -> 356.
+    ChainedLaunch at((unsigned)grid, kTcThreads, C::SMEM, s->stream, !fresh);
     QI_CUDA(cudaLaunchKernelEx(&at.cfg, k_fused_tc<K, ROT, PHASE>, (float2 *)s->amps, (const float *)d_tc, g, s->d_flag,
                                (const uint32_t *)poly));
     count_launch();

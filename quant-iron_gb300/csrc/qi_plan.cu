@@ -436,10 +436,10 @@ static void build_schedule(qi_plan *p, const std::vector<Elem> &elems, const std
 
 // Plans that execute as gate runs from end to end, without looking at their ops: per-gate plans whose
 // every element a pass can apply, and FP32 fused plans of run_min to run_max qubits for which the
-// caller chose neither block size nor tensor cores.  A tensor-core block of a small state fills a few of
-// the SMs (17 qubits: 16 tiles) for 4 to 8 us; 40 layers + QFT, fused blocks / gate runs, among others and
-// alone (us): 13 qubits 125 / 107, 323 / 323; 15 qubits 152 / 127, 395 / 374; 16 qubits 160 / 140, 420 / 420;
-// 17 qubits 174 / 165, 445 / 438; 18 qubits 180 / 216, 462 / 471.  The
+// caller chose neither block size nor tensor cores.  Below 13 qubits blocks of six do not fit the
+// tensor-core kernel's tiles; 40 layers + QFT, fused blocks / gate runs, among others and alone (us): 10 qubits
+// 103 / 71, 264 / 220; 12 qubits 193 / 97, 560 / 300; 13 qubits 76 / 107, 210 / 322; 15 qubits 100 / 128, 266 /
+// 376; 17 qubits 115 / 164, 307 / 433 (8 and 9 qubits, where a block covers most of the state, about even).  The
 // ops (with the fused blocks' matrices, most of a plan's build time) are made when something asks for them.
 
 static bool build_runs(qi_plan *p, const std::vector<Elem> &elems, int fusion, int kmax) {
@@ -1352,13 +1352,15 @@ qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_t
         plan.device_blocks = true;
         // FP32: gate runs cost by the exponential, blocks by the step (about 10 blocks of a lattice, whether it
         // has 50 terms or 140) and by the plan (composing).  Per call, us, runs / blocks: 20 qubits, 113-term
-        // XYZ, 1 step 228 / 239, 5 steps 823 / 680, 51-term TFIM, 20 steps 1423 / 2292; 21 qubits, XYZ 332 / 378
-        // and 1336 / 816, TFIM 2231 / 2655; 22 qubits XYZ, 1 step 474 / 406, TFIM, 2 and 10 steps 403 / 554,
-        // 1819 / 1580; 24 qubits, XYZ and TFIM, 1 step 1786 / 823, 667 / 712; second order, 20 qubits XYZ, 1 and 5
-        // steps 370 / 554, 1286 / 1256.  The constants below are fitted to these.
+        // XYZ, 1 step 230 / 359, 5 steps 822 / 733, 51-term TFIM, 20 steps 1413 / 2028; 18 qubits XYZ, 10 and 20
+        // steps 851 / 943, 1612 / 1635; 21 qubits, XYZ, 1 and 5 steps 329 / 372, 1329 / 815, TFIM, 20 steps 2229 /
+        // 2820; 22 qubits XYZ, 1 step 474 / 406, TFIM, 2 and 10 steps 403 / 554, 1819 / 1580; 24 qubits, XYZ and
+        // TFIM, 1 step 1786 / 823, 667 / 712; second order, 20 qubits XYZ, 2 and 5 steps 599 / 662, 1286 / 1103.
+        // The constants below are fitted to these.
         const double size = std::ldexp(1.0, s->n - 20), halves = (double)(order * num_steps), nt = (double)n_terms;
         const double runs = halves * nt * (0.65 + 0.68 * size);
-        const double blocks = 150.0 * order + halves * std::max(1.0, nt / 140.0) * std::max(110.0, 33.0 * size);
+        const double pass = std::max({55.0, 15.0 * (s->n - 14), 33.0 * size});
+        const double blocks = 250.0 * order + halves * std::max(1.0, nt / 140.0) * pass;
         plan.run_min = 4;
         plan.run_max = runs <= blocks ? s->n : 0;
         plan.opts.renorm_every = unitary ? 0 : -1;

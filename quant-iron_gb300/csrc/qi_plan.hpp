@@ -100,7 +100,7 @@ struct qi_plan {
     bool run_normalise = false;   // a renormalisation follows the runs
     // ops not made yet (every op is in a run): what they are made from
     bool lazy = false;
-    int32_t run_min = 10, run_max = 17;   // qubits of an FP32 fused plan that executes as gate runs
+    int32_t run_min = 10, run_max = 12;   // qubits of an FP32 fused plan that executes as gate runs
     std::vector<qi::Elem> lazy_elems;
     std::vector<qi::Block> lazy_blocks;
     int32_t run_device = -1;
