@@ -25,8 +25,9 @@ namespace qi {
 // unmeasured qubits are then added by shuffles, and the sums of threads that differ in the other
 // unmeasured thread bits (chunks) by k_meas_reduce, always in the same order.
 // Measured (measure_n, 4096 shots, host call to result; before: one block per outcome and chunk gathering
-// its amplitudes): FP64 22 qubits, 10 measured 463 -> 77 us, all 22 measured 153 -> 15 ms; FP32 24 qubits, 16
-// measured 2.4 -> 0.33 ms.  The sums are bound by the FP64 pipe (3 operations per amplitude).
+// its amplitudes): FP64 22 qubits, 10 measured 463 -> 72 us, all 22 measured 153 -> 15 ms; FP32 24 qubits, 16
+// measured 2.4 -> 0.33 ms.  The FP64 sums are bound by the FP64 pipe: two fused operations per amplitude (as
+// three the 22-qubit measurement with its collapse took 80 us, now 66).
 struct MeasGeom {
     int32_t nthread;         // thread-index bits
     int32_t nlane;           // of them within a warp
@@ -51,7 +52,7 @@ __global__ void __launch_bounds__(256) k_meas_sum(const typename Cx<T>::V2 *a, c
         if (p >= 64) chunk |= bit << (p - 64);
         else if (p >= 0) out |= bit << p;
     }
-    double acc = 0.0;
+    double acc = 0.0, acc2 = 0.0;
     uint64_t off = 0;
     do {   // subsets of the loop mask, ascending
         if constexpr (sizeof(T) == 4) {
@@ -70,10 +71,14 @@ __global__ void __launch_bounds__(256) k_meas_sum(const typename Cx<T>::V2 *a, c
                 if (u < g.unroll) v[u] = a[base | off | g.off[u]];
 #pragma unroll
             for (int u = 0; u < 8; ++u)
-                if (u < g.unroll) acc += v[u].x * v[u].x + v[u].y * v[u].y;
+                if (u < g.unroll) {   // two FP64 operations an amplitude: they bound this pass
+                    acc = ::fma(v[u].x, v[u].x, acc);
+                    acc2 = ::fma(v[u].y, v[u].y, acc2);
+                }
         }
         off = ((off | ~g.loop) + 1) & g.loop;
     } while (off);
+    acc += acc2;
     const unsigned lanes = g.nlane >= 5 ? 0xffffffffu : (1u << (1 << g.nlane)) - 1u;
     for (int j = 0; j < g.nlane; ++j)
         if ((g.lane_free >> j) & 1u) acc += __shfl_xor_sync(lanes, acc, 1 << j);
