@@ -762,7 +762,8 @@ def main():
     n_groups = len({(int(t["xmask"])) for t in terms})
     expectation = {"terms": len(terms), "x_groups": n_groups, "ms": min(ex_t) * 1e3,
                    "passes_gbs": n_groups * (1 << n) * 8 / min(ex_t) / 1e9,
-                   "note": "one read pass of the FP32 state per X-mask group, host call to result (synchronous)"}
+                   "note": "host call to result (synchronous); the rate counts one read of the FP32 state per X-mask "
+                           "group, of which a pass of the engine serves many"}
 
     extra = {}
     if rank == 0 and not args.skip_baselines:

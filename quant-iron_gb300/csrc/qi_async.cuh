@@ -48,14 +48,20 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
 }
 
 // Bounded wait that also gives up when another role raised the abort flag;
-// a timeout raises it and records status 2 in the state's error flag.
-__device__ __forceinline__ bool wait_or_abort(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *err_flag) {
+// a timeout raises it and records status 2 in the state's error flag.  started (if given): set once the
+// stream's earlier work has ended; the time before that does not count.
+__device__ __forceinline__ bool wait_or_abort(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *err_flag,
+                                              const volatile int *started = nullptr) {
     if (mbar_try_wait(bar, parity)) return true;
-    const uint64_t t0 = global_ns();
+    uint64_t t0 = global_ns();
     for (uint32_t i = 0; i < kWaitLimit; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
         if ((i & 31u) == 31u) {
             if (*abort_flag) return false;
+            if (started && !*started) {
+                t0 = global_ns();
+                i = 0;
+            }
             if (global_ns() - t0 > kWaitNs) break;
         }
     }

@@ -185,7 +185,7 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 // Warp-uniform form: every lane waits, the warp proceeds only if all saw the phase.
 __device__ __forceinline__ bool warp_wait_or_abort(uint64_t *bar, uint32_t parity, volatile int *abort_flag,
                                                    int *err_flag) {
-    const bool ok = wait_or_abort(bar, parity, abort_flag, err_flag);
+    const bool ok = wait_or_abort(bar, parity, abort_flag, err_flag, abort_flag + 1);   // the started flag
     return __all_sync(0xffffffffu, ok);
 }
 
@@ -283,8 +283,12 @@ __device__ __forceinline__ void st_cs_v8(float2 *p, float a0, float a1, float a2
 // chunk's row pairs starting at its own (lane mod 8), undone in registers.
 // PHASE: a diagonal phase polynomial exp(2 pi i f(x)) that follows the block in the plan is
 // applied by the epilogue before the store (its phase table at `poly`, tc_phase_table).
+// At most 112 registers a thread: the four of the 14 warps that share an SM quarter then leave it room for two
+// warps of 32 registers, so the blocks that read an upload over the link (k_convert_link) run beside this
+// kernel.  With 113 they wait for an SM: 30-qubit circuits through host buffers 300 ms a step instead of
+// 228-240 (the circuit alone 204 instead of 207).
 template <int K, bool ROT, bool PHASE>
-__global__ void __launch_bounds__(kTcThreads, 1) k_fused_tc(float2 *a, const float *blocks, TileGeom g, int *err_flag,
+__global__ void __maxnreg__(112) k_fused_tc(float2 *a, const float *blocks, TileGeom g, int *err_flag,
                                                             const uint32_t *__restrict__ poly) {
     using C = TcCfg<K>;
     constexpr int R = C::R, NB = C::NBUF;
@@ -331,7 +335,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_fused_tc(float2 *a, const flo
         }
         mbar_init(mma_done, 1);
         mbar_init(b_full, 1);
-        *abort_flag = 0;
+        abort_flag[0] = abort_flag[1] = 0;   // abort, started
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == 0) tmem_alloc(tmem_slot, C::TMEM_COLS);
@@ -531,10 +535,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_fused_tc(float2 *a, const flo
             mbar_arrive_expect_tx(b_full, (uint32_t)C::OFF_TILES);
             bulk_load(sB, blocks, (uint32_t)C::OFF_TILES, b_full);
         }
-        // The amplitudes are the earlier kernels'; the operand blocks and phase tables are not.  The next
-        // kernel of the stream may start its own prologue from here on (it waits likewise).
+        // The amplitudes are the earlier kernels'; the operand blocks and phase tables are not.  This warp alone
+        // waits for them: everything that touches amplitudes follows from its copies, and a wait in every
+        // thread cost 0.8 us a launch (40 layers of 17 qubits 311 -> 343 us).  The next kernel of the stream
+        // may start its own set-up from here on.
         launch_wait();
         launch_next();
+        if (lane == 0) abort_flag[1] = 1;   // started: the other roles' waits count from here
         const uint32_t run_bytes = (uint32_t)sizeof(float2) << g.L;
         const int nruns = 1 << g.nhigh;
         int issued = 0;
@@ -753,8 +760,11 @@ static Status launch_tc_t(qi_state *s, const TileGeom &g, const void *d_tc, cons
     // for the kernel that writes the operand blocks.  With the operand blocks as one copy beside the first
     // tile's: 20 layers of 20 / 22 / 24 / 27 qubits 0.46 / 0.75 / 2.06 / 8.27 -> 0.36 / 0.53 / 1.73 / 8.03 ms.
     // Also where the grid leaves SMs free, although its successor then waits on them: 40 layers of 18 qubits,
-    // alone 462 -> 320 us, among three streams 178 -> 125; 20 qubits 531 -> 420 and 355 -> 356.
-    ChainedLaunch at((unsigned)grid, kTcThreads, C::SMEM, s->stream, !fresh);
+    // alone 462 -> 320 us, among three streams 178 -> 125; 20 qubits 531 -> 420 and 355 -> 356.  Not for launches
+    // of more than 32 tiles an SM (26 qubits on: 0-3 % to gain): the waiting kernel takes every SM as it comes
+    // free, and other streams' conversions and copies wait for the plan's end (30-qubit circuits through host
+    // buffers 320 ms a step instead of 240).
+    ChainedLaunch at((unsigned)grid, kTcThreads, C::SMEM, s->stream, !fresh && g.ntiles <= 32ull * (uint64_t)num_sms);
     QI_CUDA(cudaLaunchKernelEx(&at.cfg, k_fused_tc<K, ROT, PHASE>, (float2 *)s->amps, (const float *)d_tc, g, s->d_flag,
                                (const uint32_t *)poly));
     count_launch();

@@ -3,7 +3,7 @@
 // A per-gate plan applies each gate with the gate's own arithmetic (2x2 updates of amplitude
 // pairs, phases, index exchanges), not with composed matrices.  One kernel per gate streams the
 // whole state for every gate; here the host cuts the gate list into passes.  A pass holds the
-// amplitudes of a tile (up to 2^12 16-byte units) in shared memory and applies every gate whose
+// amplitudes of a tile (up to 2^11 16-byte units) in shared memory and applies every gate whose
 // non-diagonal qubits are local to the tile; diagonal factors and controls may sit on any qubit
 // (they are conditions on the amplitude index).  Inside a pass the gates are grouped into phases:
 // a thread holds the 2^r units that differ in r of the tile's bits and applies all of the phase's
@@ -220,7 +220,8 @@ Status launch_run_pass(qi_state *s, const RunPass &p, const void *d_prog) {
     }
     // A pass's setup (row table, program) overlaps the end of the pass before it: 20 layers of FP64, 12 / 16 /
     // 20 qubits 0.255 / 0.351 / 1.503 -> 0.239 / 0.328 / 1.458 ms; FP32, 17 qubits 0.255 -> 0.229 ms.
-    ChainedLaunch at(blocks, threads, sm, s->stream);
+    // From 4096 tiles on there is nothing left to gain, and other streams' kernels find SMs between passes.
+    ChainedLaunch at(blocks, threads, sm, s->stream, blocks <= 4096);
     if (f32) QI_CUDA(cudaLaunchKernelEx(&at.cfg, k_gate_run<float>, (float2 *)s->amps, prog, g));
     else QI_CUDA(cudaLaunchKernelEx(&at.cfg, k_gate_run<double>, (double2 *)s->amps, prog, g));
     count_launch();
