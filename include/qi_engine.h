@@ -306,9 +306,10 @@ qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_t
 #define QI_FUSION_NONE    0  /* one kernel per gate (the plain per-gate method) */
 #define QI_FUSION_GREEDY  1  /* greedy fixed-k fuser, k = max_block_qubits */
 #define QI_FUSION_LEARNED 2  /* partitions scored by the learned cost model (greedy fallback) */
-#define QI_FUSION_PAULI_GROUPS 3  /* one kernel per gate, except that each run of Pauli exponentials
+#define QI_FUSION_PAULI_GROUPS 3  /* as NONE, except that each run of Pauli exponentials
                                      (Gate::PauliTimeEvolution) whose X-masks lie in {0, X} is one
-                                     pass (FP64 Trotter steps use this) */
+                                     operation (FP64 Trotter steps with exponentials that a pass over
+                                     many gates cannot take use this) */
 
 typedef struct qi_exec_options {
     int32_t fusion;            /* QI_FUSION_* */
