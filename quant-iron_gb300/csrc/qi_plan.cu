@@ -746,13 +746,20 @@ static bool not_uploaded(const qi_plan *p) {
     return (!p->d_mats && !p->mats.empty()) || (!p->d_tc && !p->tc.empty());
 }
 
+// A copy that has arrived when it returns: cudaMemcpy of pageable memory may return while its last part is
+// still on its way in the default stream, which the states' (non-blocking) streams do not wait for.
+static cudaError_t copy_in(void *d, const void *h, size_t bytes) {
+    const cudaError_t e = cudaMemcpy(d, h, bytes, cudaMemcpyHostToDevice);
+    return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 Status upload_plan(qi_plan *p) {
     if (p->d_mats) { cudaFree(p->d_mats); p->d_mats = nullptr; }
     if (p->d_tc) { cudaFree(p->d_tc); p->d_tc = nullptr; }
     if (!p->tc.empty()) {
         QI_CUDA(cudaMalloc(&p->d_tc, (p->tc.size() + p->compose.words) * sizeof(float)));
         p->composed = false;
-        QI_CUDA(cudaMemcpy(p->d_tc, p->tc.data(), p->tc.size() * sizeof(float), cudaMemcpyHostToDevice));
+        QI_CUDA(copy_in(p->d_tc, p->tc.data(), p->tc.size() * sizeof(float)));
     }
     if (p->mats.empty()) return ok_status();
     const size_t cnt = p->mats.size();
@@ -760,12 +767,12 @@ Status upload_plan(qi_plan *p) {
         std::vector<float2> h(cnt);
         for (size_t i = 0; i < cnt; ++i) h[i] = make_float2((float)p->mats[i].real(), (float)p->mats[i].imag());
         QI_CUDA(cudaMalloc(&p->d_mats, cnt * sizeof(float2)));
-        QI_CUDA(cudaMemcpy(p->d_mats, h.data(), cnt * sizeof(float2), cudaMemcpyHostToDevice));
+        QI_CUDA(copy_in(p->d_mats, h.data(), cnt * sizeof(float2)));
     } else {
         std::vector<double2> h(cnt);
         for (size_t i = 0; i < cnt; ++i) h[i] = make_double2(p->mats[i].real(), p->mats[i].imag());
         QI_CUDA(cudaMalloc(&p->d_mats, cnt * sizeof(double2)));
-        QI_CUDA(cudaMemcpy(p->d_mats, h.data(), cnt * sizeof(double2), cudaMemcpyHostToDevice));
+        QI_CUDA(copy_in(p->d_mats, h.data(), cnt * sizeof(double2)));
     }
     return ok_status();
 }
@@ -811,7 +818,7 @@ static bool runs_ready(qi_plan *p, qi_state *s) {
         (void)cudaGetLastError();
         return false;
     }
-    if (cudaMemcpy(d, p->run_prog.data(), p->run_prog.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (copy_in(d, p->run_prog.data(), p->run_prog.size()) != cudaSuccess) {
         (void)cudaGetLastError();
         cudaFree(d);
         return false;
