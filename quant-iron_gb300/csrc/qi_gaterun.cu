@@ -213,7 +213,8 @@ Status launch_run_pass(qi_state *s, const RunPass &p, const void *d_prog) {
     const size_t sm = run_smem(p, ub0);
     const unsigned threads = 1u << (ubits - kRunSelBits), blocks = (unsigned)(s->dim() >> p.tbits);
     const uint4 *prog = reinterpret_cast<const uint4 *>((const char *)d_prog + p.prog_off);
-    if (sm > 48 * 1024) {
+    // The default limit of 48 KB counts the kernel's static block (the slots) too.
+    if (sm + kRunMaxSlots * sizeof(double2) > 48 * 1024) {
         constexpr int cap = (16 << kRunTileBits) + (8 << kRunTileBits) + kRunMaxProg;   // every pass's bound
         if (f32) QI_CUDA(cudaFuncSetAttribute(k_gate_run<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));
         else QI_CUDA(cudaFuncSetAttribute(k_gate_run<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));
