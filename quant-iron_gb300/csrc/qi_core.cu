@@ -466,7 +466,9 @@ Status read_end(qi_state *dst, const qi_state *src) {
 // there.  Destroyed handles of up to kCacheState bytes are kept, at most kCacheHandles of them and
 // kCacheBytes in all (the oldest goes first), and taken over by the next handle of the same size,
 // precision and device.  The new owner works on the same stream, so its work is ordered behind
-// whatever the old owner and the readers of its buffer (read_end) still have in flight.  Handles whose
+// whatever the old owner and the readers of its buffer (read_end) still have in flight; before the
+// buffer can be reached from another stream (its pointer or stream handed out, a caller's stream
+// taken in) that stream is waited for (hand_out).  Handles whose
 // buffer or stream was handed out are freed as ever; a handle that moved host data is waited for.
 // An allocation that fails empties the cache first; qi_cache_trim does so on request.
 constexpr size_t kCacheState = 8u << 20, kCacheBytes = 64u << 20;
@@ -557,6 +559,14 @@ cudaError_t device_malloc(void **p, size_t bytes) {
     (void)cudaGetLastError();
     cache_clear();
     return cudaMalloc(p, bytes);
+}
+
+// The caller may use the handle's buffer on a stream of its own from here on.
+static Status hand_out(qi_state *s) {
+    s->exposed = true;
+    if (s->recycled) QI_CUDA(cudaStreamSynchronize(s->own_stream));
+    s->recycled = false;
+    return ok_status();
 }
 
 Status state_workspace(qi_state *s, size_t bytes, void **out, bool program) {
@@ -686,6 +696,7 @@ qi_status qi_state_create(int32_t num_qubits, int32_t precision, qi_state **out)
     if (e != cudaSuccess) return publish(cuda_status(e, "cudaSetDevice"));
     if (qi_state *s = cache_take(num_qubits, precision, g_device)) {
         s->host_io = false;
+        s->recycled = true;
         if ((e = cudaMemsetAsync(s->d_flag, 0, sizeof(int), s->stream)) != cudaSuccess) {
             free_handle(s);
             return publish(cuda_status(e, "memset"));
@@ -744,23 +755,23 @@ qi_status qi_state_info(const qi_state *s, int32_t *num_qubits, int32_t *precisi
 
 qi_status qi_state_set_stream(qi_state *s, void *cuda_stream) {
     QI_GUARD(s);
-    s->exposed = true;
-    s->stream = cuda_stream ? (cudaStream_t)cuda_stream : s->own_stream;
-    return publish(ok_status());
+    Status st = hand_out(s);
+    if (st.ok()) s->stream = cuda_stream ? (cudaStream_t)cuda_stream : s->own_stream;
+    return publish(st);
 }
 
 qi_status qi_state_get_stream(qi_state *s, void **cuda_stream) {
     QI_GUARD(s);
-    s->exposed = true;
+    Status st = hand_out(s);
     if (cuda_stream) *cuda_stream = (void *)s->stream;
-    return publish(ok_status());
+    return publish(st);
 }
 
 qi_status qi_state_device_ptr(qi_state *s, void **dev_ptr) {
     QI_GUARD(s);
-    s->exposed = true;
+    Status st = hand_out(s);
     if (dev_ptr) *dev_ptr = s->amps;
-    return publish(ok_status());
+    return publish(st);
 }
 
 qi_status qi_state_wait(qi_state *s, qi_state *other) {

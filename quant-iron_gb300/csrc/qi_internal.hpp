@@ -74,6 +74,7 @@ struct qi_state {
     cudaEvent_t ev = nullptr;         // position of this handle's stream, for other handles' streams to wait on
     bool exposed = false;             // its buffer or stream was handed out, or the caller's stream came in
     bool host_io = false;             // a host buffer may still be in use by its stream
+    bool recycled = false;            // own_stream may still hold an earlier owner's work, and waits for readers of its buffer
 
     uint64_t dim() const { return 1ull << n; }
     size_t amp_bytes() const { return prec == QI_F64 ? 16 : 8; }
