@@ -58,9 +58,14 @@ __device__ static inline float4 ldg_stream(const float4 *p) { return __ldcs(p); 
 __device__ static inline double2 ldg_stream(const double2 *p) { return __ldcs(p); }
 __device__ static inline float2 ldg_stream(const float2 *p) { return __ldcs(p); }
 
-// Block-wide sum of one double (blockDim.x a multiple of 32, <= 1024).
+// Block-wide sum of one double (blockDim.x a multiple of 32, <= 1024, or 1, 2, 4, 8 or 16).
 __device__ static inline double block_sum(double v) {
     __shared__ double warp_part[32];
+    if (blockDim.x < 32) {   // less than a warp: only the lanes that exist take part
+        const unsigned lanes = (1u << blockDim.x) - 1u;
+        for (unsigned o = blockDim.x >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(lanes, v, o);
+        return v;
+    }
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     __syncthreads();   // warp_part may still be read by a previous call
