@@ -446,15 +446,29 @@ Status state_scratch(qi_state *s, void **out) {
     return ok_status();
 }
 
+// Whether one of the streams is being captured without the other: no event can order them then.  (Own streams
+// that nobody was given are not captured.)
+static bool one_captured(const qi_state *a, const qi_state *b) {
+    if (!a->exposed && !b->exposed) return false;
+    cudaStreamCaptureStatus ca = cudaStreamCaptureStatusNone, cb = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(a->stream, &ca) != cudaSuccess || cudaStreamIsCapturing(b->stream, &cb) != cudaSuccess)
+        (void)cudaGetLastError();
+    return (ca == cudaStreamCaptureStatusNone) != (cb == cudaStreamCaptureStatusNone);
+}
+
 Status read_begin(qi_state *dst, const qi_state *src) {
     if (src->stream == dst->stream) return ok_status();
+    if (one_captured(dst, src)) {   // the host waits: what the graph reads later is the caller's to order
+        QI_CUDA(cudaStreamSynchronize(src->stream));
+        return ok_status();
+    }
     QI_CUDA(cudaEventRecord(src->ev, src->stream));
     QI_CUDA(cudaStreamWaitEvent(dst->stream, src->ev, 0));
     return ok_status();
 }
 
 Status read_end(qi_state *dst, const qi_state *src) {
-    if (src->stream == dst->stream) return ok_status();
+    if (src->stream == dst->stream || one_captured(dst, src)) return ok_status();
     QI_CUDA(cudaEventRecord(dst->ev, dst->stream));
     QI_CUDA(cudaStreamWaitEvent(src->stream, dst->ev, 0));
     return ok_status();

@@ -91,7 +91,8 @@ Status state_normalise_device_async(qi_state *s);   // norm on device, divides i
 Status state_read_flag(qi_state *s, int *flag);      // sync; resets the flag
 Status state_copy_async(qi_state *dst, const qi_state *src);
 // Around work on dst's stream that reads src's buffer: dst's stream waits for the work issued on src, and
-// src's later work (and the next owner of its buffer) waits for the read.
+// src's later work (and the next owner of its buffer) waits for the read.  While one of the two streams alone is
+// being captured, the host waits for src's stream instead.
 Status read_begin(qi_state *dst, const qi_state *src);
 Status read_end(qi_state *dst, const qi_state *src);
 // cudaMalloc; on failure the cached handles are freed and it is tried once more.
