@@ -159,6 +159,8 @@ static Status basis_change(qi_state *s, int basis, const double *u, const int32_
     return st;
 }
 
+constexpr size_t kKeptSums = 2u << 20;
+
 // Outcome probabilities (host, unnormalised, outcome order) for the caller's qubit list.
 static Status outcome_probs(qi_state *s, const int32_t *q, int m, std::vector<double> &prob, double *total_out) {
     const int n = s->n;
@@ -203,8 +205,14 @@ static Status outcome_probs(qi_state *s, const int32_t *q, int m, std::vector<do
     }
     g.loop = loop;
     const uint64_t outcomes = 1ull << nd, chunks = 1ull << g.nchunk;
+    // The workspace stays with the state, so only sums of the size that the thread split makes (2^17) lie
+    // there; many measured qubits take memory for this call alone.
+    const size_t sum_bytes = (chunks > 1 ? outcomes * chunks + outcomes : outcomes) * sizeof(double);
+    const bool keep = sum_bytes <= kKeptSums;
     void *ws = nullptr;
-    Status st = state_workspace(s, (outcomes * chunks + outcomes) * sizeof(double), &ws);
+    Status st = ok_status();
+    if (keep) st = state_workspace(s, sum_bytes, &ws);
+    else QI_CUDA(cudaMallocAsync(&ws, sum_bytes, s->stream));
     if (!st.ok()) return st;
     double *d_part = static_cast<double *>(ws), *d_P = d_part + outcomes * chunks;
     const unsigned tpb = 1u << std::min(8, (int)g.nthread), nb = 1u << (g.nthread - std::min(8, (int)g.nthread));
@@ -220,10 +228,13 @@ static Status outcome_probs(qi_state *s, const int32_t *q, int m, std::vector<do
         d_P = d_part;
     }
     st = check_launch("k_meas_sum");
+    std::vector<double> P(st.ok() ? outcomes : 0);
+    cudaError_t e = cudaSuccess;
+    if (st.ok()) e = cudaMemcpyAsync(P.data(), d_P, outcomes * sizeof(double), cudaMemcpyDeviceToHost, s->stream);
+    if (!keep) cudaFreeAsync(ws, s->stream);
     if (!st.ok()) return st;
-    std::vector<double> P(outcomes);
-    QI_CUDA(cudaMemcpyAsync(P.data(), d_P, outcomes * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
-    QI_CUDA(cudaStreamSynchronize(s->stream));
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+    if (e != cudaSuccess) return cuda_status(e, "measure");
     // map to the caller's outcome integers (bit k = qubit q[k]); duplicated qubits must agree
     const uint64_t no = 1ull << m;
     bool sorted = nd == m;
