@@ -890,7 +890,7 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
     }
     const bool swept = tiles && n_theta > 0;
     if (st.ok() && !swept && nslots > 0) {
-        e = cudaMalloc(&d_gres, (size_t)nslots * sizeof(double));
+        e = device_malloc(&d_gres, (size_t)nslots * sizeof(double));
         if (e != cudaSuccess) st = cuda_status(e, "cudaMalloc(gradient slots)");
     }
     if (st.ok() && f32 && !swept) st = state_reduce_norm_sqr(s, &npsi0);

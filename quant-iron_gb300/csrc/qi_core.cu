@@ -575,6 +575,14 @@ cudaError_t device_malloc(void **p, size_t bytes) {
     return cudaMalloc(p, bytes);
 }
 
+cudaError_t device_malloc_async(void **p, size_t bytes, cudaStream_t stream) {
+    cudaError_t e = cudaMallocAsync(p, bytes, stream);
+    if (e != cudaErrorMemoryAllocation) return e;
+    (void)cudaGetLastError();
+    cache_clear();
+    return cudaMallocAsync(p, bytes, stream);
+}
+
 // The caller may use the handle's buffer on a stream of its own from here on.
 static Status hand_out(qi_state *s) {
     s->exposed = true;

@@ -320,8 +320,8 @@ extern "C" qi_status qi_costmodel_collect(int32_t num_qubits, int64_t count, uin
     void *d_mat = nullptr, *d_tc = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     Status st = ok_status();
-    cudaError_t ce = cudaMalloc(&d_mat, 64 * 64 * sizeof(double2));
-    if (ce == cudaSuccess) ce = cudaMalloc(&d_tc, 6 * 64 * 64 * sizeof(float));
+    cudaError_t ce = device_malloc(&d_mat, 64 * 64 * sizeof(double2));
+    if (ce == cudaSuccess) ce = device_malloc(&d_tc, 6 * 64 * 64 * sizeof(float));
     if (ce == cudaSuccess) ce = cudaEventCreate(&e0);
     if (ce == cudaSuccess) ce = cudaEventCreate(&e1);
     if (ce != cudaSuccess) st = cuda_status(ce, "costmodel collect");

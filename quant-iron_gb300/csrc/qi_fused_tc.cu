@@ -853,7 +853,7 @@ extern "C" qi_status qi_tf32_rate_probe(int32_t iters, int32_t reps, double *tfl
     const int dyn = 120 * 1024;
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_tf32_rate_probe, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
     int *d_flag = nullptr;
-    if (e == cudaSuccess) e = cudaMalloc(&d_flag, sizeof(int));
+    if (e == cudaSuccess) e = device_malloc(&d_flag, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(d_flag, 0, sizeof(int));
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     if (e == cudaSuccess) e = cudaEventCreate(&ev0);

@@ -95,8 +95,13 @@ Status state_copy_async(qi_state *dst, const qi_state *src);
 // being captured, the host waits for src's stream instead.
 Status read_begin(qi_state *dst, const qi_state *src);
 Status read_end(qi_state *dst, const qi_state *src);
-// cudaMalloc; on failure the cached handles are freed and it is tried once more.
+// cudaMalloc, or cudaMallocAsync; on failure the cached handles are freed and it is tried once more.
 cudaError_t device_malloc(void **p, size_t bytes);
+cudaError_t device_malloc_async(void **p, size_t bytes, cudaStream_t stream);
+template <typename T> cudaError_t device_malloc(T **p, size_t bytes) { return device_malloc((void **)p, bytes); }
+template <typename T> cudaError_t device_malloc_async(T **p, size_t bytes, cudaStream_t stream) {
+    return device_malloc_async((void **)p, bytes, stream);
+}
 
 // ----------------------------------------------------------------- gates --
 // A gate lowered to one primitive device operation.

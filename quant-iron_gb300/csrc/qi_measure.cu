@@ -212,7 +212,7 @@ static Status outcome_probs(qi_state *s, const int32_t *q, int m, std::vector<do
     void *ws = nullptr;
     Status st = ok_status();
     if (keep) st = state_workspace(s, sum_bytes, &ws);
-    else QI_CUDA(cudaMallocAsync(&ws, sum_bytes, s->stream));
+    else QI_CUDA(device_malloc_async(&ws, sum_bytes, s->stream));
     if (!st.ok()) return st;
     double *d_part = static_cast<double *>(ws), *d_P = d_part + outcomes * chunks;
     const unsigned tpb = 1u << std::min(8, (int)g.nthread), nb = 1u << (g.nthread - std::min(8, (int)g.nthread));

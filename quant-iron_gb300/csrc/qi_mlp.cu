@@ -106,12 +106,12 @@ Mlp &global_mlp() {
 
 Status Mlp::ensure_device(int N) {
     if (!d_params) {
-        QI_CUDA(cudaMalloc(&d_params, kParams * sizeof(float)));
-        QI_CUDA(cudaMalloc(&d_grads, kParams * sizeof(float)));
-        QI_CUDA(cudaMalloc(&d_m, kParams * sizeof(float)));
-        QI_CUDA(cudaMalloc(&d_v, kParams * sizeof(float)));
-        QI_CUDA(cudaMalloc(&d_loss, sizeof(float)));
-        QI_CUDA(cudaMalloc(&d_partials, 1024 * sizeof(double)));
+        QI_CUDA(device_malloc(&d_params, kParams * sizeof(float)));
+        QI_CUDA(device_malloc(&d_grads, kParams * sizeof(float)));
+        QI_CUDA(device_malloc(&d_m, kParams * sizeof(float)));
+        QI_CUDA(device_malloc(&d_v, kParams * sizeof(float)));
+        QI_CUDA(device_malloc(&d_loss, sizeof(float)));
+        QI_CUDA(device_malloc(&d_partials, 1024 * sizeof(double)));
     }
     if (N > cap) {
         for (float *&p : act) if (p) { cudaFree(p); p = nullptr; }
@@ -119,7 +119,7 @@ Status Mlp::ensure_device(int N) {
         const size_t sizes[kActBufs] = {(size_t)N * kFeat, (size_t)N, (size_t)N, (size_t)N,
                                         (size_t)N * kH, (size_t)N * kH, (size_t)N * kH, (size_t)N * kH,
                                         (size_t)N * kH, (size_t)N * kH, (size_t)N * kH, (size_t)N * kH};
-        for (int i = 0; i < kActBufs; ++i) QI_CUDA(cudaMalloc(&act[i], sizes[i] * sizeof(float)));
+        for (int i = 0; i < kActBufs; ++i) QI_CUDA(device_malloc(&act[i], sizes[i] * sizeof(float)));
         cap = N;
     }
     return ok_status();

@@ -1181,7 +1181,7 @@ static Status launch_sumop_apply_tiles_f32(qi_state *o, qi_state *in, const std:
     const size_t off_grp = off_term + up16(std::max<size_t>(1, terms.size()) * sizeof(TileTerm<IDX>));
     const size_t bytes = off_grp + up16(groups.size() * sizeof(TileGroup));
     unsigned char *d = nullptr;
-    QI_CUDA(cudaMallocAsync((void **)&d, bytes, o->stream));
+    QI_CUDA(device_malloc_async(&d, bytes, o->stream));
     ApplyStep *d_steps = reinterpret_cast<ApplyStep *>(d);
     TileTerm<IDX> *d_term = reinterpret_cast<TileTerm<IDX> *>(d + off_term);
     TileGroup *d_grp = reinterpret_cast<TileGroup *>(d + off_grp);
@@ -1216,9 +1216,9 @@ static Status launch_sumop_apply_f32(qi_state *o, qi_state *in, const std::vecto
     ApplyHdr<IDX> *d_hdr = nullptr;
     ApplyTerm<IDX> *d_term = nullptr;
     float2 *d_tab = nullptr;
-    QI_CUDA(cudaMallocAsync((void **)&d_hdr, std::max<size_t>(1, ap.hdrs.size()) * sizeof(ApplyHdr<IDX>), o->stream));
-    QI_CUDA(cudaMallocAsync((void **)&d_term, std::max<size_t>(1, ap.terms.size()) * sizeof(ApplyTerm<IDX>), o->stream));
-    QI_CUDA(cudaMallocAsync((void **)&d_tab, std::max<size_t>(1, ap.tables.size()) * sizeof(float2), o->stream));
+    QI_CUDA(device_malloc_async(&d_hdr, std::max<size_t>(1, ap.hdrs.size()) * sizeof(ApplyHdr<IDX>), o->stream));
+    QI_CUDA(device_malloc_async(&d_term, std::max<size_t>(1, ap.terms.size()) * sizeof(ApplyTerm<IDX>), o->stream));
+    QI_CUDA(device_malloc_async(&d_tab, std::max<size_t>(1, ap.tables.size()) * sizeof(float2), o->stream));
     QI_CUDA(cudaMemcpyAsync(d_hdr, ap.hdrs.data(), ap.hdrs.size() * sizeof(ApplyHdr<IDX>), cudaMemcpyHostToDevice, o->stream));
     QI_CUDA(cudaMemcpyAsync(d_term, ap.terms.data(), ap.terms.size() * sizeof(ApplyTerm<IDX>), cudaMemcpyHostToDevice,
                             o->stream));
@@ -1266,8 +1266,8 @@ static void group_terms(const qi_pauli_term *terms, int64_t nt, std::vector<Grou
 
 static Status upload_groups(qi_state *s, const std::vector<GroupHdr> &hdrs, const std::vector<GroupTerm> &terms,
                             GroupHdr **d_hdr, GroupTerm **d_terms) {
-    QI_CUDA(cudaMallocAsync((void **)d_hdr, std::max<size_t>(1, hdrs.size()) * sizeof(GroupHdr), s->stream));
-    QI_CUDA(cudaMallocAsync((void **)d_terms, std::max<size_t>(1, terms.size()) * sizeof(GroupTerm), s->stream));
+    QI_CUDA(device_malloc_async(d_hdr, std::max<size_t>(1, hdrs.size()) * sizeof(GroupHdr), s->stream));
+    QI_CUDA(device_malloc_async(d_terms, std::max<size_t>(1, terms.size()) * sizeof(GroupTerm), s->stream));
     QI_CUDA(cudaMemcpyAsync(*d_hdr, hdrs.data(), hdrs.size() * sizeof(GroupHdr), cudaMemcpyHostToDevice, s->stream));
     QI_CUDA(cudaMemcpyAsync(*d_terms, terms.data(), terms.size() * sizeof(GroupTerm), cudaMemcpyHostToDevice, s->stream));
     // host vectors are pageable: the copies complete before cudaMemcpyAsync returns
@@ -1363,8 +1363,8 @@ Status sumop_expectation(qi_state *s, const qi_pauli_term *terms, int64_t nt, do
                     G[it] = make_float2((float)re, (float)im);
                 }
                 void *dG = nullptr, *dT = nullptr;
-                QI_CUDA(cudaMallocAsync(&dG, G.size() * sizeof(float2), s->stream));
-                QI_CUDA(cudaMallocAsync(&dT, std::max<size_t>(1, lm.size()) * sizeof(GroupTerm), s->stream));
+                QI_CUDA(device_malloc_async(&dG, G.size() * sizeof(float2), s->stream));
+                QI_CUDA(device_malloc_async(&dT, std::max<size_t>(1, lm.size()) * sizeof(GroupTerm), s->stream));
                 scratch.push_back(dG);
                 scratch.push_back(dT);
                 QI_CUDA(cudaMemcpyAsync(dG, G.data(), G.size() * sizeof(float2), cudaMemcpyHostToDevice, s->stream));
@@ -1392,7 +1392,7 @@ Status sumop_expectation(qi_state *s, const qi_pauli_term *terms, int64_t nt, do
                     else nz.push_back(gt[k]);
                 }
                 void *dT = nullptr;
-                QI_CUDA(cudaMallocAsync(&dT, std::max<size_t>(1, nz.size()) * sizeof(GroupTerm), s->stream));
+                QI_CUDA(device_malloc_async(&dT, std::max<size_t>(1, nz.size()) * sizeof(GroupTerm), s->stream));
                 scratch.push_back(dT);
                 if (!nz.empty())
                     QI_CUDA(cudaMemcpyAsync(dT, nz.data(), nz.size() * sizeof(GroupTerm), cudaMemcpyHostToDevice, s->stream));

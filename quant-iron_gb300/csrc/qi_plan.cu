@@ -757,7 +757,7 @@ Status upload_plan(qi_plan *p) {
     if (p->d_mats) { cudaFree(p->d_mats); p->d_mats = nullptr; }
     if (p->d_tc) { cudaFree(p->d_tc); p->d_tc = nullptr; }
     if (!p->tc.empty()) {
-        QI_CUDA(cudaMalloc(&p->d_tc, (p->tc.size() + p->compose.words) * sizeof(float)));
+        QI_CUDA(device_malloc(&p->d_tc, (p->tc.size() + p->compose.words) * sizeof(float)));
         p->composed = false;
         QI_CUDA(copy_in(p->d_tc, p->tc.data(), p->tc.size() * sizeof(float)));
     }
@@ -766,12 +766,12 @@ Status upload_plan(qi_plan *p) {
     if (p->prec == QI_F32) {
         std::vector<float2> h(cnt);
         for (size_t i = 0; i < cnt; ++i) h[i] = make_float2((float)p->mats[i].real(), (float)p->mats[i].imag());
-        QI_CUDA(cudaMalloc(&p->d_mats, cnt * sizeof(float2)));
+        QI_CUDA(device_malloc(&p->d_mats, cnt * sizeof(float2)));
         QI_CUDA(copy_in(p->d_mats, h.data(), cnt * sizeof(float2)));
     } else {
         std::vector<double2> h(cnt);
         for (size_t i = 0; i < cnt; ++i) h[i] = make_double2(p->mats[i].real(), p->mats[i].imag());
-        QI_CUDA(cudaMalloc(&p->d_mats, cnt * sizeof(double2)));
+        QI_CUDA(device_malloc(&p->d_mats, cnt * sizeof(double2)));
         QI_CUDA(copy_in(p->d_mats, h.data(), cnt * sizeof(double2)));
     }
     return ok_status();
@@ -814,7 +814,7 @@ static bool runs_ready(qi_plan *p, qi_state *s) {
         return false;
     }
     void *d = nullptr;
-    if (cudaMalloc(&d, p->run_prog.size()) != cudaSuccess) {
+    if (device_malloc(&d, p->run_prog.size()) != cudaSuccess) {
         (void)cudaGetLastError();
         return false;
     }
