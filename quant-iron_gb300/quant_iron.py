@@ -640,7 +640,7 @@ class Circuit:
             return np.zeros(0, dtype=GATE_DTYPE)
         rows = [g.row if isinstance(g, Gate) else g for g in self.gates]
         if all(isinstance(r, (np.void, np.ndarray)) and r.dtype == GATE_DTYPE and r.ndim == 0 for r in rows):
-            return np.frombuffer(b"".join([r.tobytes() for r in rows]), dtype=GATE_DTYPE)
+            return np.frombuffer(bytearray().join([r.tobytes() for r in rows]), dtype=GATE_DTYPE)
         return np.stack(rows).astype(GATE_DTYPE)
 
     def execute(self, initial_state):   # circuit.rs:160-172
