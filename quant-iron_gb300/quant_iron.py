@@ -361,10 +361,10 @@ assert _ROW.size == GATE_DTYPE.itemsize
 
 def _packed_row(kind, targets, controls, params):
     """The bytes of a gate row (the C struct), or None where GateList has to build (or refuse) it."""
-    nt, nc, npar = len(targets), len(controls), len(params)
-    if nt > 2 or nc > MAX_CONTROLS or npar > 8:
-        return None
     try:
+        nt, nc, npar = len(targets), len(controls), len(params)
+        if nt > 2 or nc > MAX_CONTROLS or npar > 8:
+            return None
         return _ROW.pack(GATE_KINDS[kind], nt, nc, -1, -1, -1, *targets, *_NO_INTS[:2 - nt], *controls,
                          *_NO_INTS[:MAX_CONTROLS - nc], *params, *_NO_FLOATS[:8 - npar], 0, 0)
     except (struct.error, TypeError, KeyError):
@@ -392,7 +392,9 @@ class Operator:
         return gl.array()[0]
 
     def apply(self, state, target_qubits, control_qubits=()):
-        row = _packed_row(self.KIND, target_qubits, control_qubits, self.params())
+        row = None
+        if type(self).gate_row is Operator.gate_row:   # a subclass's own row is asked for
+            row = _packed_row(self.KIND, target_qubits, control_qubits, self.params())
         if row is None:
             row = self.gate_row(target_qubits, control_qubits).tobytes()
         src = state._resident()
