@@ -232,8 +232,9 @@ static Status outcome_probs(qi_state *s, const int32_t *q, int m, std::vector<do
     cudaError_t e = cudaSuccess;
     if (st.ok()) e = cudaMemcpyAsync(P.data(), d_P, outcomes * sizeof(double), cudaMemcpyDeviceToHost, s->stream);
     if (!keep) cudaFreeAsync(ws, s->stream);
+    const cudaError_t done = cudaStreamSynchronize(s->stream);   // after a failure too: the workspace is in use until then
     if (!st.ok()) return st;
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+    if (e == cudaSuccess) e = done;
     if (e != cudaSuccess) return cuda_status(e, "measure");
     // map to the caller's outcome integers (bit k = qubit q[k]); duplicated qubits must agree
     const uint64_t no = 1ull << m;

@@ -1605,7 +1605,10 @@ qi_status qi_sumop_apply(qi_state *out, qi_state *in, const qi_pauli_term *terms
         return publish(state_scale_async(out, 0.0, 0.0));
     }
     Status st = sumop_apply(out, in, terms, n_terms);
-    if (!st.ok()) return publish(st);
+    if (!st.ok()) {
+        cudaStreamSynchronize(out->stream);   // earlier passes may be running on its workspace
+        return publish(st);
+    }
     int flag = 0;
     st = state_read_flag(out, &flag);
     if (st.ok() && flag == 2) st = err(QI_ERR_TIMEOUT, -1, -1, "SumOp::apply: a device wait timed out");
@@ -1621,7 +1624,9 @@ qi_status qi_sumop_expectation(qi_state *s, const qi_pauli_term *terms, int64_t 
         Status st = validate_pauli(s->n, terms[k]);
         if (!st.ok()) return publish(st);
     }
-    return publish(sumop_expectation(s, terms, n_terms, out));
+    Status st = sumop_expectation(s, terms, n_terms, out);
+    if (!st.ok()) cudaStreamSynchronize(s->stream);   // earlier passes may be running on its workspace
+    return publish(st);
 }
 
 }  // extern "C"

@@ -1286,8 +1286,8 @@ qi_status qi_circuit_execute(qi_state *s, const qi_gate *gates, int64_t n_gates,
     std::lock_guard<std::recursive_mutex> lk(s->mu);   // held until the plan's program is no longer in use
     if (cudaSetDevice(s->device) == cudaSuccess) borrow_runs({p}, s);
     st = qi_plan_execute(p, s);
+    const cudaError_t e = cudaStreamSynchronize(s->stream);   // after a failure too: earlier passes may be running
     if (st == QI_OK) {
-        cudaError_t e = cudaStreamSynchronize(s->stream);
         if (e != cudaSuccess) {
             st = publish(cuda_status(e, "execute"));
         } else {
