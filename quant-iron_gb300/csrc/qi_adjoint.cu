@@ -735,7 +735,10 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
     // alone took the gradient from 7e-7 to 1.3e-6 of the FP64 result.
     qi_exec_options plan_opts = {QI_FUSION_GREEDY, 0, 0, 0};
     if (forward_opts) plan_opts = *forward_opts;
-    const int chosen_block = plan_opts.max_block_qubits;
+    // the forward pass is the engine's to choose unless the caller named a partition, a block size or (FP32)
+    // the units that blocks run on
+    const bool chosen = plan_opts.fusion != QI_FUSION_GREEDY || plan_opts.max_block_qubits > 0 ||
+                        (s->prec == QI_F32 && (plan_opts.use_tensor_cores != 0 || plan_opts.renorm_every != 0));
     if (s->prec == QI_F32 && plan_opts.max_block_qubits <= 0) plan_opts.max_block_qubits = 5;
     // psi_0 stays untouched in the caller's buffer: the sweep runs on a copy (un-applying psi in
     // FP32 would hand back psi_0 with the sweep's rounding in it); without room for the copy it
@@ -780,13 +783,16 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
         plan.prec = s->prec;
         plan.device_blocks = true;
         plan.opts = plan_opts;
-        // FP64 (dense FP64 blocks are bound by the FP64 pipe) and FP32 up to 22 qubits unless the caller
-        // chose a block size: the gate runs' own arithmetic, with no block matrices to compose (FP32
-        // gradients, fused / gate runs: 8 qubits 1.57 / 0.37 ms, 20 qubits 4.25 / 2.58, 22 qubits 7.8 /
-        // 6.2, 24 qubits 18.0 / 20.1; relative error at 20 qubits 6.1e-7 / 4.7e-7)
-        if (s->prec == QI_F64 || (chosen_block <= 0 && n <= kSweepMaxF32)) plan.opts.fusion = QI_FUSION_NONE;
         std::vector<Elem> elems;
         Status st = plan_elems_from_gates(n, gates, n_gates, theta, n_theta, elems);
+        // FP64 (dense FP64 blocks are bound by the FP64 pipe) and FP32 up to 22 qubits: the gate runs' own
+        // arithmetic, with no block matrices to compose (FP32 gradients, fused / gate runs: 8 qubits 1.57 /
+        // 0.37 ms, 20 qubits 4.25 / 2.58, 22 qubits 7.8 / 6.2, 24 qubits 18.0 / 20.1; relative error at 20
+        // qubits 6.1e-7 / 4.7e-7).  FP32 only where every gate joins a run: each that cannot (a matchgate) is a
+        // pass of its own where a block takes several.
+        bool runs = !chosen && (s->prec == QI_F64 || n <= kSweepMaxF32);
+        for (size_t i = 0; runs && s->prec == QI_F32 && i < elems.size(); ++i) runs = run_supported(n, s->prec, elems[i]);
+        if (runs) plan.opts.fusion = QI_FUSION_NONE;
         if (st.ok()) st = build_plan(&plan, elems);
         if (st.ok()) st = upload_plan(&plan);
         if (st.ok()) st = plan_execute(&plan, s);
