@@ -14,8 +14,11 @@
 // A parametric gate is U = exp(-i theta P / 2) (or a phase), so its term is Im <lambda| P |psi> / 2, two
 // operations per amplitude instead of a general 2x2 derivative, and both states take the same scaled
 // inverse with unit entries; the size of the scales left out multiplies the term on the host.
-// A term is reduced over the warp, per tile over the block's warps, and over tiles in FP64 by one
-// thread per term.
+// A thread's part of a term is summed in the state's precision, everything above it in FP64 or as finely: over
+// the warp in FP64, or (FP32) as integers of 2^-26 of the largest part or less, then over the block's warps and
+// the tiles in FP64 by one thread per term.  (Terms whose products have one sign, 12 qubits: 0.44 * 2^-24 off with
+// FP32 sums over the block, 0.05 as integers; FP32 gradients of 8 to 22 qubits take 1-3 % less time, as two integer
+// reductions take the place of five shuffles.)
 #include "qi_gaterun.hpp"
 #include "qi_runops.cuh"
 
@@ -91,6 +94,17 @@ __device__ __forceinline__ T der_diag_m(int m, const typename Cx<T>::V2 (&v)[1 <
     }
 }
 
+// Sum over the warp's lanes as a multiple of a power of two that holds the largest |p| in 26 bits (32 of them
+// in 31): every p is rounded to at most 2^-26 of that.  e: its biased exponent, 255 when some p is not finite.
+__device__ __forceinline__ int warp_sum_fixed(unsigned lanes, float p, uint8_t &e) {
+    const uint32_t big = __reduce_max_sync(lanes, __float_as_uint(p) & 0x7fffffffu) >> 23;
+    e = (uint8_t)max(big, 25u);   // the scale stays a normal number
+    return __reduce_add_sync(lanes, __float2int_rn(p * __uint_as_float((279u - e) << 23)));
+}
+__device__ __forceinline__ double fixed_value(int sum, uint8_t e) {
+    return (double)sum * __hiloint2double(e == 255 ? 0x7ff80000 : ((int)e + 871) << 20, 0);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3 : 2) k_sweep_run(typename Cx<T>::V2 *psi, typename Cx<T>::V2 *lam, uint64_t ntiles,
                                                    const uint4 *prog, const __grid_constant__ SweepGeom g, double *partials) {
@@ -98,7 +112,9 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
     constexpr int S = kRunSelBits, NV = 1 << RunShape<T>::kRegBits, UB0 = RunShape<T>::kUnitBits;
     extern __shared__ uint4 sm[];
     __shared__ V2 slot[kRunMaxSlots];
-    __shared__ T part[kSweepTerms * (sizeof(T) == 8 ? 4 : 8)];
+    constexpr int kParts = kSweepTerms * (sizeof(T) == 8 ? 4 : 8);
+    __shared__ T part[kParts];                                  // of each term and warp; FP32: integer bits
+    __shared__ uint8_t part_exp[sizeof(T) == 8 ? 1 : kParts];
     __shared__ double total[kSweepTerms];
     __shared__ uint64_t next_base;
     const int ubits = g.tbits - UB0, lowu = g.low - UB0;
@@ -198,8 +214,18 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
                     if (nsub == kDerX) p = der_pair_x<T, false>(xi, v, l);
                     else if (nsub == kDerY) p = der_pair_x<T, true>(xi, v, l);
                     else p = der_diag_m<T>(xi, v, l, odd, nsub == kDerZ);
-                    for (uint32_t w = min(nt, 32u) >> 1; w; w >>= 1) p += __shfl_xor_sync(lanes, p, w);
-                    if (lane == 0) part[(uint32_t)h.cg * nwarp + warp] = p;
+                    const uint32_t at_part = (uint32_t)h.cg * nwarp + warp;
+                    if constexpr (sizeof(T) == 4) {
+                        uint8_t e;
+                        const int sum = warp_sum_fixed(lanes, p, e);
+                        if (lane == 0) {
+                            part[at_part] = __int_as_float(sum);
+                            part_exp[at_part] = e;
+                        }
+                    } else {
+                        for (uint32_t w = min(nt, 32u) >> 1; w; w >>= 1) p += __shfl_xor_sync(lanes, p, w);
+                        if (lane == 0) part[at_part] = p;
+                    }
                 } else if (!rotation) {
                     const uint64_t cg = h.cg;
                     if ((lbase & h.cl) != h.cl || (tbase & cg) != cg) continue;
@@ -255,9 +281,12 @@ __global__ void __launch_bounds__(sizeof(T) == 8 ? 128 : 256, sizeof(T) == 8 ? 3
             __syncthreads();
         }
         for (uint32_t i = tid; i < (uint32_t)g.nterm; i += nt) {
-            T s = T(0);
-            for (uint32_t w = 0; w < nwarp; ++w) s += part[i * nwarp + w];
-            total[i] += (double)s;
+            double s = 0.0;
+            for (uint32_t w = 0; w < nwarp; ++w) {
+                if constexpr (sizeof(T) == 4) s += fixed_value(__float_as_int(part[i * nwarp + w]), part_exp[i * nwarp + w]);
+                else s += part[i * nwarp + w];
+            }
+            total[i] += s;
         }
         for (uint32_t u = 0; u < nunit; u += nt) {
             const uint32_t at = mine.at ^ (run_swizzle(u) << 4);
