@@ -743,37 +743,21 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
     // psi_0 stays untouched in the caller's buffer: the sweep runs on a copy (un-applying psi in
     // FP32 would hand back psi_0 with the sweep's rounding in it); without room for the copy it
     // runs in place and psi_0 is restored by the sweep itself.
-    // A scratch handle's buffers are used on s's stream, behind what its own stream still holds.
-    auto join = [&](qi_state *q) {
-        cudaError_t je = cudaEventRecord(q->ev, q->own_stream);
-        if (je == cudaSuccess) je = cudaStreamWaitEvent(s->stream, q->ev, 0);
-        q->stream = s->stream;
-        return je;
-    };
-    auto give_back = [&](qi_state *q) {   // s's stream has been waited for
-        q->stream = q->own_stream;
-        qi_state_destroy(q);
-    };
     void *const psi_home = s->amps;
     qi_state *work = nullptr;
-    if (qi_state_create(n, s->prec, &work) == QI_OK) {
-        e = join(work);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(work->amps, psi_home, s->bytes(), cudaMemcpyDeviceToDevice, s->stream);
+    if (scratch_take(s, s->prec, &work).ok()) {
+        e = cudaMemcpyAsync(work->amps, psi_home, s->bytes(), cudaMemcpyDeviceToDevice, s->stream);
         if (e != cudaSuccess) {
-            cudaStreamSynchronize(s->stream);
-            give_back(work);
+            scratch_give(work);
             return publish(cuda_status(e, "copy psi_0"));
         }
         s->amps = work->amps;
-    } else {
-        work = nullptr;
-        cudaGetLastError();
     }
     auto bail = [&](Status st) {   // before lambda exists: psi is in `work` (or in place)
         cudaStreamSynchronize(s->stream);
         if (work) {
             s->amps = psi_home;
-            give_back(work);
+            scratch_give(work);
         }
         return publish(st);
     };
@@ -804,10 +788,8 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
     // lambda = H psi, and E = <psi|lambda> (one read pass of two states with FP64 sums, in place of
     // one pass per X-mask group of H)
     qi_state *lam = nullptr;
-    qi_status cs = qi_state_create(n, s->prec, &lam);
-    if (cs != QI_OK) return bail(err(cs, -1, -1, "lambda state"));
-    Status st = ok_status();
-    if ((e = join(lam)) != cudaSuccess) st = cuda_status(e, "lambda state");
+    Status st = scratch_take(s, s->prec, &lam);
+    if (!st.ok()) return bail(err(st.code, -1, -1, "lambda state"));
     double ev[2] = {0, 0};
     if (n_terms > 0) {
         if (st.ok()) st = sumop_apply(lam, s, terms, n_terms);
@@ -1145,7 +1127,7 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
     if (work) {   // psi_0 never left the caller's buffer; psi ends in one of the sweep's buffers
         work->amps = s->amps;
         s->amps = psi_home;
-        give_back(work);
+        scratch_give(work);
     } else if (s->amps != psi_home) {   // psi_home is lambda's or the scratch buffer now
         e = cudaMemcpyAsync(psi_home, s->amps, s->bytes(), cudaMemcpyDeviceToDevice, s->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
@@ -1161,6 +1143,6 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
         release_runs(sp.get());
     }
     if (d_gres) cudaFree(d_gres);
-    give_back(lam);
+    scratch_give(lam);
     return publish(st);
 }

@@ -591,6 +591,71 @@ static Status hand_out(qi_state *s) {
     return ok_status();
 }
 
+Status state_make(int n, int prec, int device, qi_state **out) {
+    cudaError_t e = cudaSetDevice(device);
+    if (e != cudaSuccess) return cuda_status(e, "cudaSetDevice");
+    if (qi_state *s = cache_take(n, prec, device)) {
+        s->host_io = false;
+        s->recycled = true;
+        if ((e = cudaMemsetAsync(s->d_flag, 0, sizeof(int), s->stream)) != cudaSuccess) {
+            free_handle(s);
+            return cuda_status(e, "memset");
+        }
+        *out = s;
+        return ok_status();
+    }
+    qi_state *s = new qi_state();
+    s->n = n;
+    s->prec = prec;
+    s->device = device;
+    auto fail = [&](Status st) {
+        free_handle(s);
+        return st;
+    };
+    if ((e = cudaStreamCreateWithFlags(&s->own_stream, cudaStreamNonBlocking)) != cudaSuccess)
+        return fail(cuda_status(e, "cudaStreamCreate"));
+    s->stream = s->own_stream;
+    if ((e = cudaEventCreateWithFlags(&s->ev, cudaEventDisableTiming)) != cudaSuccess)
+        return fail(cuda_status(e, "cudaEventCreate"));
+    if ((e = device_malloc(&s->amps, s->bytes())) != cudaSuccess) return fail(cuda_status(e, "cudaMalloc(state)"));
+    // one block: partials, results, error flag
+    constexpr size_t parts = kReduceBlocks * 4 * sizeof(double);
+    void *small = nullptr;
+    if ((e = device_malloc(&small, parts + 128)) != cudaSuccess) return fail(cuda_status(e, "cudaMalloc(partials)"));
+    s->d_partials = (double *)small;
+    s->d_result = (double *)((char *)small + parts);
+    s->d_flag = (int *)((char *)small + parts + 64);
+    if ((e = cudaMallocHost(&s->h_result, 8 * sizeof(double))) != cudaSuccess) return fail(cuda_status(e, "cudaMallocHost"));
+    if ((e = cudaMemsetAsync(s->d_flag, 0, sizeof(int), s->stream)) != cudaSuccess) return fail(cuda_status(e, "memset"));
+    *out = s;
+    return ok_status();
+}
+
+Status scratch_take(qi_state *s, int prec, qi_state **out) {
+    Status st = state_make(s->n, prec, s->device, out);
+    if (!st.ok()) {
+        (void)cudaGetLastError();
+        *out = nullptr;
+        return st;
+    }
+    qi_state *q = *out;
+    cudaError_t e = cudaEventRecord(q->ev, q->own_stream);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s->stream, q->ev, 0);
+    q->stream = s->stream;
+    if (e == cudaSuccess) return ok_status();
+    scratch_give(q);
+    *out = nullptr;
+    return cuda_status(e, "scratch state");
+}
+
+void scratch_give(qi_state *q) {
+    const int device = q->device;
+    cudaStreamSynchronize(q->stream);
+    q->stream = q->own_stream;
+    qi_state_destroy(q);
+    cudaSetDevice(device);   // the cache may have freed a handle of another one
+}
+
 Status state_workspace(qi_state *s, size_t bytes, void **out, bool program) {
     void *&have = program ? s->d_prog : s->d_work;
     size_t &have_bytes = program ? s->prog_bytes : s->work_bytes;
@@ -714,43 +779,7 @@ qi_status qi_state_create(int32_t num_qubits, int32_t precision, qi_state **out)
     if (num_qubits <= 0) return publish(err(QI_ERR_INVALID_NUMBER_OF_QUBITS, num_qubits < 0 ? 0 : num_qubits));
     if (num_qubits > 40) return publish(err(QI_ERR_INVALID_NUMBER_OF_QUBITS, num_qubits));
     if (precision != QI_F32 && precision != QI_F64) return publish(err(QI_ERR_INVALID_INPUT_VALUE, precision));
-    cudaError_t e = cudaSetDevice(g_device);
-    if (e != cudaSuccess) return publish(cuda_status(e, "cudaSetDevice"));
-    if (qi_state *s = cache_take(num_qubits, precision, g_device)) {
-        s->host_io = false;
-        s->recycled = true;
-        if ((e = cudaMemsetAsync(s->d_flag, 0, sizeof(int), s->stream)) != cudaSuccess) {
-            free_handle(s);
-            return publish(cuda_status(e, "memset"));
-        }
-        *out = s;
-        return publish(ok_status());
-    }
-    qi_state *s = new qi_state();
-    s->n = num_qubits;
-    s->prec = precision;
-    s->device = g_device;
-    auto fail = [&](Status st) {
-        free_handle(s);
-        return publish(st);
-    };
-    if ((e = cudaStreamCreateWithFlags(&s->own_stream, cudaStreamNonBlocking)) != cudaSuccess)
-        return fail(cuda_status(e, "cudaStreamCreate"));
-    s->stream = s->own_stream;
-    if ((e = cudaEventCreateWithFlags(&s->ev, cudaEventDisableTiming)) != cudaSuccess)
-        return fail(cuda_status(e, "cudaEventCreate"));
-    if ((e = device_malloc(&s->amps, s->bytes())) != cudaSuccess) return fail(cuda_status(e, "cudaMalloc(state)"));
-    // one block: partials, results, error flag
-    constexpr size_t parts = kReduceBlocks * 4 * sizeof(double);
-    void *small = nullptr;
-    if ((e = device_malloc(&small, parts + 128)) != cudaSuccess) return fail(cuda_status(e, "cudaMalloc(partials)"));
-    s->d_partials = (double *)small;
-    s->d_result = (double *)((char *)small + parts);
-    s->d_flag = (int *)((char *)small + parts + 64);
-    if ((e = cudaMallocHost(&s->h_result, 8 * sizeof(double))) != cudaSuccess) return fail(cuda_status(e, "cudaMallocHost"));
-    if ((e = cudaMemsetAsync(s->d_flag, 0, sizeof(int), s->stream)) != cudaSuccess) return fail(cuda_status(e, "memset"));
-    *out = s;
-    return publish(ok_status());
+    return publish(state_make(num_qubits, precision, g_device, out));
 }
 
 qi_status qi_state_destroy(qi_state *s) {

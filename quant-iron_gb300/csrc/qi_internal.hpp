@@ -95,6 +95,12 @@ Status state_copy_async(qi_state *dst, const qi_state *src);
 // being captured, the host waits for src's stream instead.
 Status read_begin(qi_state *dst, const qi_state *src);
 Status read_end(qi_state *dst, const qi_state *src);
+// A new handle on `device` (which becomes the current one).
+Status state_make(int n, int prec, int device, qi_state **out);
+// A scratch state of s's size on s's device, used on s's stream: ordered behind what its own stream still
+// holds.  scratch_give waits for the stream.
+Status scratch_take(qi_state *s, int prec, qi_state **out);
+void scratch_give(qi_state *q);
 // cudaMalloc, or cudaMallocAsync; on failure the cached handles are freed and it is tried once more.
 cudaError_t device_malloc(void **p, size_t bytes);
 cudaError_t device_malloc_async(void **p, size_t bytes, cudaStream_t stream);
