@@ -315,8 +315,10 @@ typedef struct qi_exec_options {
     int32_t fusion;            /* QI_FUSION_* */
     int32_t max_block_qubits;  /* k <= 6; 0 = default (6) */
     int32_t use_tensor_cores;  /* 0 (default) or 1: 3xTF32 tcgen05 kernel for FP32 blocks of k >= 5; 2: CUDA cores only.
-                                  0 with max_block_qubits 0: greedy FP32 plans of 10 to 12 qubits execute as passes
-                                  over their gates instead of blocks (qi_plan_run_info), which is faster there */
+                                  0 with max_block_qubits 0: greedy FP32 plans of 10 to 12 qubits (without Pauli
+                                  exponentials) execute as passes over their gates instead of blocks
+                                  (qi_plan_run_info), which is faster there and, on circuits of generic angles,
+                                  more exact; any other value keeps the blocks */
     int32_t renorm_every;      /* FP64 renormalisation on the device: 0 = once at the end when tensor-core
                                   blocks ran (their FP32 accumulation rounds toward zero, so the norm drifts
                                   down by ~1e-6 per block); N > 0 = also after every N tensor-core blocks;

@@ -439,7 +439,12 @@ static void build_schedule(qi_plan *p, const std::vector<Elem> &elems, const std
 // caller chose neither block size nor tensor cores.  Below 13 qubits blocks of six do not fit the
 // tensor-core kernel's tiles; 40 layers + QFT, fused blocks / gate runs, among others and alone (us): 10 qubits
 // 103 / 71, 264 / 220; 12 qubits 193 / 97, 560 / 300; 13 qubits 76 / 107, 210 / 322; 15 qubits 100 / 128, 266 /
-// 376; 17 qubits 115 / 164, 307 / 433 (8 and 9 qubits, where a block covers most of the state, about even).  The
+// 376; 17 qubits 115 / 164, 307 / 433 (8 and 9 qubits, where a block covers most of the state, about even).
+// Error, relative to blocks: a run rounds every gate, a block of six qubits on the CUDA cores (below 13) every
+// sum of 64 products, a tensor-core block truncates.  1 to 30 layers of the benchmark family, of an RY / RZ / CNOT
+// ansatz and of a QAOA ansatz: 4 qubits 0.7-4.0, 6 qubits 0.5-2.5 (one block holds the state), 7 to 12 qubits
+// 0.47-0.87, 13 to 18 qubits 0.18-0.31.  Pauli exponentials of a time step are near the identity and cost a block
+// less: 1.4-1.9 on 7 to 12 qubits (0.2-0.34 from 13 on), so circuits with some keep blocks there.  The
 // ops (with the fused blocks' matrices, most of a plan's build time) are made when something asks for them.
 
 static bool build_runs(qi_plan *p, const std::vector<Elem> &elems, int fusion, int kmax) {
@@ -452,7 +457,7 @@ static bool build_runs(qi_plan *p, const std::vector<Elem> &elems, int fusion, i
     if (!per_gate && !small_fused) return false;
     int64_t count = 0;
     for (const Elem &e : elems) {
-        if (!run_supported(p->n, p->prec, e)) return false;
+        if (!run_supported(p->n, p->prec, e) || (small_fused && p->n < 13 && e.pauli)) return false;
         count += e.gm.pauli || e.gm.nt > 0;
     }
     if (count < 2) return false;
@@ -1001,9 +1006,10 @@ static qi_status plan_create(int32_t num_qubits, int32_t precision, const qi_gat
     // as much: 4 / 10 / 20 / 40 layers, runs and (blocks), us: 20 qubits 486 / 720 / 1159 / 1981 (1661 / 1868 /
     // 2183 / 2726); 21 qubits 640 / 1018 / 1628 / 2829 (1764 / 1848 / 2195 / 2781); 22 qubits 927 / 1463 / 2371 /
     // 4156 (1860 / 2055 / 2486 / 3226); 23 qubits 1559 / 2458 / 4054 / 7189 (2172 / 2386 / 3129 / 3976): even at
-    // about 1700 gates of 21 qubits (40 layers), half as many a qubit more.
+    // about 1700 gates of 21 qubits (40 layers), half as many a qubit more.  Below 7 qubits blocks are more exact
+    // (build_runs).
     if (one_call) {
-        p->run_min = 4;
+        p->run_min = 7;
         if (num_qubits <= 23 && std::ldexp((double)elems.size(), num_qubits - 21) <= 1700.0) p->run_max = 23;
     }
     if (st.ok()) st = build_plan(p, elems);
