@@ -1307,20 +1307,9 @@ qi_status qi_circuit_execute(qi_state *s, const qi_gate *gates, int64_t n_gates,
     return st;
 }
 
-qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_terms, double dt, int64_t num_steps,
-                            int32_t order, const qi_pauli_term *observable, int64_t n_obs, int64_t observe_every,
-                            double *energies_out) {
-    if (!s || (!terms && n_terms > 0)) return publish(err(QI_ERR_NULL_ARGUMENT));
-    std::lock_guard<std::recursive_mutex> lk(s->mu);
-    cudaError_t e = cudaSetDevice(s->device);
-    if (e != cudaSuccess) return publish(cuda_status(e, "cudaSetDevice"));
-    if (n_terms == 0) return publish(err(QI_ERR_INVALID_NUMBER_OF_QUBITS, 0));   // time_evolution.rs:51-53
-    if (order != 1 && order != 2) return publish(err(QI_ERR_INVALID_INPUT_VALUE, order));
-    for (int64_t k = 0; k < n_terms; ++k) {
-        Status st = validate_pauli(s->n, terms[k]);
-        if (!st.ok()) return publish(st);
-    }
-    if (observable && observe_every > 0 && !energies_out) return publish(err(QI_ERR_NULL_ARGUMENT));
+static Status trotter_steps(qi_state *s, const qi_pauli_term *terms, int64_t n_terms, double dt, int64_t num_steps,
+                            int32_t order, bool unitary, const qi_pauli_term *observable, int64_t n_obs,
+                            int64_t observe_every, double *energies_out) {
     // `steps` steps as an ordered list of exponentials (time_evolution.rs:45-115).
     auto step_list = [&](int64_t steps) {
         std::vector<Elem> elems;
@@ -1341,8 +1330,6 @@ qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_t
     // compute-bound), so the exponentials run as gate runs, two operations per
     // amplitude each; where some cannot (wide X strings), each run of exponentials whose
     // X-masks lie in {0, X} is one pass with a parity-indexed table.
-    bool unitary = true;
-    for (int64_t k = 0; k < n_terms; ++k) unitary = unitary && terms[k].coeff_im == 0.0;
     const bool observing = observable && observe_every > 0;
     // FP64 second-order steps: the terms that end one step begin the next, and equal exponentials with
     // nothing between join (qi_gaterun.cu), so a plan covers several steps: the most up to 6 that divide
@@ -1374,8 +1361,10 @@ qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_t
         const double runs = halves * nt * (0.65 + 0.68 * size);
         const double pass = std::max({55.0, 15.0 * (s->n - 14), 33.0 * size});
         const double blocks = 250.0 * order + halves * std::max(1.0, nt / 140.0) * pass;
-        plan.run_min = 4;
-        plan.run_max = runs <= blocks ? s->n : 0;
+        // Nor where blocks are more exact: below 13 qubits, and in one or two passes over the terms (13 to 21
+        // qubits: 0.44-1.7 times the blocks' error; in three and more 0.09-0.82).
+        plan.run_min = 13;
+        plan.run_max = runs <= blocks && order * num_steps >= 3 ? s->n : 0;
         plan.opts.renorm_every = unitary ? 0 : -1;
         plan.opts.max_block_qubits = 0;
         std::vector<Elem> elems = step_list(steps);
@@ -1424,10 +1413,43 @@ qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_t
         plan->d_tc = nullptr;
         plan->d_mats = nullptr;
     }
-    e = cudaStreamSynchronize(s->stream);   // the programs are in use until then
-    if (!st.ok()) return publish(st);
-    if (e != cudaSuccess) return publish(cuda_status(e, "trotter"));
-    return publish(ok_status());
+    const cudaError_t e = cudaStreamSynchronize(s->stream);   // the programs are in use until then
+    if (st.ok() && e != cudaSuccess) st = cuda_status(e, "trotter");
+    return st;
+}
+
+qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_terms, double dt, int64_t num_steps,
+                            int32_t order, const qi_pauli_term *observable, int64_t n_obs, int64_t observe_every,
+                            double *energies_out) {
+    if (!s || (!terms && n_terms > 0)) return publish(err(QI_ERR_NULL_ARGUMENT));
+    std::lock_guard<std::recursive_mutex> lk(s->mu);
+    cudaError_t e = cudaSetDevice(s->device);
+    if (e != cudaSuccess) return publish(cuda_status(e, "cudaSetDevice"));
+    if (n_terms == 0) return publish(err(QI_ERR_INVALID_NUMBER_OF_QUBITS, 0));   // time_evolution.rs:51-53
+    if (order != 1 && order != 2) return publish(err(QI_ERR_INVALID_INPUT_VALUE, order));
+    for (int64_t k = 0; k < n_terms; ++k) {
+        Status st = validate_pauli(s->n, terms[k]);
+        if (!st.ok()) return publish(st);
+    }
+    if (observable && observe_every > 0 && !energies_out) return publish(err(QI_ERR_NULL_ARGUMENT));
+    bool unitary = true;
+    for (int64_t k = 0; k < n_terms; ++k) unitary = unitary && terms[k].coeff_im == 0.0;
+    // FP32 states of fewer than 12 qubits evolve in FP64 and are rounded at the end.  A small step's
+    // exponentials are near the identity: FP32 gate runs had 1.3-8 times the error of blocks on one to three
+    // steps (lattices of 4 to 10 qubits), and blocks of these sizes take a plan of 1 ms to compose.
+    qi_state *wide = nullptr;
+    if (s->prec == QI_F32 && s->n < 12 && unitary && num_steps > 0 && scratch_take(s, QI_F64, &wide).ok()) {
+        Status st = state_copy_async(wide, s);
+        if (st.ok())
+            st = trotter_steps(wide, terms, n_terms, dt, num_steps, order, unitary, observable, n_obs, observe_every, energies_out);
+        if (st.ok()) st = state_copy_async(s, wide);
+        e = cudaStreamSynchronize(s->stream);
+        if (st.ok() && e != cudaSuccess) st = cuda_status(e, "trotter");
+        scratch_give(wide);
+        return publish(st);
+    }
+    return publish(trotter_steps(s, terms, n_terms, dt, num_steps, order, unitary, observable, n_obs, observe_every,
+                                 energies_out));
 }
 
 }  // extern "C"
