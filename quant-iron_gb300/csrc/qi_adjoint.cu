@@ -769,17 +769,30 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
         plan.opts = plan_opts;
         std::vector<Elem> elems;
         Status st = plan_elems_from_gates(n, gates, n_gates, theta, n_theta, elems);
-        // FP64 (dense FP64 blocks are bound by the FP64 pipe) and FP32 up to 22 qubits: the gate runs' own
-        // arithmetic, with no block matrices to compose (FP32 gradients, fused / gate runs: 8 qubits 1.57 /
-        // 0.37 ms, 20 qubits 4.25 / 2.58, 22 qubits 7.8 / 6.2, 24 qubits 18.0 / 20.1; relative error at 20
-        // qubits 6.1e-7 / 4.7e-7).  FP32 only where every gate joins a run: each that cannot (a matchgate) is a
-        // pass of its own where a block takes several.
+        // FP64: gate runs (dense FP64 blocks are bound by the FP64 pipe).  FP32, where every gate joins a run (a
+        // matchgate is a pass of its own where a block takes several): below 12 qubits gate runs in FP64 on a
+        // scratch copy, rounded at the end (blocks of these sizes take 1 ms to compose, FP32 runs had up to 1.4
+        // times the gradient's error); up to 22 qubits FP32 runs from the depth on where blocks of five on the
+        // tensor cores, which truncate, have the larger error (RY / RZ / CNOT layers, n = 12 / 14 / 16 / 18: equal
+        // at 4 / 5 / 6 / 9 layers, gradient's error of runs relative to blocks 1.1-1.2 at 3, 0.6 / 0.6 / 0.7 / 0.9
+        // at 10; 20 and 22 qubits 1.05-1.3 up to 10 layers); else blocks.
         bool runs = !chosen && (s->prec == QI_F64 || n <= kSweepMaxF32);
         for (size_t i = 0; runs && s->prec == QI_F32 && i < elems.size(); ++i) runs = run_supported(n, s->prec, elems[i]);
+        qi_state *wide = nullptr;
+        if (runs && s->prec == QI_F32) {
+            if (n < 12) runs = st.ok() && scratch_take(s, QI_F64, &wide).ok();
+            else runs = (double)elems.size() >= 150.0 * std::exp2(0.29 * (n - 12));
+        }
         if (runs) plan.opts.fusion = QI_FUSION_NONE;
+        if (wide) {
+            plan.prec = QI_F64;
+            st = state_copy_async(wide, s);
+        }
         if (st.ok()) st = build_plan(&plan, elems);
         if (st.ok()) st = upload_plan(&plan);
-        if (st.ok()) st = plan_execute(&plan, s);
+        if (st.ok()) st = plan_execute(&plan, wide ? wide : s);
+        if (st.ok() && wide) st = state_copy_async(s, wide);
+        if (wide) scratch_give(wide);
         if (plan.d_mats) cudaFree(plan.d_mats);
         if (plan.d_tc) cudaFree(plan.d_tc);
         release_runs(&plan);
