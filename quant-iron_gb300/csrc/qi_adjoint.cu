@@ -791,6 +791,9 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
         if (st.ok()) st = build_plan(&plan, elems);
         if (st.ok()) st = upload_plan(&plan);
         if (st.ok()) st = plan_execute(&plan, wide ? wide : s);
+        // tensor-core blocks are followed by a renormalisation, so that psi_0 of another norm is taken as normalised;
+        // the same where runs take their place
+        if (st.ok() && runs && s->prec == QI_F32 && !wide) st = state_normalise_device_async(s);
         if (st.ok() && wide) st = state_copy_async(s, wide);
         if (wide) scratch_give(wide);
         if (plan.d_mats) cudaFree(plan.d_mats);

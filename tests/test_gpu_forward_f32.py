@@ -1,4 +1,5 @@
-"""FP32 gradients: the forward pass is no less exact than fused blocks (block size named), whatever the size and depth."""
+"""FP32 gradients: the forward pass is no less exact than fused blocks (block size named), whatever the size and depth,
+and treats a state of another norm as blocks do."""
 import numpy as np
 import pytest
 
@@ -38,3 +39,18 @@ def test_error_is_no_larger_than_with_blocks(qi, n, layers):
                 _, g = qi.adjoint_gradient(a, gates, theta, terms, max_block_qubits=block)
                 err[block].append(np.linalg.norm(g - want) / np.linalg.norm(want))
     assert np.sqrt(np.mean(np.square(err[0]))) <= 1.15 * np.sqrt(np.mean(np.square(err[5])))
+
+
+@pytest.mark.parametrize("layers", [2, 12])
+@pytest.mark.parametrize("n", [8, 14])
+def test_states_of_another_norm(qi, n, layers):
+    """|psi_0| = 2, against the call with blocks: energies within FP32 rounding of up to 500 gates."""
+    gates, theta = ansatz(n, layers, np.random.default_rng(n))
+    terms = workloads.heisenberg_open_chain(n, seed=n)
+    with qi.DeviceState(n, qi.F32) as s:
+        s.set_zero()
+        s.scale(2.0)
+        e, g = qi.adjoint_gradient(s, gates, theta, terms)
+        e5, g5 = qi.adjoint_gradient(s, gates, theta, terms, max_block_qubits=5)
+        assert abs(e - e5) <= 500 * 2.0 ** -24 * 4.0 * len(terms)
+        assert np.linalg.norm(g - g5) <= 500 * 2.0 ** -24 * 4.0 * len(terms)
