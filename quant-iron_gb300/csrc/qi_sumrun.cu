@@ -27,6 +27,7 @@
 #include "qi_runtile.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <map>
 
@@ -52,10 +53,15 @@ static_assert(sizeof(SumHdr) == 32, "program layout");
 // Weights of a pair, c = conj(psi_i) psi_j.  Expectation: kPairFirst re += w Re c; kPairSecond
 // re += w Im c; kPairGeneral (p, q, s, t) re += p Re c + q Im c, im += s Re c + t Im c.
 // Apply, f(i) and f(j): kPairFirst real (f, g); kPairSecond imaginary; kPairGeneral (f, g) complex.
-enum SumKind : int { kPairFirst = 0, kPairSecond = 1, kPairGeneral = 2, kDiagReal = 3, kDiagComplex = 4 };
+// kDiagSplit (FP32, real coefficients): every coefficient as a multiple of 2^-23 of their sum's size, whose sums are
+// exact in FP32, and the rest; both are summed and transformed.  Sums of rounded coefficients err alike in all
+// amplitudes that share them: <H> of fields and bonds on 10 to 19 qubits 1.2-2.2 times the error of a factor per
+// amplitude (0.5-0.8 from 20 on), split 0.04-0.35.
+enum SumKind : int { kPairFirst = 0, kPairSecond = 1, kPairGeneral = 2, kDiagReal = 3, kDiagComplex = 4, kDiagSplit = 5 };
 constexpr int kMaxPhases = 24;  // phases of a pass (their thread tables: 1 KB each at most)
 constexpr int kMaxDiag = 96;   // distinct local Z masks of a pass's diagonal group
 constexpr int kMaxDiagTerms = 256;
+constexpr int kSplitExpect = 19, kSplitApply = 11;   // kDiagSplit up to this many qubits
 // Register bits of a phase: FP64 3 (its arithmetic is the bound), FP32 4 (a phase's set-up and an
 // operation's decoding are shared by 32 amplitudes instead of 16)
 // of an expectation; an applied phase holds the sums too and keeps to 3
@@ -97,14 +103,49 @@ __device__ __forceinline__ void load_weights(T (&w)[N], const T *c) {   // c 16-
     }
 }
 
-template <typename T, int X, int KIND, bool APPLY>
+// A thread's sum.  FP64: of a tile.  FP32: of all its tiles, as two lanes of a float and the sum of its additions'
+// rounding errors (Knuth's two-sum, exact), seven packed operations for two addends: FP64 operations would
+// bound the pass, and FP32 sums of a tile's groups lost up to eight times the bits of sums of single pairs.
+template <typename T> struct SumAcc {
+    T v = T(0);
+};
+template <> struct SumAcc<float> {
+    uint64_t hi = 0, lo = 0;
+    static __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+        uint64_t d;
+        asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+        return d;
+    }
+    static __device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {   // a - b, rounded once
+        uint64_t d;
+        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(b), "l"(0xbf800000bf800000ull), "l"(a));
+        return d;
+    }
+    __device__ __forceinline__ void add(float a, float b) {
+        uint64_t x;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(a), "f"(b));
+        const uint64_t s = add2(hi, x), t = sub2(s, hi);
+        lo = add2(lo, add2(sub2(hi, sub2(s, t)), sub2(x, t)));
+        hi = s;
+    }
+    __device__ __forceinline__ double total() const {
+        const float h0 = __uint_as_float((uint32_t)hi), h1 = __uint_as_float((uint32_t)(hi >> 32));
+        const float l0 = __uint_as_float((uint32_t)lo), l1 = __uint_as_float((uint32_t)(lo >> 32));
+        // infinities and NaN have no rounding error
+        return ((double)h0 + (isfinite(h0) ? l0 : 0.0f)) + ((double)h1 + (isfinite(h1) ? l1 : 0.0f));
+    }
+};
+
+// FINE (FP32 expectations): every pair on its own enters the sum, else chains of eight do.
+template <typename T, int X, int KIND, bool APPLY, bool FINE>
 __device__ __forceinline__ void sum_pair(const typename Cx<T>::V2 (&v)[1 << SumShape<T, APPLY>::kRegBits],
-                                         typename Cx<T>::V2 (&o)[APPLY ? 1 << SumShape<T, APPLY>::kRegBits : 1], const T *c, T &re,
-                                         T &im) {
+                                         typename Cx<T>::V2 (&o)[APPLY ? 1 << SumShape<T, APPLY>::kRegBits : 1], const T *c,
+                                         SumAcc<T> &re, SumAcc<T> &im) {
     using V2 = typename Cx<T>::V2;
     constexpr int NV = 1 << SumShape<T, APPLY>::kRegBits, NP = NV / 2, NW = KIND == kPairGeneral ? 4 : APPLY ? 2 : 1;
     constexpr int STEP = 4 / NW;   // pairs whose weights are loaded together
-    T part = T(0);
+    [[maybe_unused]] T part = T(0);
+    [[maybe_unused]] T t[2] = {T(0), T(0)}, u[2] = {T(0), T(0)};   // FP32: two chains of each component
 #pragma unroll
     for (int p0 = 0; p0 < NP; p0 += STEP) {
         T w[STEP * NW];
@@ -125,8 +166,23 @@ __device__ __forceinline__ void sum_pair(const typename Cx<T>::V2 (&v)[1 << SumS
                     o[k] = Cx<T>::fma(Cx<T>::make(f[0], f[1]), b, o[k]);
                     o[k ^ X] = Cx<T>::fma(Cx<T>::make(f[2], f[3]), a, o[k ^ X]);
                 }
+            } else if constexpr (sizeof(T) == 4) {
+                T &acc = t[p & 1], &acc_im = u[p & 1];
+                if (FINE) acc = acc_im = T(0);
+                if constexpr (KIND == kPairGeneral) {
+                    const T cr = ::fma(a.x, b.x, a.y * b.y), ci = ::fma(a.x, b.y, -a.y * b.x);
+                    acc = ::fma(f[0], cr, ::fma(f[1], ci, acc));
+                    acc_im = ::fma(f[2], cr, ::fma(f[3], ci, acc_im));
+                } else {
+                    const T x = KIND == kPairFirst ? ::fma(a.x, b.x, a.y * b.y) : ::fma(a.x, b.y, -a.y * b.x);
+                    acc = ::fma(f[0], x, acc);
+                }
+                if ((p & 1) && (FINE || p == NP - 1)) {
+                    re.add(t[0], t[1]);
+                    if constexpr (KIND == kPairGeneral) im.add(u[0], u[1]);
+                }
             } else {
-                T &acc = (p & 1) ? part : re;   // two chains
+                T &acc = (p & 1) ? part : re.v;   // two chains
                 if constexpr (KIND == kPairFirst) {
                     acc = ::fma(f[0], ::fma(a.x, b.x, a.y * b.y), acc);
                 } else if constexpr (KIND == kPairSecond) {
@@ -134,26 +190,26 @@ __device__ __forceinline__ void sum_pair(const typename Cx<T>::V2 (&v)[1 << SumS
                 } else {
                     const T cr = ::fma(a.x, b.x, a.y * b.y), ci = ::fma(a.x, b.y, -a.y * b.x);
                     acc = ::fma(f[0], cr, ::fma(f[1], ci, acc));
-                    im = ::fma(f[2], cr, ::fma(f[3], ci, im));
+                    im.v = ::fma(f[2], cr, ::fma(f[3], ci, im.v));
                 }
             }
         }
     }
-    if constexpr (!APPLY) re += part;
+    if constexpr (!APPLY && sizeof(T) == 8) re.v += part;
 }
 
 // Dispatch on the partner mask; MASKS of three bits only for the one-component kinds.
-template <typename T, int KIND, bool APPLY>
+template <typename T, int KIND, bool APPLY, bool FINE>
 __device__ __forceinline__ void sum_pair_x(int xi, const typename Cx<T>::V2 (&v)[1 << SumShape<T, APPLY>::kRegBits],
-                                           typename Cx<T>::V2 (&o)[APPLY ? 1 << SumShape<T, APPLY>::kRegBits : 1], const T *c, T &re,
-                                           T &im) {
-#define QI_X(M) case M: sum_pair<T, M, KIND, APPLY>(v, o, c, re, im); break;
+                                           typename Cx<T>::V2 (&o)[APPLY ? 1 << SumShape<T, APPLY>::kRegBits : 1], const T *c,
+                                           SumAcc<T> &re, SumAcc<T> &im) {
+#define QI_X(M) case M: sum_pair<T, M, KIND, APPLY, FINE>(v, o, c, re, im); break;
     switch (xi) {
         QI_X(1) QI_X(2) QI_X(3) QI_X(4) QI_X(5) QI_X(6)
     default: break;
     }
     if constexpr (KIND != kPairGeneral || sizeof(T) == 8) {
-        if (xi == 7) sum_pair<T, 7, KIND, APPLY>(v, o, c, re, im);
+        if (xi == 7) sum_pair<T, 7, KIND, APPLY, FINE>(v, o, c, re, im);
     }
     if constexpr (sizeof(T) == 4) {
         switch (xi) {
@@ -170,7 +226,7 @@ __device__ __forceinline__ void sum_pair_x(int xi, const typename Cx<T>::V2 (&v)
 #undef QI_X
 }
 
-template <typename T, bool APPLY>
+template <typename T, bool APPLY, bool FINE>
 __global__ void __launch_bounds__(1 << (kRunTileBits - SumShape<T, APPLY>::S), 512 >> (kRunTileBits - SumShape<T, APPLY>::S))
     k_sum_run(const typename Cx<T>::V2 *in, typename Cx<T>::V2 *out, int add,
                                                  uint64_t ntiles, const uint4 *prog, const __grid_constant__ SumGeom g,
@@ -195,6 +251,7 @@ __global__ void __launch_bounds__(1 << (kRunTileBits - SumShape<T, APPLY>::S), 5
     const uint4 *in4 = reinterpret_cast<const uint4 *>(in);
     uint4 *out4 = reinterpret_cast<uint4 *>(out);
     double dre = 0.0, dim = 0.0;
+    SumAcc<T> re, im;
     copy_wait();
     __syncthreads();
     uint32_t pc0 = 0;
@@ -233,7 +290,7 @@ __global__ void __launch_bounds__(1 << (kRunTileBits - SumShape<T, APPLY>::S), 5
             }
             __syncthreads();
         }
-        T re = T(0), im = T(0);
+        if constexpr (sizeof(T) == 8) re.v = im.v = T(0);
         uint32_t pc = 0;
         for (int ph = 0; ph < g.nphase; ++ph) {
             const RunPhaseHdr &hd = *reinterpret_cast<const RunPhaseHdr *>(code + pc);
@@ -264,7 +321,7 @@ __global__ void __launch_bounds__(1 << (kRunTileBits - SumShape<T, APPLY>::S), 5
                 const int kind = h.kind;
                 if (kind >= kDiagReal) {
                     const uint16_t *range = reinterpret_cast<const uint16_t *>(code + pc + 2), *mask = range + NV + 1;
-                    for (int part = 0; part < (kind == kDiagComplex ? 2 : 1); ++part) {
+                    for (int part = 0; part < (kind == kDiagReal ? 1 : 2); ++part) {
                         T A[NV];
 #pragma unroll
                         for (int m = 0; m < NV; ++m) {
@@ -288,15 +345,24 @@ __global__ void __launch_bounds__(1 << (kRunTileBits - SumShape<T, APPLY>::S), 5
                                     A[m] = x + y;
                                     A[m | b] = x - y;
                                 }
+                        [[maybe_unused]] T t[2] = {T(0), T(0)};   // FP32: two chains, FINE: two values
 #pragma unroll
                         for (int k = 0; k < NV; ++k) {
                             if constexpr (APPLY) {
-                                if (part == 0) o[k] = Cx<T>::make(::fma(A[k], v[k].x, o[k].x), ::fma(A[k], v[k].y, o[k].y));
+                                if (part == 0 || kind == kDiagSplit) o[k] = Cx<T>::make(::fma(A[k], v[k].x, o[k].x), ::fma(A[k], v[k].y, o[k].y));
                                 else o[k] = Cx<T>::make(::fma(-A[k], v[k].y, o[k].x), ::fma(A[k], v[k].x, o[k].y));
                             } else {
                                 const T p = ::fma(v[k].x, v[k].x, v[k].y * v[k].y);
-                                if (part == 0) re = ::fma(A[k], p, re);
-                                else im = ::fma(A[k], p, im);
+                                if constexpr (sizeof(T) == 4) {
+                                    t[k & 1] = ::fma(A[k], p, FINE ? T(0) : t[k & 1]);
+                                    if ((k & 1) && (FINE || k == NV - 1)) {
+                                        if (part && kind == kDiagComplex) im.add(t[0], t[1]);
+                                        else re.add(t[0], t[1]);
+                                    }
+                                } else {
+                                    if (part == 0) re.v = ::fma(A[k], p, re.v);
+                                    else im.v = ::fma(A[k], p, im.v);
+                                }
                             }
                         }
                     }
@@ -308,9 +374,9 @@ __global__ void __launch_bounds__(1 << (kRunTileBits - SumShape<T, APPLY>::S), 5
                 if (h.r == 2 && ((__popc(lbase & h.zl1) + __popcll(tbase & h.zg1)) & 1)) c += 2 * h.stride;
                 const int xi = h.xi;
                 pc += h.units;
-                if (kind == kPairFirst) sum_pair_x<T, kPairFirst, APPLY>(xi, v, o, c, re, im);
-                else if (kind == kPairSecond) sum_pair_x<T, kPairSecond, APPLY>(xi, v, o, c, re, im);
-                else sum_pair_x<T, kPairGeneral, APPLY>(xi, v, o, c, re, im);
+                if (kind == kPairFirst) sum_pair_x<T, kPairFirst, APPLY, FINE>(xi, v, o, c, re, im);
+                else if (kind == kPairSecond) sum_pair_x<T, kPairSecond, APPLY, FINE>(xi, v, o, c, re, im);
+                else sum_pair_x<T, kPairGeneral, APPLY, FINE>(xi, v, o, c, re, im);
             }
             if constexpr (APPLY) {
                 run_store<T, S>(o, otile, at);
@@ -321,14 +387,18 @@ __global__ void __launch_bounds__(1 << (kRunTileBits - SumShape<T, APPLY>::S), 5
             for (uint32_t u = 0; u < nunit; u += nt)
                 out4[first + RunCopy::step(rows, u, lowu)] =
                     *reinterpret_cast<uint4 *>((char *)otile + (mine.at ^ (run_swizzle(u) << 4)));
-        } else {
-            dre += (double)re;   // one conversion and addition per tile (FP64 is the scarce pipe)
-            if (g.cplx) dim += (double)im;
+        } else if constexpr (sizeof(T) == 8) {
+            dre += re.v;
+            if (g.cplx) dim += im.v;
         }
         tbase = next_base;
         __syncthreads();   // the tile is read to the end before the next one lands
     }
     if constexpr (!APPLY) {
+        if constexpr (sizeof(T) == 4) {
+            dre = re.total();
+            if (g.cplx) dim = im.total();
+        }
         const double r0 = block_sum(dre), r1 = block_sum(dim);
         if (tid == 0) {
             partials[blockIdx.x * 4 + 0] = r0;
@@ -358,7 +428,7 @@ static size_t sum_smem(const SumPass &p, int ub0, int tiles, int sel) {
 }
 constexpr int kSumSmemCap = 160 * 1024;   // tiles 64 KB, rows 16 KB, program 24 KB, places 24 KB at most
 
-template <typename T, bool APPLY>
+template <typename T, bool APPLY, bool FINE = false>
 static Status launch_sum(cudaStream_t st, uint64_t dim, const void *in, void *out, bool add, const SumPass &p,
                          const void *d_prog, double *partials, unsigned cap, unsigned *blocks) {
     const int ub0 = RunShape<T>::kUnitBits;
@@ -368,8 +438,8 @@ static Status launch_sum(cudaStream_t st, uint64_t dim, const void *in, void *ou
     const unsigned nb = (unsigned)std::min<uint64_t>(ntiles, cap);
     if (sm > (size_t)kSumSmemCap) return err(QI_ERR_UNKNOWN, (int64_t)sm, kSumSmemCap, "SumOp pass too large");
     if (sm > 36 * 1024)   // beside the static block
-        QI_CUDA(cudaFuncSetAttribute(k_sum_run<T, APPLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSumSmemCap));
-    k_sum_run<T, APPLY><<<nb, threads, sm, st>>>((const typename Cx<T>::V2 *)in, (typename Cx<T>::V2 *)out, add ? 1 : 0, ntiles,
+        QI_CUDA(cudaFuncSetAttribute(k_sum_run<T, APPLY, FINE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSumSmemCap));
+    k_sum_run<T, APPLY, FINE><<<nb, threads, sm, st>>>((const typename Cx<T>::V2 *)in, (typename Cx<T>::V2 *)out, add ? 1 : 0, ntiles,
                                                  (const uint4 *)((const char *)d_prog + p.tile.prog_off), sum_geom(p), partials);
     count_launch();
     if (blocks) *blocks = nb;
@@ -378,6 +448,10 @@ static Status launch_sum(cudaStream_t st, uint64_t dim, const void *in, void *ou
 
 Status launch_sum_expect(qi_state *s, const SumPass &p, const void *d_prog, unsigned *nblocks) {
     const unsigned cap = kReduceBlocks;   // 8 blocks per SM; one row of partials each
+    // FP32 up to 22 qubits: every pair on its own, as one launch per group summed them (a thread had 1 pair of a
+    // group up to 19 qubits, 7 at 22, 32 from 24 on; here a chain of eight).
+    if (s->prec == QI_F32 && s->n <= 22)
+        return launch_sum<float, false, true>(s->stream, s->dim(), s->amps, nullptr, false, p, d_prog, s->d_partials, cap, nblocks);
     if (s->prec == QI_F32)
         return launch_sum<float, false>(s->stream, s->dim(), s->amps, nullptr, false, p, d_prog, s->d_partials, cap, nblocks);
     return launch_sum<double, false>(s->stream, s->dim(), s->amps, nullptr, false, p, d_prog, s->d_partials, cap, nblocks);
@@ -431,6 +505,12 @@ bool pair_table(const SumGroup &g, TwoParities &par, double f[4][4]) {
     return true;
 }
 
+bool any_imaginary(const SumGroup &g) {
+    for (const SumTerm &t : g.terms)
+        if (t.im != 0) return true;
+    return false;
+}
+
 // Weights of the parities' values and which of them are needed (SumKind).
 int pair_weights(const double f[4][4], bool apply, double w[4][4], bool *cplx) {
     bool v[4] = {false, false, false, false};
@@ -470,7 +550,7 @@ bool schedule_sum(int n, int prec, bool apply, const std::vector<SumGroup> &grou
         double f[4][4], w[4][4];
         bool cplx;
         if (n < rbits) leave(i);
-        else if (g.x == 0 && ub0 && !apply && n >= 25) leave(i);   // k_diag_expect_f32 streams at the copy rate
+        else if (g.x == 0 && ub0 && !apply && (n >= 25 || any_imaginary(g))) leave(i);   // k_diag_expect_f32 streams at the copy rate
         else if (g.x == 0 && g.terms.size() <= (size_t)kMaxDiagTerms) diag = (int)i;
         else if (g.x == 0 || __builtin_popcountll(g.x) > 3 || !pair_table(g, par, f)) leave(i);
         else if (ub0 && __builtin_popcountll(g.x) == 3 && pair_weights(f, apply, w, &cplx) == kPairGeneral) leave(i);
@@ -539,6 +619,17 @@ bool schedule_sum(int n, int prec, bool apply, const std::vector<SumGroup> &grou
                 raw(c, (size_t)k * 8);
             }
         };
+        double grid = 0.0;   // of the coefficients' larger parts (kDiagSplit), 0: not split
+        if (diag >= 0 && ub0 && n <= (apply ? kSplitApply : kSplitExpect) && !any_imaginary(groups[(size_t)diag])) {
+            double size = 0.0;
+            for (const SumTerm &t : groups[(size_t)diag].terms) size += std::fabs(t.re);
+            int e = 0;
+            std::frexp(size, &e);
+            const double unit = std::ldexp(1.0, e - 23);   // multiples up to 2^23: their sums fit 24 bits
+            for (const SumTerm &t : groups[(size_t)diag].terms)
+                if (std::isfinite(size) && std::nearbyint(t.re / unit) * unit != t.re) grid = unit;
+        }
+        const bool in_two = grid > 0.0;
         // diagonal terms by local mask (first pass that has room for them: the first)
         std::map<uint32_t, std::vector<SumTerm>> dterms;   // key: local Z mask
         bool with_diag = false;
@@ -656,10 +747,10 @@ bool schedule_sum(int n, int prec, bool apply, const std::vector<SumGroup> &grou
                 }
                 SumHdr h;
                 std::memset(&h, 0, sizeof(h));
-                h.kind = cplx ? kDiagComplex : kDiagReal;
+                h.kind = in_two ? kDiagSplit : cplx ? kDiagComplex : kDiagReal;
                 h.zg0 = present;
                 h.units = (uint32_t)(2 + (body.size() * 2 + 15) / 16);
-                p.diag_complex = cplx;
+                p.diag_complex = cplx || in_two;
                 p.complex_out |= cplx;
                 raw(&h, sizeof(h));
                 raw(body.data(), body.size() * 2);
@@ -684,7 +775,8 @@ bool schedule_sum(int n, int prec, bool apply, const std::vector<SumGroup> &grou
             for (uint32_t l : dorder)
                 for (const SumTerm &t : dterms[l]) {
                     if (ub0) {
-                        const DiagTerm<float> d{t.z & ~W, (float)t.re, (float)t.im};
+                        const double whole = in_two ? std::nearbyint(t.re / grid) * grid : t.re;
+                        const DiagTerm<float> d{t.z & ~W, (float)whole, in_two ? (float)(t.re - whole) : (float)t.im};
                         raw(&d, sizeof(d));
                     } else {
                         const DiagTerm<double> d{t.z & ~W, t.re, t.im};
