@@ -80,6 +80,35 @@ __device__ static inline double block_sum(double v) {
     return r;   // valid in thread 0
 }
 
+// Sum of FP32 values that keeps about 48 bits, two addends at a time: two lanes of a float and the sum of its
+// additions' rounding errors (Knuth's two-sum, exact), seven packed FP32 operations.
+struct PairSum {
+    uint64_t hi = 0, lo = 0;
+    static __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+        uint64_t d;
+        asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+        return d;
+    }
+    static __device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {   // a - b, rounded once
+        uint64_t d;
+        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(b), "l"(0xbf800000bf800000ull), "l"(a));
+        return d;
+    }
+    __device__ __forceinline__ void add(float a, float b) {
+        uint64_t x;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(a), "f"(b));
+        const uint64_t s = add2(hi, x), t = sub2(s, hi);
+        lo = add2(lo, add2(sub2(hi, sub2(s, t)), sub2(x, t)));
+        hi = s;
+    }
+    __device__ __forceinline__ double total() const {
+        const float h0 = __uint_as_float((uint32_t)hi), h1 = __uint_as_float((uint32_t)(hi >> 32));
+        const float l0 = __uint_as_float((uint32_t)lo), l1 = __uint_as_float((uint32_t)(lo >> 32));
+        // infinities and NaN have no rounding error
+        return ((double)h0 + (isfinite(h0) ? l0 : 0.0f)) + ((double)h1 + (isfinite(h1) ? l1 : 0.0f));
+    }
+};
+
 // Insert a zero bit at each of the `np` ascending positions `pos[]` of w.
 __device__ static inline uint64_t insert_zeros(uint64_t w, const int8_t *pos, int np) {
     for (int k = 0; k < np; ++k) {

@@ -1,8 +1,8 @@
 // qi_measure.cu — State::measure / measure_n on the device.
 //
 // Reference: src/components/state.rs:525-784.  Probabilities of the measured
-// qubits are summed in FP64 on the device in a fixed order (FP32 states: FP32
-// sums of 8 |a|^2, each folded into the FP64 sum), copied to the host,
+// qubits are summed in FP64 on the device in a fixed order (FP32 states: a
+// thread's |a|^2 as two floats), copied to the host,
 // normalised and sampled exactly as the reference does (sequential CDF in
 // outcome order, `r < cumulative`, last outcome on fall-through).  The
 // reference draws r from an unseeded rand::rng() (state.rs:601); here r comes
@@ -53,17 +53,22 @@ __global__ void __launch_bounds__(256) k_meas_sum(const typename Cx<T>::V2 *a, c
         else if (p >= 0) out |= bit << p;
     }
     double acc = 0.0, acc2 = 0.0;
+    PairSum sum;   // FP32: every |a|^2 on its own (FP64 additions would bound this pass)
     uint64_t off = 0;
     do {   // subsets of the loop mask, ascending
         if constexpr (sizeof(T) == 4) {
-            float part = 0.0f;   // FP32 sum of eight |a|^2, folded into FP64 once per step
+            float p[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
+            for (int u = 0; u < 8; ++u) {
+                p[u] = 0.0f;
                 if (u < g.unroll) {
                     const float2 v = a[base | off | g.off[u]];
-                    part += fmaf(v.x, v.x, v.y * v.y);
+                    p[u] = fmaf(v.x, v.x, v.y * v.y);
                 }
-            acc += (double)part;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u += 2)
+                if (u < g.unroll) sum.add(p[u], p[u + 1]);
         } else {
             double2 v[8];
 #pragma unroll
@@ -79,6 +84,7 @@ __global__ void __launch_bounds__(256) k_meas_sum(const typename Cx<T>::V2 *a, c
         off = ((off | ~g.loop) + 1) & g.loop;
     } while (off);
     acc += acc2;
+    if constexpr (sizeof(T) == 4) acc = sum.total();
     const unsigned lanes = g.nlane >= 5 ? 0xffffffffu : (1u << (1 << g.nlane)) - 1u;
     for (int j = 0; j < g.nlane; ++j)
         if ((g.lane_free >> j) & 1u) acc += __shfl_xor_sync(lanes, acc, 1 << j);
