@@ -331,13 +331,10 @@ Status measure_state(qi_state *s, int basis, const double *custom_u, const int32
     count_launch();
     st = check_launch("k_collapse");
     if (st.ok()) st = basis_change(s, basis, custom_u, qubits, n_qubits, 1);
-    if (st.ok()) {   // the collapsed state is there when the call returns, for whichever stream reads it
-        int flag = 0;
-        st = state_read_flag(s, &flag);
-    }
     if (!st.ok()) return st;
     *outcome_out = o;
     if (probs_out) std::copy(prob.begin(), prob.end(), probs_out);
+    QI_CUDA(cudaStreamSynchronize(s->stream));   // the collapsed state is there for whichever stream reads it next
     return ok_status();
 }
 
