@@ -807,6 +807,21 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
     Status st = scratch_take(s, s->prec, &lam);
     if (!st.ok()) return bail(err(st.code, -1, -1, "lambda state"));
     double ev[2] = {0, 0};
+    // The tile passes let psi and lambda grow by up to 2^54 each in FP32 (schedule_elems), so a large H is taken as
+    // a power of two times one of size 1 (exact): products of the two then stay within FP32.
+    std::vector<qi_pauli_term> unit_terms;
+    double hsize = 0.0, back = 1.0;
+    for (int64_t k = 0; k < n_terms; ++k) hsize += std::hypot(terms[k].coeff_re, terms[k].coeff_im);
+    if (s->prec == QI_F32 && std::isfinite(hsize) && hsize > 0x1p16) {
+        const int e2 = std::ilogb(hsize);
+        back = std::ldexp(1.0, e2);
+        unit_terms.assign(terms, terms + n_terms);
+        for (qi_pauli_term &t : unit_terms) {
+            t.coeff_re = std::ldexp(t.coeff_re, -e2);
+            t.coeff_im = std::ldexp(t.coeff_im, -e2);
+        }
+        terms = unit_terms.data();
+    }
     if (n_terms > 0) {
         if (st.ok()) st = sumop_apply(lam, s, terms, n_terms);
         if (st.ok()) st = state_inner(s, lam, ev);
@@ -816,7 +831,7 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
     } else {
         e = cudaMemsetAsync(lam->amps, 0, lam->bytes(), s->stream);
     }
-    if (energy_out) *energy_out = ev[0];
+    if (energy_out) *energy_out = back * ev[0];
     // derivative slots (one per parameter of a gate; a gate group uses one per member)
     const int64_t nslots = 3 * n_gates + kMultiComps;
     double *d_gres = nullptr;
@@ -888,7 +903,7 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
                 for (size_t k = 0; k < p.slot.size(); ++k, ++i) {
                     const auto &tp = term_param[(size_t)p.slot[k]];
                     const double f = mats[(size_t)tp.first].kind == QI_GATE_P ? -2.0 : 1.0;   // 2 Re <lambda| dU U^dagger |psi>
-                    grads_out[tp.second] += f * p.size2[k] * h[i];
+                    grads_out[tp.second] += f * p.size2[k] * back * h[i];
                 }
         }
     }
@@ -1137,7 +1152,7 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
                                             s->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
         if (e != cudaSuccess) st = cuda_status(e, "adjoint");
-        for (auto &sp : slot_param) grads_out[sp.param] += 2.0 * h[(size_t)sp.slot] * sp.factor;
+        for (auto &sp : slot_param) grads_out[sp.param] += 2.0 * back * h[(size_t)sp.slot] * sp.factor;
     }
     cudaStreamSynchronize(s->stream);
     if (work) {   // psi_0 never left the caller's buffer; psi ends in one of the sweep's buffers
