@@ -11,7 +11,8 @@ layers/s (40 layers per step).  Inputs (8 GiB of FP32 amplitudes) are far
 larger than the 129 MB L2, so no L2 flush is needed between steps.
 
 Besides the JSON keys the contract requires, the line carries the other
-configurations of the workload family, each against an FP64 result on the device:
+configurations of the workload family, each against an FP64 result on the device
+(seeds and per_gate, which are long, as a line of their own on standard error):
   seeds       the 30-qubit circuit on seeds 0-4: fused FP32 against the plain FP64
               per-gate path (the >= 8x target's denominator), infidelity, full-state
               max amplitude error, energy error, both times;
@@ -629,6 +630,16 @@ def profile_case_adjoint26():
     print("profile case done, E = %.9f, |grad| = %.9f" % (e, float(np.linalg.norm(g))))
 
 
+DETAILS = ("per_gate", "seeds")   # 21 of the line's 28 KB
+
+
+def report(line):
+    """The result as one line on standard output; the long tables go to standard error as a line of their own (a
+    reader that keeps only the last few KB of the output would lose the line's beginning, the value with it)."""
+    print(json.dumps({"details": {k: line.pop(k) for k in DETAILS if k in line}}), file=sys.stderr, flush=True)
+    print(json.dumps(line), flush=True)
+
+
 def main():
     args = parse()
     if args.impl == "reference":
@@ -929,7 +940,7 @@ def main():
                            "plan_build_s": plan_s},
                 "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e, "clocks": clk, "gpu_launches": launches}
         line.update(extra)
-        print(json.dumps(line))
+        report(line)
     if world > 1:
         torch.distributed.destroy_process_group()
 
