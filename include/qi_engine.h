@@ -294,7 +294,8 @@ qi_status qi_sumop_expectation_noalloc(const void *amps, int32_t num_qubits, int
  * first_order_trotter_step, 2 = second_order_trotter_step.  If observable !=
  * NULL and observe_every > 0, <observable> is evaluated (FP64 reduction)
  * after every observe_every steps and written to energies_out[2*k..2*k+1]
- * (k = 0 .. num_steps/observe_every - 1). */
+ * (k = 0 .. num_steps/observe_every - 1).  FP32 states of fewer than 12 qubits and
+ * real coefficients evolve in FP64 on a scratch copy and are rounded at the end. */
 qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_terms,
                             double dt, int64_t num_steps, int32_t order,
                             const qi_pauli_term *observable, int64_t n_obs,
@@ -303,7 +304,8 @@ qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_t
 /* ------------------------------------------------------------------------ */
 /* Circuits (src/circuit.rs:160-202) and the fusion pass                      */
 /* ------------------------------------------------------------------------ */
-#define QI_FUSION_NONE    0  /* one kernel per gate (the plain per-gate method) */
+#define QI_FUSION_NONE    0  /* the plain per-gate method: every gate with its own arithmetic, many to a launch
+                                (qi_plan_run_info) */
 #define QI_FUSION_GREEDY  1  /* greedy fixed-k fuser, k = max_block_qubits */
 #define QI_FUSION_LEARNED 2  /* partitions scored by the learned cost model (greedy fallback) */
 #define QI_FUSION_PAULI_GROUPS 3  /* as NONE, except that each run of Pauli exponentials
@@ -350,15 +352,16 @@ qi_status qi_plan_destroy(qi_plan *p);
  * SumOp, pauli_string.rs:390-507).  No reference counterpart: it sits beside
  * Circuit::execute (circuit.rs:160-172) and differentiates through the
  * parametric gates (parametric_gate.rs:30-211, Parameter::get parameter.rs:52-57).
- * One forward sweep (fused plan), lambda = H psi, then one reverse sweep in
+ * One forward sweep (a fused plan, or per gate where that is faster and no less exact,
+ * unless forward_opts name something; FP32 below 12 qubits in FP64), lambda = H psi, then one reverse sweep in
  * which gates are un-applied to psi and lambda while 2 Re<lambda|dU/dtheta|psi>
  * accumulates in FP64: runs of single-qubit gates share one pass, runs of fixed
  * X / CNOT / SWAP gates are one index permutation, other fixed runs one fused
  * plan of their inverses, the rest one pass per gate (qi_adjoint_sweep_plan
  * lists the passes).  Where every gate is an uncontrolled RX / RY / RZ / P with
  * a parameter or a fixed gate (FP64 states; FP32 up to 22 qubits), the sweep runs
- * as passes over tiles of psi and lambda that hold many gates each.  Differentiable kinds: RX, RY, RZ, P, RYPHASE,
- * RYPHASE_DAG, MATCHGATE (any controls).
+ * as passes over tiles of psi and lambda that hold many gates each.  Differentiable
+ * kinds: RX, RY, RZ, P, RYPHASE, RYPHASE_DAG, MATCHGATE (any controls).
  * On entry `s` holds |psi0>; on return it holds |psi0> again (restored by the
  * reverse sweep up to rounding).  energy_out (may be NULL) receives E;
  * grads_out[j] = dE/dtheta_j for j < n_theta (parameters that no gate uses get 0). */
@@ -480,7 +483,8 @@ qi_status qi_plan_op_phase_poly(const qi_plan *p, int64_t i, uint64_t *c0, uint6
 qi_status qi_plan_op_pauli_group(const qi_plan *p, int64_t i, int32_t *n_tables, int32_t *rank, uint64_t *basis);
 /* How a per-gate plan (QI_FUSION_NONE, QI_FUSION_PAULI_GROUPS) is executed: n_passes launches that each
  * apply a run of operations to tiles held in shared memory, in n_phases register phases altogether, and
- * n_single operations with a launch of their own.  All 0 for fused plans.  Introspection aid. */
+ * n_single operations with a launch of their own.  Greedy FP32 plans of 10 to 12 qubits run the same way
+ * (qi_exec_options); all 0 for other fused plans.  Introspection aid. */
 qi_status qi_plan_run_info(const qi_plan *p, int64_t *n_passes, int64_t *n_phases, int64_t *n_single);
 /* The same passes executed on the host (FP64 plans without single operations) on 2^num_qubits
  * interleaved amplitudes: a check of schedule and programs that needs no device. */

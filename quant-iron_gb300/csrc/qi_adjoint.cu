@@ -856,7 +856,8 @@ extern "C" qi_status qi_adjoint_gradient(qi_state *s, const qi_gate *gates, int6
     // parameter, any fixed gate of a gate run.  They need the copy of psi_0 (psi ends scaled); without
     // fusion each gate keeps its own pass.  FP32 sweeps of more than 22 qubits stream faster through the
     // grouped kernels, which keep one group's arithmetic in the instruction cache (12-layer ansatz, tiles
-    // against groups: 20 qubits 4.2 / 5.9 ms, 22 qubits 7.2 / 8.1, 23 qubits 11.4 / 11.3, 26 qubits 72 / 57).
+    // against groups: 20 qubits 4.2 / 5.9 ms, 22 qubits 7.2 / 8.1, 23 qubits 11.4 / 11.3, 26 qubits 72 / 57;
+    // k_sweep_run<float> as compiled then and now, held to 128 registers, with 0.9 KB of spills a thread).
     bool tiles = st.ok() && work != nullptr && plan_opts.fusion != QI_FUSION_NONE && (!f32 || n <= kSweepMaxF32);
     std::vector<SweepGate> sweep_gates;
     std::vector<std::pair<int, int32_t>> term_param;   // term -> gate, parameter

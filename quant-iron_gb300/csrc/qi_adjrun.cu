@@ -9,7 +9,8 @@
 // passes): FP64 12 qubits, 4 layers 3.4 -> 0.70 ms, 16 qubits, 8 layers 6.8 -> 1.7; FP32 8 qubits 1.75 ->
 // 0.37, 20 qubits, 12 layers 5.9 -> 2.6.  FP64 passes are bound by FP64 arithmetic (6 operations per
 // amplitude and rotation instead of 28), FP32 passes by instruction issue and fetch (issue 42 %, the
-// operations' straight-line code for both states passes through the instruction cache).
+// operations' straight-line code for both states passes through the instruction cache; 128 registers for two blocks
+// an SM leave 0.9 KB of spills a thread).
 //
 // A parametric gate is U = exp(-i theta P / 2) (or a phase), so its term is Im <lambda| P |psi> / 2, two
 // operations per amplitude instead of a general 2x2 derivative, and both states take the same scaled
@@ -325,8 +326,11 @@ static Status launch_sweep(cudaStream_t st, uint64_t dim, void *psi, void *lam, 
     const unsigned threads = 1u << (ubits - kRunSelBits);
     const size_t sm = ((size_t)32 << ubits) + (((size_t)8 << (ubits - lowu)) + 15) / 16 * 16 + (size_t)p.run.prog_bytes +
                       (size_t)g.nphase * 4 * threads;
-    // tiles 32 KB, rows 8 KB, program 24 KB, places 12 KB at most
+    // at most: tiles of 2^11 units of two states 64 KB, 2^8 rows 2 KB (16 KB should a tile have no rows),
+    // program 24 KB, places of 24 phases 24 KB
     constexpr int cap = 128 * 1024;
+    static_assert((32 << kRunTileBits) + (8 << kRunTileBits) + kRunMaxProg + kSweepPhases * 4 * (1 << (kRunTileBits - kRunSelBits)) <= cap,
+                  "every pass fits");
     if (sm > (size_t)cap) return err(QI_ERR_UNKNOWN, (int64_t)sm, cap, "sweep pass too large");
     if (sm > 36 * 1024) QI_CUDA(cudaFuncSetAttribute(k_sweep_run<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, cap));
     const uint64_t ntiles = dim >> g.tbits;

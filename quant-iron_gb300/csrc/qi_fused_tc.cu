@@ -286,7 +286,7 @@ __device__ __forceinline__ void st_cs_v8(float2 *p, float a0, float a1, float a2
 // At most 112 registers a thread: the four of the 14 warps that share an SM quarter then leave it room for two
 // warps of 32 registers, so the blocks that read an upload over the link (k_convert_link) run beside this
 // kernel.  With 113 they wait for an SM: 30-qubit circuits through host buffers 300 ms a step instead of
-// 228-240 (the circuit alone 204 instead of 207).
+// 228-240 (the circuit alone 204 instead of 207).  K = 6 without the rotation spills 28 bytes at 112.
 template <int K, bool ROT, bool PHASE>
 __global__ void __maxnreg__(112) k_fused_tc(float2 *a, const float *blocks, TileGeom g, int *err_flag,
                                                             const uint32_t *__restrict__ poly) {

@@ -17,7 +17,7 @@
 // signs and factors of +-i take none.
 //
 // Measured (benchmark family, FP64): 20 qubits, 40 layers + QFT (1400 gates) 8.6 ms in 1400 launches ->
-// 2.6 ms in 25, 25 qubits, 12 layers + QFT 106 -> 36 ms; the FP64 pipe is 86-88 % busy.  FP32 runs are bound
+// 2.6 ms in 24, 25 qubits, 12 layers + QFT 106 -> 34 ms in 14; the FP64 pipe is 86-88 % busy.  FP32 runs are bound
 // by instruction issue (77 %, mostly register moves, index and sign arithmetic).
 //
 // Reference: Gate::apply / Circuit::execute (src/components/gate.rs:99-122, src/circuit.rs:160-172),
@@ -885,8 +885,9 @@ static void schedule_elems(int n, int prec, const std::vector<RunElem> &E, CDD s
     const int ub0 = prec == QI_F32 ? 1 : 0;
     const int low = tbits >= n ? n : 3 + ub0;   // rows of 128 bytes (rows of 512: up to 10 % slower, more passes)
     const uint64_t lowmask = (1ull << low) - 1, always = ub0 ? 1ull : 0ull;
-    // The product of the scales left out so far; it is applied at the end of the run, or earlier
-    // when it has become small (the amplitudes grow as its reciprocal).
+    // The product of the scales left out so far; it is applied at the end of the run, or at the end of a phase when
+    // it has become small.  The amplitudes grow as its reciprocal, and a phase of 48 rotations adds 2^24 at most:
+    // FP32 states of amplitudes above 2^73 may overflow inside a run (no normalised state comes near).
     const double small = prec == QI_F32 ? 0x1p-30 : 0x1p-300;
     if (E.empty() && (sweep || scalar.one())) return;
     std::vector<int> rem(E.size()), take, ptake, inner, group, rest, free_q, sel_q;

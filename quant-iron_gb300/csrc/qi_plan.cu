@@ -1356,7 +1356,9 @@ static Status trotter_steps(qi_state *s, const qi_pauli_term *terms, int64_t n_t
         // steps 851 / 943, 1612 / 1635; 21 qubits, XYZ, 1 and 5 steps 329 / 372, 1329 / 815, TFIM, 20 steps 2229 /
         // 2820; 22 qubits XYZ, 1 step 474 / 406, TFIM, 2 and 10 steps 403 / 554, 1819 / 1580; 24 qubits, XYZ and
         // TFIM, 1 step 1786 / 823, 667 / 712; second order, 20 qubits XYZ, 2 and 5 steps 599 / 662, 1286 / 1103.
-        // The constants below are fitted to these.
+        // The constants below are fitted to these: lattices of strings on two neighbouring qubits.  Strings of more
+        // than six qubits join no block, and 200 of them are 200 launches a step as blocks, which the rule does
+        // not know.
         const double size = std::ldexp(1.0, s->n - 20), halves = (double)(order * num_steps), nt = (double)n_terms;
         const double runs = halves * nt * (0.65 + 0.68 * size);
         const double pass = std::max({55.0, 15.0 * (s->n - 14), 33.0 * size});
