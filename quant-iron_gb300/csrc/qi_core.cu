@@ -1034,11 +1034,13 @@ qi_status qi_state_set_ghz(qi_state *s) {   // state.rs:305-325
     if (st != QI_OK) return st;
     if (s->prec == QI_F32) {
         float2 v = {(float)r, 0.0f};
-        cudaError_t e = cudaMemcpy((float2 *)s->amps + (s->dim() - 1), &v, sizeof(v), cudaMemcpyHostToDevice);
+        cudaError_t e = cudaMemcpyAsync((float2 *)s->amps + (s->dim() - 1), &v, sizeof(v), cudaMemcpyHostToDevice, s->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
         if (e != cudaSuccess) return publish(cuda_status(e, "ghz"));
     } else {
         double2 v = {r, 0.0};
-        cudaError_t e = cudaMemcpy((double2 *)s->amps + (s->dim() - 1), &v, sizeof(v), cudaMemcpyHostToDevice);
+        cudaError_t e = cudaMemcpyAsync((double2 *)s->amps + (s->dim() - 1), &v, sizeof(v), cudaMemcpyHostToDevice, s->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
         if (e != cudaSuccess) return publish(cuda_status(e, "ghz"));
     }
     return publish(ok_status());
