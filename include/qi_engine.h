@@ -294,7 +294,7 @@ qi_status qi_sumop_expectation_noalloc(const void *amps, int32_t num_qubits, int
  * first_order_trotter_step, 2 = second_order_trotter_step.  If observable !=
  * NULL and observe_every > 0, <observable> is evaluated (FP64 reduction)
  * after every observe_every steps and written to energies_out[2*k..2*k+1]
- * (k = 0 .. num_steps/observe_every - 1).  FP32 states of fewer than 12 qubits and
+ * (k = 0 .. num_steps/observe_every - 1).  FP32 states of up to 12 qubits and
  * real coefficients evolve in FP64 on a scratch copy and are rounded at the end. */
 qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_terms,
                             double dt, int64_t num_steps, int32_t order,
@@ -493,7 +493,9 @@ qi_status qi_plan_run_replay(const qi_plan *p, double *amps);
  * state's stream, and write each operation's device time in milliseconds to
  * ms_out (qi_plan_num_ops entries).  Measurement aid; no reference counterpart. */
 qi_status qi_plan_profile(qi_plan *p, qi_state *s, float *ms_out);
-/* `Circuit::execute` (circuit.rs:160-172) on a resident state: plan + run. */
+/* `Circuit::execute` (circuit.rs:160-172) on a resident state: plan + run.  Greedy FP32 circuits
+ * (other options 0, no measurements) of fewer than 7 qubits, or fewer than 12 with Pauli gates, run
+ * per gate in FP64 on a scratch copy and are rounded at the end. */
 qi_status qi_circuit_execute(qi_state *s, const qi_gate *gates, int64_t n_gates,
                              const double *theta, int64_t n_theta, const qi_exec_options *opts);
 

@@ -447,6 +447,23 @@ static void build_schedule(qi_plan *p, const std::vector<Elem> &elems, const std
 // less: 1.4-1.9 on 7 to 12 qubits (0.2-0.34 from 13 on), so circuits with some keep blocks there.  The
 // ops (with the fused blocks' matrices, most of a plan's build time) are made when something asks for them.
 
+// Whether some of an FP32 plan's blocks run on the tensor cores.
+static bool any_tc_block(int n, const std::vector<Elem> &elems, const std::vector<Block> &blocks) {
+    for (const Block &b : blocks) {
+        const int k = __builtin_popcountll(b.mask);
+        bool diag = true;
+        for (int i : b.members) diag = diag && elems[(size_t)i].diagonal;
+        if (!b.single && !b.perm && !diag && ((k >= 3 && k <= 5 && n >= 12) || (k == 6 && n >= 13))) return true;
+    }
+    return false;
+}
+
+// Pauli exponentials narrow enough become dense elements when fusing.
+static void fuse_narrow_exponentials(std::vector<Elem> &elems, int kmax) {
+    for (Elem &e : elems)
+        if (e.pauli && !e.gm.normalise_after && __builtin_popcountll(e.mask) <= kmax) e.fusable = true;
+}
+
 static bool build_runs(qi_plan *p, const std::vector<Elem> &elems, int fusion, int kmax) {
     p->lazy = false;
     p->run_normalise = false;
@@ -464,13 +481,7 @@ static bool build_runs(qi_plan *p, const std::vector<Elem> &elems, int fusion, i
     if (small_fused) {
         // the state is renormalised at the end when tensor-core blocks would have run (build_plan)
         p->lazy_blocks = partition_with_permutations(p, elems, kmax);
-        for (const Block &b : p->lazy_blocks) {
-            const int k = __builtin_popcountll(b.mask);
-            bool diag = true;
-            for (int i : b.members) diag = diag && elems[(size_t)i].diagonal;
-            if (!b.single && !b.perm && !diag && ((k >= 3 && k <= 5 && p->n >= 12) || (k == 6 && p->n >= 13)))
-                p->run_normalise = p->opts.renorm_every >= 0;
-        }
+        p->run_normalise = p->opts.renorm_every >= 0 && any_tc_block(p->n, elems, p->lazy_blocks);
     }
     std::vector<const Elem *> run;
     for (const Elem &e : elems) run.push_back(&e);
@@ -537,11 +548,7 @@ static Status build_plan_ops(qi_plan *p, std::vector<Elem> &elems, bool ops) {
             use_tc = tcbest;
         }
     }
-    // Pauli exponentials narrow enough become dense elements when fusing.
-    for (Elem &e : elems) {
-        if (e.pauli && !e.gm.normalise_after && fusion != QI_FUSION_NONE && __builtin_popcountll(e.mask) <= kmax)
-            e.fusable = true;
-    }
+    if (fusion != QI_FUSION_NONE) fuse_narrow_exponentials(elems, kmax);
     if (!ops && build_runs(p, elems, fusion, kmax)) return ok_status();
     auto lower_single = [&](const Elem &e) {
         Op op = lower_gate(n, e.gm);
@@ -1283,9 +1290,41 @@ qi_status qi_plan_destroy(qi_plan *p) {
     return QI_OK;
 }
 
+// One-call FP32 circuits that run per gate in FP64 on a scratch copy and are rounded at the end: those of fewer than
+// 12 qubits where FP32 gate runs are less exact than blocks (build_runs), which take 0.7-3 ms to compose (5 and 6 qubits,
+// 20 layers: runs 0.13 and 0.15 ms, blocks 0.76 and 2.9).  Not with measurements: their outcomes are those of the
+// FP32 probabilities.
+static bool wide_circuit(int n, const qi_gate *gates, int64_t n_gates) {
+    if (n >= 12 || !gates) return false;
+    bool exponentials = false;
+    for (int64_t i = 0; i < n_gates; ++i) {
+        if (gates[i].kind == QI_GATE_MEASUREMENT) return false;
+        exponentials = exponentials || gates[i].kind == QI_GATE_PAULI_EVOLUTION || gates[i].kind == QI_GATE_PAULI_STRING;
+    }
+    return n < 7 || exponentials;
+}
+
 qi_status qi_circuit_execute(qi_state *s, const qi_gate *gates, int64_t n_gates, const double *theta, int64_t n_theta,
                              const qi_exec_options *opts) {
     if (!s) return publish(err(QI_ERR_NULL_ARGUMENT));
+    if (s->prec == QI_F32 && opts && opts->fusion == QI_FUSION_GREEDY && opts->max_block_qubits == 0 &&
+        opts->use_tensor_cores == 0 && wide_circuit(s->n, gates, n_gates)) {
+        std::lock_guard<std::recursive_mutex> lk(s->mu);
+        qi_state *wide = nullptr;
+        if (cudaSetDevice(s->device) == cudaSuccess && scratch_take(s, QI_F64, &wide).ok()) {
+            Status st = state_copy_async(wide, s);
+            const qi_exec_options per_gate = {QI_FUSION_NONE, 0, 0, 0};
+            qi_status run = st.ok() ? qi_circuit_execute(wide, gates, n_gates, theta, n_theta, &per_gate) : publish(st);
+            if (run == QI_OK) {
+                st = state_copy_async(s, wide);
+                const cudaError_t e = cudaStreamSynchronize(s->stream);
+                if (st.ok() && e != cudaSuccess) st = cuda_status(e, "execute");
+                run = publish(st);
+            }
+            scratch_give(wide);
+            return run;
+        }
+    }
     qi_plan *p = nullptr;
     qi_status st = plan_create(s->n, s->prec, gates, n_gates, theta, n_theta, opts, true, &p);
     if (st != QI_OK) return st;
@@ -1307,20 +1346,21 @@ qi_status qi_circuit_execute(qi_state *s, const qi_gate *gates, int64_t n_gates,
     return st;
 }
 
+// `steps` steps as an ordered list of exponentials (time_evolution.rs:45-115).
+static std::vector<Elem> step_list(const qi_pauli_term *terms, int64_t n_terms, double dt, int32_t order, int64_t steps) {
+    std::vector<Elem> elems;
+    for (int64_t r = 0; r < steps; ++r) {
+        const double f = order == 1 ? -dt : -dt / 2.0;
+        for (int64_t k = 0; k < n_terms; ++k) elems.push_back(pauli_exp_elem(terms[k], 0.0, f, (int)k));
+        for (int64_t k = n_terms - 1; order == 2 && k >= 0; --k)
+            elems.push_back(pauli_exp_elem(terms[k], 0.0, f, (int)k));
+    }
+    return elems;
+}
+
 static Status trotter_steps(qi_state *s, const qi_pauli_term *terms, int64_t n_terms, double dt, int64_t num_steps,
                             int32_t order, bool unitary, const qi_pauli_term *observable, int64_t n_obs,
                             int64_t observe_every, double *energies_out) {
-    // `steps` steps as an ordered list of exponentials (time_evolution.rs:45-115).
-    auto step_list = [&](int64_t steps) {
-        std::vector<Elem> elems;
-        for (int64_t r = 0; r < steps; ++r) {
-            const double f = order == 1 ? -dt : -dt / 2.0;
-            for (int64_t k = 0; k < n_terms; ++k) elems.push_back(pauli_exp_elem(terms[k], 0.0, f, (int)k));
-            for (int64_t k = n_terms - 1; order == 2 && k >= 0; --k)
-                elems.push_back(pauli_exp_elem(terms[k], 0.0, f, (int)k));
-        }
-        return elems;
-    };
     // FP32: the step is one fused plan: narrow exponentials compose into dense
     // blocks (FP64 composition) and runs of Z-type exponentials into phase
     // polynomials.  With real coefficients every exponential is unitary, so the
@@ -1369,7 +1409,7 @@ static Status trotter_steps(qi_state *s, const qi_pauli_term *terms, int64_t n_t
         plan.run_max = runs <= blocks && order * num_steps >= 3 ? s->n : 0;
         plan.opts.renorm_every = unitary ? 0 : -1;
         plan.opts.max_block_qubits = 0;
-        std::vector<Elem> elems = step_list(steps);
+        std::vector<Elem> elems = step_list(terms, n_terms, dt, order, steps);
         // FP64: grouped exponentials only where some element cannot join a gate run
         plan.opts.fusion = QI_FUSION_GREEDY;
         if (s->prec == QI_F64) {
@@ -1436,14 +1476,23 @@ qi_status qi_trotter_evolve(qi_state *s, const qi_pauli_term *terms, int64_t n_t
     if (observable && observe_every > 0 && !energies_out) return publish(err(QI_ERR_NULL_ARGUMENT));
     bool unitary = true;
     for (int64_t k = 0; k < n_terms; ++k) unitary = unitary && terms[k].coeff_im == 0.0;
-    // FP32 states of fewer than 12 qubits evolve in FP64 and are rounded at the end.  A small step's
+    // FP32 states of up to 12 qubits evolve in FP64 and are rounded at the end.  A small step's
     // exponentials are near the identity: FP32 gate runs had 1.3-8 times the error of blocks on one to three
-    // steps (lattices of 4 to 10 qubits), and blocks of these sizes take a plan of 1 ms to compose.
+    // steps (lattices of 4 to 10 qubits; 12 qubits, TFIM, second order: 2.3), and blocks of these sizes take a plan
+    // of 0.4-1 ms to compose (3x4, XYZ, 1 and 10 steps: blocks 0.93 and 1.50 ms).
     qi_state *wide = nullptr;
-    if (s->prec == QI_F32 && s->n < 12 && unitary && num_steps > 0 && scratch_take(s, QI_F64, &wide).ok()) {
+    if (s->prec == QI_F32 && s->n <= 12 && unitary && num_steps > 0 && scratch_take(s, QI_F64, &wide).ok()) {
         Status st = state_copy_async(wide, s);
         if (st.ok())
             st = trotter_steps(wide, terms, n_terms, dt, num_steps, order, unitary, observable, n_obs, observe_every, energies_out);
+        if (st.ok() && s->n == 12) {   // renormalised where tensor-core blocks would have been (build_runs)
+            qi_plan probe;
+            probe.n = s->n;
+            probe.prec = s->prec;
+            std::vector<Elem> elems = step_list(terms, n_terms, dt, order, 1);
+            fuse_narrow_exponentials(elems, 6);
+            if (any_tc_block(s->n, elems, partition_with_permutations(&probe, elems, 6))) st = state_normalise_device_async(wide);
+        }
         if (st.ok()) st = state_copy_async(s, wide);
         e = cudaStreamSynchronize(s->stream);
         if (st.ok() && e != cudaSuccess) st = cuda_status(e, "trotter");
